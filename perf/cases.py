@@ -119,7 +119,8 @@ def _geometry(key):
     return uvw, freq, dict(vis_count=uvw.shape[0] * c["nt"] * c["nch"], grid_size=c["n"], subgrid_size=c["s"],
                            kernel_size=c["kernel"], max_timesteps=1024,
                            scale_arcsec=float(np.float32(synth.cell_rad(c["cell"]))), wlayer_count=c["w"],
-                           wstep=synth.wstep_for(uvw, freq, c["w"]))
+                           # a hair above max |w| / layers: one channel's largest w has a layer too
+                           wstep=synth.wstep_for(uvw, freq, c["w"]) * (1 + 1e-6))
 
 
 _GEOMETRY_KEYS = ("n", "ants", "nt", "nch", "s", "kernel", "w", "cell", "diameter", "f_lo", "f_hi", "layout")
