@@ -144,6 +144,11 @@ struct p9idg_plan {
     int32_t mode = P9IDG_MODE_FP32;
     int32_t requested_mode = P9IDG_MODE_FP32;
     double tc_w_term = -1;  // max |dw| * max |r| of the plan's samples, once a tensor-core mode was asked for
+    double dw_max = 0;      // max |k| * max |w| over the plan's samples
+    // Whether the FP32 mode's device (complex64) calls run on the tensor cores, with FP16 operands split
+    // hi + lo: see fp32_on_tensor_cores.  The host-array calls, whose results keep to the last bit and
+    // which may pass a uvw of their own, run the sincos kernels.
+    bool fp32_tc = false;
     std::vector<double> freq, wn, uvw;
     std::vector<p9idg_subgrid> subs;
     std::vector<DevSubgrid> dsub;
@@ -290,9 +295,21 @@ void build_gridder_items(p9idg_plan *p) {
     p->lyr_ready = false;
 }
 
+// The FP32 mode's tensor-core form needs its operand rows (S <= 32), the subgrids' |dw - dw0| within
+// its bound (and a field on which the n table is smooth), and enough work per subgrid to pay for a
+// work item's fixed cost (about kItemVis visibilities' worth of tensor-core time): the sincos kernels'
+// cost falls with S^2, the tensor-core form's does not.
+bool fp32_on_tensor_cores(const p9idg_plan *p, double w_dev) {
+    const int S = p->c.subgrid_size;
+    if (S < 16 || !tc_subgrid_size_supported(S) || p->subs.empty() || !(std::fabs(image_size(p->c)) < 1.0f)) return false;
+    if (!(w_dev * tc_r_max(p->lmn, S) <= kFp32MaxDev)) return false;
+    constexpr double kItemVis = 375, kSincosPerVis = 128;  // sincos the SFUs do in a visibility's tensor-core time
+    const double per = static_cast<double>(p->gridded_vis) / static_cast<double>(p->subs.size());
+    return per * S * S > kSincosPerVis * (per + kItemVis);
+}
+
 void finish_plan(p9idg_plan *p) {
     const int S = p->c.subgrid_size;
-    build_gridder_items(p);
     p->gridded_vis = 0;
     for (const auto &s : p->subs) p->gridded_vis += static_cast<int64_t>(s.time_sample_count) * p->nch;
     const float img = image_size(p->c);
@@ -315,6 +332,12 @@ void finish_plan(p9idg_plan *p) {
     }
     p->wn.resize(p->nch);
     for (int i = 0; i < p->nch; i++) p->wn[i] = wavenumber(p->freq[i]);
+    double wmax = 0, w_dev = 0, kmax = 0;
+    subgrid_w_stats(p->subs, p->wn, p->uvw.data(), p->nt, wmax, w_dev);
+    for (double k : p->wn) kmax = std::max(kmax, std::fabs(k));
+    p->dw_max = wmax * kmax;
+    p->fp32_tc = fp32_on_tensor_cores(p, w_dev);
+    build_gridder_items(p);
 }
 
 // ---------- device state ----------
@@ -463,12 +486,16 @@ GridderArgs gridder_args(p9idg_plan *p) {
 }
 
 p9idg_status ensure_tc(p9idg_plan *p) {
-    if (p->tc.ready) return P9IDG_OK;
+    if (p->tc.ready) {
+        tc_set_order(p->tc, p->mode, p->tc.want_order);
+        return P9IDG_OK;
+    }
     // degridder items do not accumulate across visibilities: 16384 measured 1.6 % faster than 8192
     // (32768 the same as 16384), 8192 3.5 % faster than 4096
     p->tc.degrid_chunk = p->dchunk > 0 ? p->dchunk : 16384;
-    return tc_prepare(p->tc, p->subs, p->lmn, p->c.subgrid_size, p->nch, p->wn, p->uvw.data(), p->nt, p->stream,
-                      g_last_error);
+    TRY(tc_prepare(p->tc, p->subs, p->lmn, p->c.subgrid_size, p->nch, p->dw_max, p->stream, g_last_error));
+    tc_set_order(p->tc, p->mode, p->tc.want_order);
+    return P9IDG_OK;
 }
 
 SubgridOpArgs subgrid_args(p9idg_plan *p) {
@@ -483,6 +510,8 @@ SubgridOpArgs subgrid_args(p9idg_plan *p) {
 }
 
 bool use_tc(const p9idg_plan *p) { return p->mode != P9IDG_MODE_FP32; }
+// Whether a degridding call runs on the tensor cores (c128: complex128 output, a host-array call).
+bool use_tc_degrid(const p9idg_plan *p, bool c128) { return use_tc(p) || (p->fp32_tc && !c128); }
 
 // Adder.Add throws "invalid grid" for subgrids outside [0, N-S) (Adder.cs:30-50).
 p9idg_status check_adder_range(const p9idg_plan *p) {
@@ -622,7 +651,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.subgrids = p->d_subgrids.as<float2>();
         a.vis_out = d_vis;
         a.out_c128 = out_c128;
-        if (use_tc(p)) {
+        if (use_tc_degrid(p, out_c128)) {
             TRY(ensure_tc(p));
             TRY(tc_degrid(p->tc, a, p->mode, p->stream, g_last_error));
         } else {
@@ -1305,8 +1334,7 @@ p9idg_status p9idg_plan_set_mode(p9idg_plan *plan, int32_t mode) {
     plan->requested_mode = mode;
     if (mode != P9IDG_MODE_FP32) {
         if (plan->tc_w_term < 0)
-            plan->tc_w_term = tc_w_term(plan->subs, plan->lmn, plan->c.subgrid_size, plan->wn, plan->uvw.data(),
-                                        plan->nt);
+            plan->tc_w_term = plan->dw_max * tc_r_max(plan->lmn, plan->c.subgrid_size);
         if (tc_order_for(plan->tc_w_term, plan->tc.want_order) == 0) {
             // outside both tensor-core forms' error bounds: the FP32 kernels grid this plan
             g_last_error = "tensor-core mode not used: |dw r| = " + std::to_string(plan->tc_w_term) + " > " +
@@ -1315,6 +1343,10 @@ p9idg_status p9idg_plan_set_mode(p9idg_plan *plan, int32_t mode) {
         }
     }
     const bool regroup = (plan->mode == P9IDG_MODE_FP32) != (mode == P9IDG_MODE_FP32);
+    if (plan->mode != mode) {  // the modes check a uvw differently: the next call recomputes its coefficients
+        plan->tc.coef_valid = false;
+        plan->tc.coef_recompute_flag = nullptr;
+    }
     plan->mode = mode;
     if (regroup) build_gridder_items(plan);
     return P9IDG_OK;
@@ -1327,7 +1359,7 @@ p9idg_status p9idg_plan_set_tc_order(p9idg_plan *plan, int32_t order) {
         TRY(ensure_device(plan));
         CK(cudaStreamSynchronize(plan->stream));  // launches in flight use the previous form's limit
     }
-    tc_set_order(plan->tc, order);
+    tc_set_order(plan->tc, plan->mode, order);
     return P9IDG_OK;
 }
 

@@ -51,6 +51,10 @@ p9idg_status validate_subgrids(const p9idg_params &c, const p9idg_subgrid *subs,
 // least one), numbering slots per subgrid, and orders the launch list by descending size.
 void build_work_items(const std::vector<p9idg_subgrid> &subs, int32_t nch, int64_t max_vis,
                       std::vector<DevSubgrid> &dsub, std::vector<WorkItem> &items);
+// Over the subgrids' samples: the largest |w|, and the largest |k w - mean(k) mean(w)|, the means
+// taken per subgrid.
+void subgrid_w_stats(const std::vector<p9idg_subgrid> &subs, const std::vector<double> &wn, const double *uvw,
+                     int32_t nt_all, double &wmax, double &dev_max);
 void fft_shift_host(void *a, int32_t n, int32_t elem_bytes);
 
 // Sets the thread-local message p9idg_last_error() returns (api.cu).

@@ -16,6 +16,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <thread>
 
 #include "p9idg_internal.h"
@@ -230,6 +231,66 @@ p9idg_status validate_subgrids(const p9idg_params &c, const p9idg_subgrid *subs,
     }
     (void)c;
     return P9IDG_OK;
+}
+
+// Per-subgrid statistics of w, with the samples split over the host threads: the largest |w|, and
+// the largest distance of any sample's k w from its subgrid's centre mean(k) mean(w).
+void subgrid_w_stats(const std::vector<p9idg_subgrid> &subs, const std::vector<double> &wn, const double *uvw,
+                     int32_t nt_all, double &wmax, double &dev_max) {
+    wmax = dev_max = 0;
+    if (subs.empty() || wn.empty()) return;
+    double kmin = wn[0], kmax = wn[0], ksum = 0;
+    for (double k : wn) {
+        kmin = std::min(kmin, k);
+        kmax = std::max(kmax, k);
+        ksum += k;
+    }
+    const double kmean = ksum / static_cast<double>(wn.size());
+    int64_t samples = 0;
+    for (const auto &s : subs) samples += s.time_sample_count;
+    // a thread costs as much to start as some 10^5 samples take
+    const int64_t useful = std::min<int64_t>(std::min<int64_t>(1 + samples / 250000, 16), static_cast<int64_t>(subs.size()));
+    const unsigned nthreads = std::max(1u, std::min(std::thread::hardware_concurrency(), static_cast<unsigned>(useful)));
+    std::vector<double> wm(nthreads, 0.0), dm(nthreads, 0.0);  // dm: infinite where a sample is NaN
+    auto worker = [&](unsigned tid) {
+        const size_t i0 = subs.size() * tid / nthreads, i1 = subs.size() * (tid + 1) / nthreads;
+        double wmx = 0, dmx = 0;
+        for (size_t i = i0; i < i1; i++) {
+            const p9idg_subgrid &s = subs[i];
+            if (s.time_sample_count <= 0) continue;
+            const double *q = uvw + (static_cast<int64_t>(s.baseline_idx) * nt_all + s.time_sample_start) * 3 + 2;
+            double lo = q[0], hi = q[0], sum = 0;
+            for (int32_t t = 0; t < s.time_sample_count; t++) {
+                const double w = q[3 * static_cast<int64_t>(t)];
+                lo = std::min(lo, w);
+                hi = std::max(hi, w);
+                sum += w;
+            }
+            const double c = kmean * (sum / s.time_sample_count);
+            wmx = std::max(wmx, std::max(std::fabs(lo), std::fabs(hi)));
+            for (double w : {lo, hi})
+                for (double k : {kmin, kmax}) {
+                    const double d = std::fabs(k * w - c);
+                    dmx = std::isnan(d) ? INFINITY : std::max(dmx, d);
+                }
+        }
+        wm[tid] = wmx;
+        dm[tid] = dmx;
+    };
+    std::vector<std::thread> pool;
+    for (unsigned t = 1; t < nthreads; t++) {
+        try {
+            pool.emplace_back(worker, t);
+        } catch (const std::exception &) {  // no thread to be had: this one does the part
+            worker(t);
+        }
+    }
+    worker(0);
+    for (auto &th : pool) th.join();
+    for (unsigned t = 0; t < nthreads; t++) {
+        wmax = std::max(wmax, wm[t]);
+        dev_max = std::max(dev_max, dm[t]);
+    }
 }
 
 void build_work_items(const std::vector<p9idg_subgrid> &subs, int32_t nch, int64_t max_vis,

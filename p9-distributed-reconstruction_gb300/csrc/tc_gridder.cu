@@ -36,6 +36,17 @@
 //       rows y and y + 1 as packed FP32 pairs
 //   MMA1: A_hi x B rows 64-191 (N128) -> cols 0..127 = [T0 | T1];  MMA2: A_hi x B0_lo (N64),
 //   MMA3: A_lo x B0_hi (N64) -> cols 0..63.  Two accumulators alternate (256 columns).
+//
+// FP32 mode (complex64 degridding): the FP16 degridder, expanded about each subgrid's centre dw0
+// (the mean of its samples' dw): the pixels are rotated by exp(-i dw0 r) in FP32 as the static
+// operand is made, and T1 is weighted by dw - dw0, which is an order smaller than dw (channels
+// and a short track).  FP16 hi + lo holds 22 bits, so what is left is the two phases' FP32
+// rounding and the hardware sincos, as in the sincos kernel: against FP64 7e-7 where that has
+// 8.5e-7 (2047^2, S = 24), and at most its error in every shape tested.  kFp32MaxDev: with
+// |dw - dw0| |r| <= 8e-4 the second-order term left out (3e-7 at most, 4e-8 rms over a subgrid's
+// samples and pixels) and the 11 bits of the first-order rows stay below that.
+// 8.0 M visibilities, S = 24: sincos kernel 2.04 ms (bound by the SFUs at 576 sincos per
+// visibility), this form 0.41 ms (48 useful of 64 sincos).
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -156,12 +167,14 @@ __device__ __forceinline__ void named_bar(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// 2^-e with m * 2^-e in [0.5, 1) (1 for m == 0): exact power-of-two scale
-__device__ __forceinline__ float pow2_scale(float m) {
+// Power-of-two scale (exact) that brings m into [2^(top - 1), 2^top) (1 for m == 0).  With top = 13 the
+// FP16 operands made of values up to sqrt(2) m stay in range and what falls below FP16's normal
+// numbers is under 2^-27 of the largest value.
+__device__ __forceinline__ float pow2_scale(float m, int top) {
     if (!(m > 0.f) || isinf(m)) return 1.f;
     int e;
     frexpf(m, &e);
-    return ldexpf(1.f, -e);
+    return ldexpf(1.f, top - max(e, -112));
 }
 
 // max over the 256 threads of warps 0-7 (named barrier 2); red: 9 floats of shared memory
@@ -180,29 +193,56 @@ __device__ __forceinline__ float block256_max(float v, float *red) {
 
 // ---------------- per-visibility coefficients (FP64 -> FP32) ----------------
 
-// dw_limit = P9IDG_TC_MAX_W_TERM / max |r|: a visibility with a larger |dw| (possible only when a
-// call passes a uvw other than the plan's, which was checked on the host) sets kStatusWTerm.
-__global__ void tc_coef_kernel(const DevSubgrid *subs, const int64_t *coef_off, const double *uvw, const double *wn,
-                               Geometry g, float4 *coef, const int32_t *recompute, double dw_limit,
-                               int32_t *status) {
+// Sum over the block (256 threads); red: 8 doubles of shared memory.
+__device__ __forceinline__ double block256_sum(double v, double *red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (int i = 1; i < 8; i++) v += red[i];
+    __syncthreads();
+    return v;
+}
+
+// One block per subgrid: its centre dw0 (the mean over its samples of dw = woff - k w; times and
+// channels are a full product, so the mean of k times the mean of w), then its visibilities'
+// coefficients.  dw_limit = the form's limit / max |r|: a visibility with a larger |dw| (possible only
+// when a call passes a uvw other than the plan's, which was checked on the host) sets kStatusWTerm
+// (status null: the FP32 mode, which takes any w).
+__global__ void __launch_bounds__(256)
+    tc_coef_kernel(const DevSubgrid *subs, const int64_t *coef_off, const double *uvw, const double *wn, Geometry g,
+                   float4 *coef, float *center, const int32_t *recompute, double dw_limit, int32_t *status) {
+    __shared__ double red[8];
     if (recompute && *recompute == 0) return;  // uvw bit-identical to the one coef was made from
     const DevSubgrid sg = subs[blockIdx.x];
+    const int nvis = sg.nt * g.nch;
+    if (nvis <= 0) {
+        if (threadIdx.x == 0) center[blockIdx.x] = 0.f;
+        return;
+    }
     const double uoff = static_cast<double>(sg.u + g.S / 2 - g.N / 2) * g.uv_scale;
     const double voff = static_cast<double>(sg.v + g.S / 2 - g.N / 2) * g.uv_scale;
     const double woff = 2 * kPi * (static_cast<double>(g.wstep_lambda) * (static_cast<double>(sg.w) + 0.5));
-    const int nvis = sg.nt * g.nch;
+    const double *base = uvw + (static_cast<int64_t>(sg.bl) * g.nt_all + sg.t0) * 3;
+    double ws = 0, ks = 0;
+    for (int t = threadIdx.x; t < sg.nt; t += blockDim.x) ws += base[3 * static_cast<int64_t>(t) + 2];
+    for (int c = threadIdx.x; c < g.nch; c += blockDim.x) ks += wn[c];
+    ws = block256_sum(ws, red);
+    ks = block256_sum(ks, red);
+    const float dw0 = static_cast<float>(woff - (ks / g.nch) * (ws / sg.nt));
+    if (threadIdx.x == 0) center[blockIdx.x] = dw0;
     float4 *out = coef + coef_off[blockIdx.x];
     bool over = false;
     for (int j = threadIdx.x; j < nvis; j += blockDim.x) {
-        const int t = sg.t0 + j / g.nch, ch = j - (j / g.nch) * g.nch;
-        const double *q = uvw + (static_cast<int64_t>(sg.bl) * g.nt_all + t) * 3;
+        const int t = j / g.nch, ch = j - t * g.nch;
+        const double *q = base + static_cast<int64_t>(t) * 3;
         const double k = wn[ch];
         const double dw = woff - k * q[2];
         over |= !(fabs(dw) <= dw_limit);
         out[j] = make_float4(static_cast<float>(uoff - k * q[0]), static_cast<float>(voff - k * q[1]),
-                             static_cast<float>(dw), 0.f);
+                             static_cast<float>(dw), static_cast<float>(dw - static_cast<double>(dw0)));
     }
-    if (over) atomicOr(status, kStatusWTerm);
+    if (over && status) atomicOr(status, kStatusWTerm);
 }
 
 // ---------------- gridder ----------------
@@ -255,7 +295,7 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
         ep_t[k] = (y < S && x < S) ? a.taper[y * S + x] : 0.f;
     }
     float2 *out = a.partials + static_cast<int64_t>(slot) * S * S;
-    const float i0 = 1.f / sv, i1 = 1.f / (sv * sw), i2 = 0.5f / (sv * sw * sw);  // exact: powers of two
+    const float i0 = 1.f / sv, i1 = i0 / sw, i2 = 0.5f * i1 / sw;  // exact: powers of two
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int p = threadIdx.x + k * kGProducerWarps * 32;
@@ -461,7 +501,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
                 const float2 v = load_vis(vrow, j);
                 mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
             }
-            sv = pow2_scale(block256_max(mx, red));
+            sv = pow2_scale(block256_max(mx, red), 0);
         }
         const float sw = BF16 ? 1.f : a.dw_scale;
         for (int i = 0; i < nstages; i++) {
@@ -633,6 +673,10 @@ template <bool BF16, typename OutT, bool BATCH, bool TMA, bool O2>
 __global__ void __launch_bounds__(kDThreads, 2)
     tc_degridder_kernel(const TcArgs L, const TcArgs *__restrict__ probs, const __grid_constant__ TmaMaps maps) {
     constexpr int NB = O2 ? 1 : 2;  // accumulator buffers
+    // FP16 operands with complex64 outputs expand about the subgrid's centre dw0; complex128 outputs (the
+    // host-array calls, whose results keep to the last bit) and BF16 (whose device and host calls agree
+    // to rounding) about dw = 0
+    constexpr bool kCentred = !BF16 && sizeof(OutT) == 8;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_1k(smem_raw);
     unsigned char *bstat = smem;
@@ -682,74 +726,72 @@ __global__ void __launch_bounds__(kDThreads, 2)
         tmem_alloc(tmem_slot, kDTmemCols);
         tmem_relinquish();
     }
-    // static B operand from the subgrid: row (block, 4 (y / 2) + 2 p + y % 2), k = 2x + q; pixels
-    // past the plan's S (a subgrid of S < 32 padded to 32) are zero
+    // Static B operand from the subgrid: row (block, 4 (y / 2) + 2 p + y % 2), k = 2x + q.  A thread
+    // makes the four pixels of one (y, kg) once and writes their chunk of every block: taper, the
+    // rotation by exp(-i dw0 r) to the subgrid's centre, r (.) and r^2 (.) for blocks 2 and 3; pixels
+    // past the plan's S (a subgrid of S < 32 padded to 32) are zero.
     float sq = 1.f;  // FP16: power-of-two scale of this subgrid's pixels
     if (warp < 8) {
         const int S = g.S;
-        const float2 *data = a.subgrids + static_cast<int64_t>(it.subgrid) * S * S;
-        if (!BF16) {
-            float mx = 0.f;
-            for (int pi = threadIdx.x; pi < kS * kS; pi += 256) {
-                const int y = pi >> 5, x = pi & 31;
-                if (y < S && x < S) {
-                    const float2 d = data[shift_half(y, S) * S + shift_half(x, S)];
-                    const float tap = fabsf(a.taper[y * S + x]);
-                    mx = fmaxf(mx, fmaxf(fabsf(d.x), fabsf(d.y)) * tap);
-                }
-            }
-            sq = pow2_scale(block256_max(mx, red));
-        }
-        const float sr = BF16 ? 1.f : a.r_scale;
-        const uint32_t bs = smem_u32(bstat);
-        for (int cc = threadIdx.x; cc < (O2 ? 256 : 192) * 8; cc += 256) {
-            const int cm = cc >> 3, r8 = cc & 7;
-            const int row = (cm >> 3) * 8 + r8, kg = cm & 7;
-            const int blk = row >> 6, rr = row & 63, y = ((rr >> 2) << 1) | (rr & 1), p = (rr >> 1) & 1;
-            // the four x of this chunk: S is a multiple of 4, so they are wholly inside or outside the
-            // subgrid and on one side of the fftshift wrap (consecutive source pixels)
-            const int x0 = kg * 4;
-            float2 dv[4];
-            float tv[4];
-            if (y < S && x0 < S) {
-                const float2 *src = data + shift_half(y, S) * S + shift_half(x0, S);
-                const float *tsrc = a.taper + y * S + x0;
+        const int y = threadIdx.x & 31, kg = threadIdx.x >> 5, x0 = kg * 4;
+        float2 d[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    dv[u] = src[u];
-                    tv[u] = tsrc[u] * sq;
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    dv[u] = make_float2(0.f, 0.f);
-                    tv[u] = 0.f;
-                }
-            }
-            uint32_t w[4];
+        for (int u = 0; u < 4; u++) d[u] = make_float2(0.f, 0.f);
+        // S is a multiple of 4: the four x are wholly inside or outside the subgrid and on one side of
+        // the fftshift wrap (consecutive source pixels)
+        if (y < S && x0 < S) {
+            const float2 *src = a.subgrids + static_cast<int64_t>(it.subgrid) * S * S + shift_half(y, S) * S + shift_half(x0, S);
+            const float *tsrc = a.taper + y * S + x0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const int x = x0 + u;
-                const float2 d = dv[u];
-                const float tap = tv[u];
-                float qre = tap * d.x, qim = tap * d.y;
-                if (blk >= 2) {  // r (.) pix, and r^2 (.) pix for block 3
-                    const float rr2 = a.tabs[kTabR + y * kS + x] * sr;
-                    qre *= rr2;
-                    qim *= rr2;
-                    if (blk == 3) {
-                        qre *= rr2;
-                        qim *= rr2;
-                    }
-                }
-                // p = re: (Q_re, Q_im);  p = im: (Q_im, -Q_re)
-                const float e0 = p == 0 ? qre : qim, e1 = p == 0 ? qim : -qre;
-                uint32_t hi, lo;
-                split_pair<BF16>(e0, e1, hi, lo);
-                w[u] = blk == 0 ? lo : hi;
+                const float2 v = src[u];
+                const float tap = tsrc[u];
+                d[u] = make_float2(tap * v.x, tap * v.y);
             }
-            st_shared_v4(bs + cc * 16, w[0], w[1], w[2], w[3]);
         }
+        if (!BF16) {
+            float mx = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) mx = fmaxf(mx, fmaxf(fabsf(d[u].x), fabsf(d[u].y)));
+            sq = pow2_scale(block256_max(mx, red), kCentred ? 13 : 0);
+        }
+        const float sr = BF16 ? 1.f : a.r_scale;
+        const float dw0 = kCentred ? a.center[it.subgrid] * 0.318309886f : 0.f;  // over pi
+        uint32_t hi[4], lo[4], r1[4], r2[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float r = a.tabs[kTabR + y * kS + x0 + u];
+            float qre = d[u].x * sq, qim = d[u].y * sq;
+            if (kCentred) {  // times exp(-i dw0 r)
+                float sn, cs;
+                sincospif(dw0 * r, &sn, &cs);
+                const float t = qre;
+                qre = t * cs + qim * sn;
+                qim = qim * cs - t * sn;
+            }
+            const float rr = r * sr;
+            split_pair<BF16>(qre, qim, hi[u], lo[u]);
+            r1[u] = Half16<BF16>::pack(qre * rr, qim * rr);
+            if (O2) r2[u] = Half16<BF16>::pack(qre * rr * rr, qim * rr * rr);
+        }
+        // row p = re: (Q_re, Q_im);  p = im: (Q_im, -Q_re) = the halves swapped, the upper one negated
+        auto im_row = [](uint32_t w) { return __byte_perm(w, w, 0x1032) ^ 0x80000000u; };
+        const uint32_t at = smem_u32(bstat) + static_cast<uint32_t>(kg * 128);
+        auto put = [&](int blk, const uint32_t *w) {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const int row = blk * 64 + 4 * (y >> 1) + 2 * p + (y & 1);
+                const uint32_t addr = at + static_cast<uint32_t>((row >> 3) * 1024 + (row & 7) * 16);
+                if (p == 0)
+                    st_shared_v4(addr, w[0], w[1], w[2], w[3]);
+                else
+                    st_shared_v4(addr, im_row(w[0]), im_row(w[1]), im_row(w[2]), im_row(w[3]));
+            }
+        };
+        put(0, lo);
+        put(1, hi);
+        put(2, r1);
+        if (O2) put(3, r2);
         fence_proxy_async();
     }
     tc_fence_before();
@@ -929,7 +971,8 @@ __global__ void __launch_bounds__(kDThreads, 2)
                 break;
             }
             tc_fence_after();
-            const float dwe = BF16 ? c.z : c.z / a.r_scale;  // T1 was formed from r * r_scale
+            const float dwc = kCentred ? c.w : c.z;  // dw - dw0
+            const float dwe = BF16 ? dwc : dwc / a.r_scale;  // T1 was formed from r * r_scale
             const uint32_t acc = tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(b * 128);
             // accumulator columns come in groups of four: (re y, re y+1, im y, im y+1), so rows y and
             // y + 1 are handled side by side in packed FP32x2 arithmetic; vis = sum over y of
@@ -1111,6 +1154,7 @@ void fill_args(TcArgs &t, const GridderArgs &a, const TcPlanState &st) {
     t.subs = a.subs;
     t.coef_off = static_cast<const int64_t *>(st.coef_off);
     t.coef = static_cast<const float4 *>(st.coef);
+    t.center = static_cast<const float *>(st.center);
     t.lmn = a.lmn;
     t.tabs = static_cast<const float *>(st.tables);
     t.taper = a.taper;
@@ -1133,8 +1177,14 @@ int tc_order_for(double w_term, int want_order) {
     return 0;
 }
 
-void tc_set_order(TcPlanState &st, int want_order) {
+void tc_set_order(TcPlanState &st, int mode, int want_order) {
     st.want_order = want_order;
+    st.any_w = mode == P9IDG_MODE_FP32;
+    if (st.any_w) {
+        st.order = 1;
+        st.dw_limit = INFINITY;
+        return;
+    }
     st.order = tc_order_for(st.max_w_r, want_order);
     const double limit = st.order == 1 ? P9IDG_TC_MAX_W_TERM : P9IDG_TC_MAX_W_TERM2;
     st.dw_limit = st.r_max > 0 ? limit / st.r_max : INFINITY;
@@ -1179,34 +1229,16 @@ double separable_tables(const std::vector<float> &lmn, int S, std::vector<float>
     return rmax;
 }
 
-// max |w| over the gridded samples and max |k| over the channels
-void w_k_max(const std::vector<p9idg_subgrid> &subs, const std::vector<double> &wn, const double *uvw_host,
-             int nt_all, double &wmax, double &kmax) {
-    wmax = 0;
-    kmax = 0;
-    for (double k : wn) kmax = std::max(kmax, std::fabs(k));
-    for (const auto &sg : subs)
-        for (int t = 0; t < sg.time_sample_count; t++) {
-            const double w = uvw_host[(static_cast<int64_t>(sg.baseline_idx) * nt_all + sg.time_sample_start + t) * 3 + 2];
-            wmax = std::max(wmax, std::fabs(w));
-        }
-}
-
 }  // namespace
 
-double tc_w_term(const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn, int S,
-                 const std::vector<double> &wn, const double *uvw_host, int nt_all) {
+double tc_r_max(const std::vector<float> &lmn, int S) {
     if (!tc_subgrid_size_supported(S)) return INFINITY;
     std::vector<float> tabs;
-    const double rmax = separable_tables(lmn, S, tabs);
-    double wmax, kmax;
-    w_k_max(subs, wn, uvw_host, nt_all, wmax, kmax);
-    return wmax * kmax * rmax;
+    return separable_tables(lmn, S, tabs);
 }
 
 p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn,
-                        int S, int nch, const std::vector<double> &wn, const double *uvw_host, int nt_all,
-                        cudaStream_t stream, std::string &err) {
+                        int S, int nch, double dw_max, cudaStream_t stream, std::string &err) {
     if (st.ready) return P9IDG_OK;
     if (!tc_subgrid_size_supported(S)) {
         err = "tensor-core kernels support subgrid sizes 8, 16, 24 and 32";
@@ -1218,11 +1250,8 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     std::vector<int64_t> off(subs.size() + 1, 0);
     for (size_t i = 0; i < subs.size(); i++)
         off[i + 1] = off[i] + static_cast<int64_t>(subs[i].time_sample_count) * nch;
-    double wmax, kmax;
-    w_k_max(subs, wn, uvw_host, nt_all, wmax, kmax);
-    st.max_w_r = wmax * kmax * rmax;
+    st.max_w_r = dw_max * rmax;
     st.r_max = rmax;
-    tc_set_order(st, st.want_order);
     for (int i = 0; i < kS; i++) {
         st.m_tab[i] = tabs[kTabL + i];
         st.g_tab[i] = tabs[i];
@@ -1234,13 +1263,8 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
         std::frexp(m, &e);
         return static_cast<float>(std::ldexp(1.0, -e));
     };
-    st.dw_scale = pow2_below(wmax * kmax * 1.0001);
+    st.dw_scale = pow2_below(dw_max * 1.0001);
     st.r_scale = pow2_below(rmax);
-    if (st.order == 0) {
-        err = "w term too large for the separable tensor-core forms (|dw r| = " + std::to_string(st.max_w_r) +
-              " > " + std::to_string(P9IDG_TC_MAX_W_TERM2) + ")";
-        return P9IDG_UNSUPPORTED;
-    }
     // degridder work items: whole time samples, up to degrid_chunk visibilities each
     std::vector<DevSubgrid> dtmp;
     std::vector<WorkItem> ditems;
@@ -1249,6 +1273,7 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     cudaError_t e;
     if ((e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef))) != cudaSuccess ||
         (e = device_alloc(&st.coef_off, sizeof(int64_t) * off.size())) != cudaSuccess ||
+        (e = device_alloc(&st.center, sizeof(float) * std::max<size_t>(1, subs.size()))) != cudaSuccess ||
         (e = device_alloc(&st.tables, sizeof(float) * tabs.size())) != cudaSuccess ||
         (e = device_alloc(&st.ditems, sizeof(WorkItem) * std::max<size_t>(1, ditems.size()))) != cudaSuccess) {
         err = std::string("tensor-core buffers: ") + cudaGetErrorString(e);
@@ -1277,8 +1302,8 @@ static p9idg_status launch_coef(TcPlanState &st, const GridderArgs &a, int32_t n
                                 std::string &err) {
     if (nsub == 0 || st.coef_valid) return P9IDG_OK;
     tc_coef_kernel<<<nsub, 256, 0, stream>>>(a.subs, static_cast<const int64_t *>(st.coef_off), a.uvw, a.wavenumbers,
-                                             a.g, static_cast<float4 *>(st.coef), st.coef_recompute_flag,
-                                             st.dw_limit, a.status);
+                                             a.g, static_cast<float4 *>(st.coef), static_cast<float *>(st.center),
+                                             st.coef_recompute_flag, st.dw_limit, st.any_w ? nullptr : a.status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         err = std::string("coefficient kernel: ") + cudaGetErrorString(e);
@@ -1501,6 +1526,7 @@ p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t
 void tc_release(TcPlanState &st) {
     if (st.coef) cudaFree(st.coef);
     if (st.coef_off) cudaFree(st.coef_off);
+    if (st.center) cudaFree(st.center);
     if (st.tables) cudaFree(st.tables);
     if (st.ditems) cudaFree(st.ditems);
     st = TcPlanState();

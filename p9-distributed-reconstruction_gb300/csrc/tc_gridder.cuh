@@ -17,7 +17,8 @@ struct TcPlanState {
     const int32_t *coef_recompute_flag = nullptr;
     int S = 0;
     int64_t ncoef = 0;
-    void *coef = nullptr;         // float4 {du, dv, dw, 0} per gridded visibility, subgrid order
+    void *coef = nullptr;         // float4 {du, dv, dw, dw - centre} per gridded visibility, subgrid order
+    void *center = nullptr;       // float per subgrid: its centre dw0 = mean(dw)
     void *coef_off = nullptr;     // int64 per subgrid: first coefficient of the subgrid
     void *tables = nullptr;       // float: g[32] (separable part of n), r[32][32] (remainder), l[32],
                                   // zero past the plan's S
@@ -30,6 +31,7 @@ struct TcPlanState {
     int want_order = 0;           // 0: the lowest order whose bound holds; 2: always the second-order form
     int order = 1;                // the form the kernels run: 1 (first order) or 2 (second order)
     double dw_limit = 0;          // limit of the form / max |r|: the largest |dw| a visibility may have
+    bool any_w = false;           // the FP32 mode: no limit on |dw| itself
     float dw_scale = 1.f;         // FP16 mode: power of two with max |dw| * dw_scale < 1
     float r_scale = 1.f;          // FP16 mode: power of two with max |r| * r_scale < 1
     float m_tab[32] = {}, g_tab[32] = {};  // m_y and g_y (the same values serve l_x and f_x)
@@ -42,6 +44,7 @@ struct TcArgs {
     const DevSubgrid *subs;
     const int64_t *coef_off;
     const float4 *coef;
+    const float *center;
     const void *vis;
     const float *lmn;   // l[S], n[S*S]
     const float *tabs;  // f[S], r[S*S]
@@ -65,11 +68,13 @@ bool tc_subgrid_size_supported(int S);
 // Fault injection for the bounded-wait path (p9idg_debug_tc_wait): later launches use this wait
 // limit and have their loader skip input stage `skip_stage` of every work item (-1: off).
 void tc_debug_set(uint64_t wait_ns, int32_t skip_stage);
-// max |dw| * max |r| over the gridded samples of a plan: the largest phase dw * r(x, y) the
-// tensor-core form expands to first order (|dw| <= max |k| * max |w|, as WStepLambda is 0).
-// Host only; compared with P9IDG_TC_MAX_W_TERM before a plan selects a tensor-core mode.
-double tc_w_term(const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn, int S,
-                 const std::vector<double> &wn, const double *uvw_host, int nt_all);
+// max |r| of the plan's pixel table (infinite where the tensor-core kernels do not run its subgrid
+// size).  Host only: times max |dw| (|dw| <= max |k| * max |w|, as WStepLambda is 0) it is the w term
+// compared with P9IDG_TC_MAX_W_TERM before a plan selects a tensor-core mode.
+double tc_r_max(const std::vector<float> &lmn, int S);
+// Largest |dw - dw0| * max |r| of a subgrid (dw0: its centre) up to which the FP32 mode runs on the
+// tensor cores; see tc_gridder.cu.
+constexpr double kFp32MaxDev = 8e-4;
 // Per-problem arguments of a prepared plan (host side; device pointers inside).
 void tc_fill_args(const TcPlanState &st, const GridderArgs &a, TcArgs &t);
 // Coefficients for the plan's current uvw (no-op when still valid).
@@ -85,12 +90,13 @@ p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t
 // The form (1 or 2) a plan with this w term runs for a requested order (0 = automatic), or 0 when
 // neither bound holds (the plan then keeps the FP32 kernels).
 int tc_order_for(double w_term, int want_order);
-// Re-selects the form of a prepared state after p9idg_plan_set_tc_order (no device work).
-void tc_set_order(TcPlanState &st, int want_order);
-// Builds the tables and uploads them (once per plan).
+// Selects the form of a prepared state for the plan's mode (no device work): the FP32 mode always
+// runs the first-order form about the subgrids' centres.
+void tc_set_order(TcPlanState &st, int mode, int want_order);
+// Builds the tables and uploads them (once per plan); dw_max = max |k| * max |w| of its samples.
+// The caller selects the form (tc_set_order) before it launches.
 p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn,
-                        int S, int nch, const std::vector<double> &wn, const double *uvw_host, int nt_all,
-                        cudaStream_t stream, std::string &err);
+                        int S, int nch, double dw_max, cudaStream_t stream, std::string &err);
 p9idg_status tc_grid(TcPlanState &st, const GridderArgs &a, int mode, cudaStream_t stream, std::string &err);
 p9idg_status tc_degrid(TcPlanState &st, const GridderArgs &a, int mode, cudaStream_t stream, std::string &err);
 void tc_release(TcPlanState &st);
