@@ -49,8 +49,9 @@ enum {
  * operand rows, so it costs what S = 32 costs per visibility). */
 enum {
     P9IDG_MODE_FP32 = 0,      /* FP32 accuracy, FP64 per-visibility phase argument: sincos + FMA kernels, and for
-                               * device (complex64) degridding of subgrids of 16, 24 and 32 whose w spread allows it
-                               * FP16 hi+lo tensor-core operands about each subgrid's own w, no less accurate */
+                               * device (complex64) calls on subgrids of 16, 24 and 32 whose w spread allows it
+                               * FP16 hi+lo tensor-core operands about each subgrid's own w, summed in FP32 every
+                               * 64 visibilities, no less accurate */
     P9IDG_MODE_TC_BF16X3 = 1, /* tensor cores, BF16 hi+lo split (3 products), FP32 accumulation */
     P9IDG_MODE_TC_FP16X3 = 2  /* tensor cores, FP16 hi+lo split (3 products), FP32 accumulation */
 };

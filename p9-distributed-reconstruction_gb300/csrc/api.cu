@@ -493,6 +493,7 @@ p9idg_status ensure_tc(p9idg_plan *p) {
     // degridder items do not accumulate across visibilities: 16384 measured 1.6 % faster than 8192
     // (32768 the same as 16384), 8192 3.5 % faster than 4096
     p->tc.degrid_chunk = p->dchunk > 0 ? p->dchunk : 16384;
+    p->tc.grid_chunk = p->fp32_tc ? (p->gchunk > 0 ? p->gchunk : 4096) : 0;
     TRY(tc_prepare(p->tc, p->subs, p->lmn, p->c.subgrid_size, p->nch, p->dw_max, p->stream, g_last_error));
     tc_set_order(p->tc, p->mode, p->tc.want_order);
     return P9IDG_OK;
@@ -510,8 +511,10 @@ SubgridOpArgs subgrid_args(p9idg_plan *p) {
 }
 
 bool use_tc(const p9idg_plan *p) { return p->mode != P9IDG_MODE_FP32; }
-// Whether a degridding call runs on the tensor cores (c128: complex128 output, a host-array call).
-bool use_tc_degrid(const p9idg_plan *p, bool c128) { return use_tc(p) || (p->fp32_tc && !c128); }
+// Whether a device call (complex64 arrays, the plan's uvw) of the FP32 mode runs on the tensor cores.
+bool use_fp32_tc(const p9idg_plan *p, bool device_call) {
+    return p->mode == P9IDG_MODE_FP32 && p->fp32_tc && device_call;
+}
 
 // Adder.Add throws "invalid grid" for subgrids outside [0, N-S) (Adder.cs:30-50).
 p9idg_status check_adder_range(const p9idg_plan *p) {
@@ -569,9 +572,12 @@ struct ZeroSide {
 };
 
 // Gridder over nitems work items (all of the plan's, or a group of them) into their partial slots.
-p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const WorkItem *d_items, int32_t nitems) {
+// fp32_tc: the items are the FP32 mode's tensor-core form's.
+p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const WorkItem *d_items, int32_t nitems,
+                        bool fp32_tc = false) {
     const int S = p->c.subgrid_size;
-    CK(p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->nslots)));
+    const int32_t nslots = fp32_tc ? p->tc.nslots : p->nslots;
+    CK(p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, nslots)));
     StageScope t(p, P9IDG_STAGE_GRIDDER);
     GridderArgs a = gridder_args(p);
     a.items = d_items;
@@ -579,7 +585,7 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
     a.vis = d_vis;
     a.vis_c128 = vis_c128;
     a.partials = p->d_partials.as<float2>();
-    if (use_tc(p)) {
+    if (use_tc(p) || fp32_tc) {
         TRY(ensure_tc(p));
         TRY(tc_grid(p->tc, a, p->mode, p->stream, g_last_error));
     } else {
@@ -589,9 +595,11 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
 }
 
 // Subgrid IFFT + adder of nsub subgrids (all, or the subgrid list d_list) into the layers.
-p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const int32_t *d_list, int32_t nsub) {
+p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const int32_t *d_list, int32_t nsub,
+                          bool fp32_tc = false) {
     StageScope t(p, P9IDG_STAGE_SUBGRID_IFFT_ADD);
     SubgridOpArgs a = subgrid_args(p);
+    if (fp32_tc) a.subs = static_cast<const DevSubgrid *>(p->tc.gsubs);
     a.partials = p->d_partials.as<float2>();
     a.layers = d_layers;
     a.out_shifted = true;  // IDG.cs:17,37
@@ -606,14 +614,23 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
 
 // The layers are zeroed beside the gridder (a 604 MB fill at 3072^2 with 8 layers, 0.09 ms of the
 // adder's stage when it ran there).
-p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d_layers, bool wstack) {
+p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d_layers, bool wstack,
+                      bool device_call = false) {
     const int nl = wstack ? p->c.wlayer_count : 1;
+    const bool fp32_tc = use_fp32_tc(p, device_call);
+    const WorkItem *items = p->d_gitems.as<WorkItem>();
+    int32_t nitems = static_cast<int32_t>(p->gitems.size());
+    if (fp32_tc) {
+        TRY(ensure_tc(p));
+        items = static_cast<const WorkItem *>(p->tc.gitems);
+        nitems = static_cast<int32_t>(p->tc.gitems_host.size());
+    }
     ZeroSide z{p};
     TRY(z.fork());
-    TRY(grid_items(p, d_vis, vis_c128, p->d_gitems.as<WorkItem>(), static_cast<int32_t>(p->gitems.size())));
+    TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc));
     CK(launch_zero_c64_beside(d_layers, static_cast<int64_t>(nl) * static_cast<int64_t>(nn_of(p)), p->zside));
     TRY(z.join());
-    return add_subgrids(p, d_layers, wstack, nullptr, 0);
+    return add_subgrids(p, d_layers, wstack, nullptr, 0, fp32_tc);
 }
 
 // grid (device complex64) -> vis (device, complex64 or complex128); uncovered samples are 0
@@ -651,7 +668,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.subgrids = p->d_subgrids.as<float2>();
         a.vis_out = d_vis;
         a.out_c128 = out_c128;
-        if (use_tc_degrid(p, out_c128)) {
+        if (use_tc(p) || use_fp32_tc(p, !out_c128)) {
             TRY(ensure_tc(p));
             TRY(tc_degrid(p->tc, a, p->mode, p->stream, g_last_error));
         } else {
@@ -1589,7 +1606,7 @@ p9idg_status p9idg_grid_w_device(p9idg_plan *plan, const void *d_vis, void *d_la
     if (!plan || !d_vis || !d_layers) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(check_wstack_layers(plan));
     TRY(prepare(plan, nullptr));
-    return run_grid(plan, d_vis, false, static_cast<float2 *>(d_layers), true);
+    return run_grid(plan, d_vis, false, static_cast<float2 *>(d_layers), true, true);
 }
 
 p9idg_status p9idg_degrid_w_device(p9idg_plan *plan, const void *d_grid, void *d_vis) {
@@ -1602,7 +1619,7 @@ p9idg_status p9idg_grid_device(p9idg_plan *plan, const void *d_vis, void *d_grid
     if (!plan || !d_vis || !d_grid) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(check_adder_range(plan));
     TRY(prepare(plan, nullptr));
-    return run_grid(plan, d_vis, false, static_cast<float2 *>(d_grid), false);
+    return run_grid(plan, d_vis, false, static_cast<float2 *>(d_grid), false, true);
 }
 
 p9idg_status p9idg_degrid_device(p9idg_plan *plan, const void *d_grid, void *d_vis) {

@@ -37,7 +37,7 @@
 //   MMA1: A_hi x B rows 64-191 (N128) -> cols 0..127 = [T0 | T1];  MMA2: A_hi x B0_lo (N64),
 //   MMA3: A_lo x B0_hi (N64) -> cols 0..63.  Two accumulators alternate (256 columns).
 //
-// FP32 mode (complex64 degridding): the FP16 degridder, expanded about each subgrid's centre dw0
+// FP32 mode (complex64 calls): the FP16 kernels, expanded about each subgrid's centre dw0
 // (the mean of its samples' dw): the pixels are rotated by exp(-i dw0 r) in FP32 as the static
 // operand is made, and T1 is weighted by dw - dw0, which is an order smaller than dw (channels
 // and a short track).  FP16 hi + lo holds 22 bits, so what is left is the two phases' FP32
@@ -46,7 +46,9 @@
 // |dw - dw0| |r| <= 8e-4 the second-order term left out (3e-7 at most, 4e-8 rms over a subgrid's
 // samples and pixels) and the 11 bits of the first-order rows stay below that.
 // 8.0 M visibilities, S = 24: sincos kernel 2.04 ms (bound by the SFUs at 576 sincos per
-// visibility), this form 0.41 ms (48 useful of 64 sincos).
+// visibility), this form 0.41 ms (48 useful of 64 sincos).  The gridder (EX) rotates its sums by
+// exp(i dw0 r) at the end and moves them out of the tensor core's accumulator every stage: 16.0 M
+// visibilities, S = 32, sincos kernel 6.75 ms, this form 1.05 ms, error 3.6e-7 -> 2.7e-7.
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -282,9 +284,9 @@ constexpr uint32_t kGTmemCols = 256;  // the 192 (256) columns of the y rows
 // (fftshifted as Gridder.Forward writes it).  Rows and columns past the plan's S are padding:
 // computed, never written.  SC: the subgrid size when it is the full 32 (compile-time indexing),
 // else 0 and s_rt.
-template <int SC, bool O2>
+template <int SC, bool O2, bool EX>
 __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, int s_rt, int slot, float sv,
-                                               float sw) {
+                                               float sw, float dw0) {
     const int S = SC ? SC : s_rt;
     float ep_r[4], ep_t[4];
 #pragma unroll
@@ -316,15 +318,28 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
             re = fmaf(-h2, pl(2, 0, 0) - pl(2, 1, 1), re);
             im = fmaf(-h2, pl(2, 0, 1) + pl(2, 1, 0), im);
         }
+        if (EX) {  // times exp(i dw0 r): the sums are about the subgrid's centre
+            float sn, cs;
+            sincospif(dw0 * 0.318309886f * rr, &sn, &cs);
+            const float t = re;
+            re = t * cs - im * sn;
+            im = t * sn + im * cs;
+        }
         if (y < S && x < S) out[shift_half(y, S) * S + shift_half(x, S)] = make_float2(re * tap, im * tap);
     }
 }
 
 // O2: the second-order form (|dw r| up to P9IDG_TC_MAX_W_TERM2): y rows 192-255 carry
 // B2 = dw^2 Bh (N = 256), so P = P0 + i r (.) P1 - (r^2 / 2) (.) P2 with P2 = B diag(vis dw^2) A^T.
-template <bool BF16, typename VisT, bool BATCH, bool TMA, bool O2>
+// EX: the FP32 mode (FP16 operands, first order about the subgrid's centre).  The tensor core rounds
+// its accumulator toward zero at every K step, which over a work item of 4096 visibilities costs
+// 2e-5; so the P0 columns hold one stage (4 K steps) at a time: after building the next stage, the
+// producers add them to an FP32 sum kept in columns 192-255 and clear them.  P1, weighted by
+// |dw - dw0| |r| <= 8e-4, stays in the accumulator for the whole item.
+template <bool BF16, typename VisT, bool BATCH, bool TMA, bool O2, bool EX>
 __global__ void __launch_bounds__(kGThreads, 2)
     tc_gridder_kernel(const TcArgs L, const TcArgs *__restrict__ probs, const __grid_constant__ TmaMaps maps) {
+    static_assert(!EX || (!BF16 && !O2 && sizeof(VisT) == 8), "EX: FP16 operands, first order, complex64");
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_1k(smem_raw);
     constexpr uint32_t kGStageBytes = g_stage_bytes(O2);
@@ -334,7 +349,8 @@ __global__ void __launch_bounds__(kGThreads, 2)
     uint64_t *accb = empty + kGStages;
     uint64_t *in_full = accb + 1;
     uint64_t *in_empty = in_full + kGRing;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(in_empty + kGRing);
+    uint64_t *acc_free = in_empty + kGRing;  // EX: the P0 columns are clear for the next stage
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_free + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     float *red = reinterpret_cast<float *>(tmem_slot + 2);
 
@@ -361,6 +377,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
             mbar_init(&in_empty[s], kGProducerWarps);
         }
         mbar_init(accb, 1);
+        mbar_init(acc_free, kGProducerWarps);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -381,7 +398,8 @@ __global__ void __launch_bounds__(kGThreads, 2)
             for (int i = 0; i < nstages; i++) {
                 const int s = i % kGStages;
                 const uint32_t ph = (i / kGStages) & 1;
-                if (!mbar_wait(&full[s], ph, abort_flag, a.wait_ns)) {
+                if (!mbar_wait(&full[s], ph, abort_flag, a.wait_ns) ||
+                    (EX && !mbar_wait(acc_free, i & 1, abort_flag, a.wait_ns))) {
                     *abort_flag = 1;
                     atomicOr(a.status, kStatusWait);
                     break;
@@ -391,7 +409,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
 #pragma unroll
                 for (int kc = 0; kc < kGVps / 16; kc++)
                     mma_f16(tmem, smem_desc(A + kc * 256, 128, kGSbo), smem_desc(B + kc * 256, 128, kGSbo), idn,
-                            (i > 0 || kc > 0) ? 1u : 0u);
+                            (EX || i > 0 || kc > 0) ? 1u : 0u);
                 mma_commit(&empty[s]);
             }
             mma_commit(accb);
@@ -501,9 +519,20 @@ __global__ void __launch_bounds__(kGThreads, 2)
                 const float2 v = load_vis(vrow, j);
                 mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
             }
-            sv = pow2_scale(block256_max(mx, red), 0);
+            sv = pow2_scale(block256_max(mx, red), EX ? 13 : 0);
         }
         const float sw = BF16 ? 1.f : a.dw_scale;
+        // this warp's TMEM lanes (q: the W part, lane = x) and its y columns (u: real or imaginary)
+        const int q = warp & 3, u = warp >> 2;
+        const uint32_t tq = tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(32 * u);
+        if (EX) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) tmem_zero32(tq + static_cast<uint32_t>(64 * k));
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_free);
+        }
         for (int i = 0; i < nstages; i++) {
             const int s = i % kGStages, slot = i % kGRing;
             const uint32_t ph = (i / kGStages) & 1, iph = (i / kGRing) & 1;
@@ -527,7 +556,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
                 }
                 break;
             }
-            const float dws = c.z * sw;
+            const float dws = (EX ? c.w : c.z) * sw;
             // both halves of a packed pair are rows of this lane's visibility: one dw for the pair,
             // and the first-order rows dw * Bh are one packed 16-bit multiply of the hi pair (relative
             // error 2^-8 of a term <= |dw r| <= P9IDG_TC_MAX_W_TERM of the sum: <= 4e-5 at the limit,
@@ -594,6 +623,40 @@ __global__ void __launch_bounds__(kGThreads, 2)
                 mbar_arrive(&full[s]);
                 mbar_arrive(&in_empty[slot]);
             }
+            if (EX && i > 0) {  // the previous stage's P0 columns (hi and lo rows) into the sum
+                if (!warp_wait(&empty[s ^ 1], ((i - 1) / kGStages) & 1, abort_flag, a.wait_ns)) {
+                    if (lane == 0) {
+                        *abort_flag = 1;
+                        atomicOr(a.status, kStatusWait);
+                    }
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint32_t bh[16], bl[16], sum[16];
+                    tmem_ld16(tq + 16 * h, bh);
+                    tmem_ld16(tq + 128 + 16 * h, bl);
+                    tmem_ld16(tq + 192 + 16 * h, sum);
+                    tmem_ld_wait(bh);
+                    tmem_ld_wait(bl);
+                    tmem_ld_wait(sum);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) {
+                        auto two = [j](const uint32_t *t) { return make_float2(__uint_as_float(t[j]), __uint_as_float(t[j + 1])); };
+                        const float2 v = __fadd2_rn(two(sum), __fadd2_rn(two(bh), two(bl)));
+                        sum[j] = __float_as_uint(v.x);
+                        sum[j + 1] = __float_as_uint(v.y);
+                    }
+                    tmem_st16(tq + 192 + 16 * h, sum);
+                }
+                tmem_zero32(tq);
+                tmem_zero32(tq + 128);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_free);
+            }
         }
         // ---- epilogue: TMEM -> smem planes -> partial subgrid
         const bool ok = warp_wait(accb, 0, abort_flag, a.wait_ns);
@@ -602,27 +665,31 @@ __global__ void __launch_bounds__(kGThreads, 2)
         // warp: TMEM lane quarter q (the W rows Wh_re, Wh_im, Wl_re, Wl_im; lane = x) against the real
         // (u = 0) or imaginary (u = 1) y rows: plane kind * 8 + 2 q + u holds [y][x] of
         // kind 0: (Bh + Bl) columns, 1: B1, 2: B2
-        const int q = warp & 3, u = warp >> 2;
         if (ok) {
             uint32_t r[32];
-            const uint32_t t = tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(32 * u);
             float *e0 = E + (2 * q + u) * 1056 + lane;
-            tmem_ld32(t, r);  // Bh_u
+            tmem_ld32(tq, r);  // Bh_u
             tmem_ld_wait(r);
 #pragma unroll
             for (int j = 0; j < 32; j++) e0[j * 33] = __uint_as_float(r[j]);
-            tmem_ld32(t + 128, r);  // Bl_u
+            tmem_ld32(tq + 128, r);  // Bl_u
             tmem_ld_wait(r);
 #pragma unroll
             for (int j = 0; j < 32; j++) e0[j * 33] += __uint_as_float(r[j]);
+            if (EX) {
+                tmem_ld32(tq + 192, r);  // the earlier stages
+                tmem_ld_wait(r);
+#pragma unroll
+                for (int j = 0; j < 32; j++) e0[j * 33] += __uint_as_float(r[j]);
+            }
             float *e1 = E + (8 + 2 * q + u) * 1056 + lane;
-            tmem_ld32(t + 64, r);  // B1_u
+            tmem_ld32(tq + 64, r);  // B1_u
             tmem_ld_wait(r);
 #pragma unroll
             for (int j = 0; j < 32; j++) e1[j * 33] = __uint_as_float(r[j]);
             if (O2) {
                 float *e2 = E + (16 + 2 * q + u) * 1056 + lane;
-                tmem_ld32(t + 192, r);  // B2_u
+                tmem_ld32(tq + 192, r);  // B2_u
                 tmem_ld_wait(r);
 #pragma unroll
                 for (int j = 0; j < 32; j++) e2[j * 33] = __uint_as_float(r[j]);
@@ -631,10 +698,11 @@ __global__ void __launch_bounds__(kGThreads, 2)
         tc_fence_before();
         named_bar(1, kGProducerWarps * 32);
         if (ok && !*abort_flag) {
+            const float dw0 = EX ? a.center[it.subgrid] : 0.f;
             if (g.S == kS)  // the full size with compile-time indexing, smaller subgrids padded
-                gridder_finish<kS, O2>(a, E, g.S, it.slot, sv, sw);
+                gridder_finish<kS, O2, EX>(a, E, g.S, it.slot, sv, sw, dw0);
             else
-                gridder_finish<0, O2>(a, E, g.S, it.slot, sv, sw);
+                gridder_finish<0, O2, EX>(a, E, g.S, it.slot, sv, sw, dw0);
         }
     }
     tc_fence_before();
@@ -1269,13 +1337,19 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     std::vector<DevSubgrid> dtmp;
     std::vector<WorkItem> ditems;
     build_work_items(subs, nch, st.degrid_chunk, dtmp, ditems);
+    // gridder work items of the FP32 mode's form (the other modes use the plan's own)
+    std::vector<DevSubgrid> gsubs;
+    std::vector<WorkItem> gitems;
+    if (st.grid_chunk > 0) build_work_items(subs, nch, st.grid_chunk, gsubs, gitems);
     st.ncoef = off.back();
     cudaError_t e;
     if ((e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef))) != cudaSuccess ||
         (e = device_alloc(&st.coef_off, sizeof(int64_t) * off.size())) != cudaSuccess ||
         (e = device_alloc(&st.center, sizeof(float) * std::max<size_t>(1, subs.size()))) != cudaSuccess ||
         (e = device_alloc(&st.tables, sizeof(float) * tabs.size())) != cudaSuccess ||
-        (e = device_alloc(&st.ditems, sizeof(WorkItem) * std::max<size_t>(1, ditems.size()))) != cudaSuccess) {
+        (e = device_alloc(&st.ditems, sizeof(WorkItem) * std::max<size_t>(1, ditems.size()))) != cudaSuccess ||
+        (st.grid_chunk > 0 && ((e = device_alloc(&st.gitems, sizeof(WorkItem) * std::max<size_t>(1, gitems.size()))) != cudaSuccess ||
+                               (e = device_alloc(&st.gsubs, sizeof(DevSubgrid) * std::max<size_t>(1, gsubs.size()))) != cudaSuccess))) {
         err = std::string("tensor-core buffers: ") + cudaGetErrorString(e);
         tc_release(st);
         return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
@@ -1284,12 +1358,18 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     cudaMemcpyAsync(st.tables, tabs.data(), sizeof(float) * tabs.size(), cudaMemcpyHostToDevice, stream);
     if (!ditems.empty())
         cudaMemcpyAsync(st.ditems, ditems.data(), sizeof(WorkItem) * ditems.size(), cudaMemcpyHostToDevice, stream);
+    if (!gitems.empty()) {
+        cudaMemcpyAsync(st.gitems, gitems.data(), sizeof(WorkItem) * gitems.size(), cudaMemcpyHostToDevice, stream);
+        cudaMemcpyAsync(st.gsubs, gsubs.data(), sizeof(DevSubgrid) * gsubs.size(), cudaMemcpyHostToDevice, stream);
+    }
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) {
         err = std::string("tensor-core tables: ") + cudaGetErrorString(e);
         return P9IDG_CUDA_ERROR;
     }
     st.nditems = static_cast<int32_t>(ditems.size());
     st.ditems_host = ditems;
+    st.gitems_host = gitems;
+    st.nslots = static_cast<int32_t>(gitems.size());
     st.S = S;
     st.ready = true;
     return P9IDG_OK;
@@ -1316,12 +1396,12 @@ static p9idg_status launch_coef(TcPlanState &st, const GridderArgs &a, int32_t n
 
 namespace {
 
-template <bool BF16, typename VisT, bool BATCH, bool TMA, bool O2>
+template <bool BF16, typename VisT, bool BATCH, bool TMA, bool O2, bool EX = false>
 cudaError_t run_gridder(const TcArgs &t, const TcArgs *probs, int32_t nitems, const TmaMaps &maps,
                         cudaStream_t stream) {
-    cudaError_t e = set_smem(tc_gridder_kernel<BF16, VisT, BATCH, TMA, O2>, g_smem(O2));
+    cudaError_t e = set_smem(tc_gridder_kernel<BF16, VisT, BATCH, TMA, O2, EX>, g_smem(O2));
     if (e == cudaSuccess)
-        tc_gridder_kernel<BF16, VisT, BATCH, TMA, O2><<<nitems, kGThreads, g_smem(O2), stream>>>(t, probs, maps);
+        tc_gridder_kernel<BF16, VisT, BATCH, TMA, O2, EX><<<nitems, kGThreads, g_smem(O2), stream>>>(t, probs, maps);
     return e;
 }
 
@@ -1346,8 +1426,18 @@ p9idg_status launch_tc_gridder(const TcArgs &t, const TcArgs *probs, int32_t nit
     const TmaMaps &m = maps ? *maps : kNoMaps;
     cudaError_t e = cudaSuccess;
     bool done = false;
+    if constexpr (!O2) {
+        if (mode == P9IDG_MODE_FP32) {  // complex64 only
+            if constexpr (!BATCH)
+                e = maps ? run_gridder<false, float2, false, true, false, true>(t, probs, nitems, m, stream)
+                         : run_gridder<false, float2, false, false, false, true>(t, probs, nitems, m, stream);
+            else
+                e = run_gridder<false, float2, true, false, false, true>(t, probs, nitems, m, stream);
+            done = true;
+        }
+    }
     if constexpr (!BATCH) {
-        if (maps && !c128) {
+        if (!done && maps && !c128) {
             e = bf16 ? run_gridder<true, float2, false, true, O2>(t, probs, nitems, m, stream)
                      : run_gridder<false, float2, false, true, O2>(t, probs, nitems, m, stream);
             done = true;
@@ -1529,6 +1619,8 @@ void tc_release(TcPlanState &st) {
     if (st.center) cudaFree(st.center);
     if (st.tables) cudaFree(st.tables);
     if (st.ditems) cudaFree(st.ditems);
+    if (st.gitems) cudaFree(st.gitems);
+    if (st.gsubs) cudaFree(st.gsubs);
     st = TcPlanState();
 }
 

@@ -25,6 +25,12 @@ struct TcPlanState {
     void *ditems = nullptr;       // degridder work items (<= degrid_chunk visibilities)
     int32_t nditems = 0;
     std::vector<WorkItem> ditems_host;  // the same list on the host (batches merge them)
+    // FP32 mode: its own gridder work items (<= grid_chunk visibilities; 0: none) and the subgrid list
+    // that records their slots
+    int64_t grid_chunk = 0;
+    void *gitems = nullptr, *gsubs = nullptr;
+    std::vector<WorkItem> gitems_host;
+    int32_t nslots = 0;                 // partial-subgrid slots of those items (one each)
     int64_t degrid_chunk = 16384;       // visibilities per degridder work item (set before tc_prepare)
     double max_w_r = 0;           // max |dw| * max |r|: bound on the phase the form expands
     double r_max = 0;             // max |r| of the centred remainder table

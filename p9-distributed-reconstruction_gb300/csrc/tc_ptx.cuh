@@ -222,5 +222,30 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16]) {
                  : "memory");
 }
 
+// ---- tcgen05: registers -> TMEM (32 lanes x 16 / 32 columns), and the wait for this thread's stores.
+// Every lane of the warp must call them.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    __syncwarp();
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .b32 z;\n\tmov.b32 z, 0;\n\t"
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z, z};\n\t}" ::"r"(
+            taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() {
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 }  // namespace tc
 }  // namespace p9idg

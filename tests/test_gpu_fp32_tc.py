@@ -55,3 +55,16 @@ def test_degrid(need_gpu, S, kernel, nch, nt, N, chunks):
     host = pkg.IDG.DeGridW(c, part, model.astype(np.complex128), obs.uvw, obs.frequencies)
     ref, _ = oracle.idg_degrid(cd, subs, model.astype(np.complex128), obs.uvw, obs.frequencies, wstack=True)
     _no_further_off(d_out.cpu().numpy(), host, ref)
+
+
+@pytest.mark.parametrize("S,kernel,nch,nt,N,chunks", SHAPES)
+def test_grid(need_gpu, S, kernel, nch, nt, N, chunks):
+    obs, c, cd, part, subs = _setup(S, kernel, nch, nt, N, chunks)
+    vis = obs.vis.astype(np.complex64)
+    d_vis = torch.from_numpy(vis).cuda()
+    d_layers = torch.full((cd["wlayer_count"], N, N), float("nan"), dtype=torch.complex64, device="cuda")
+    part.plan.grid_w_device(d_vis.data_ptr(), d_layers.data_ptr())
+    part.plan.synchronize()
+    host = pkg.IDG.GridW(c, part, vis.astype(np.complex128), obs.uvw, obs.frequencies)
+    ref = oracle.idg_grid_w(cd, subs, vis.astype(np.complex128), obs.uvw, obs.frequencies)
+    _no_further_off(d_layers.cpu().numpy(), host, ref)
