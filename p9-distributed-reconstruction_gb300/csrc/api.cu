@@ -486,14 +486,13 @@ GridderArgs gridder_args(p9idg_plan *p) {
 }
 
 p9idg_status ensure_tc(p9idg_plan *p) {
-    if (p->tc.ready) {
-        tc_set_order(p->tc, p->mode, p->tc.want_order);
-        return P9IDG_OK;
-    }
     // degridder items do not accumulate across visibilities: 16384 measured 1.6 % faster than 8192
-    // (32768 the same as 16384), 8192 3.5 % faster than 4096
-    p->tc.degrid_chunk = p->dchunk > 0 ? p->dchunk : 16384;
-    p->tc.grid_chunk = p->fp32_tc ? (p->gchunk > 0 ? p->gchunk : 4096) : 0;
+    // (32768 the same as 16384), 8192 3.5 % faster than 4096.  The FP32 mode's sizes (1024 and 512 by
+    // default) are its sincos kernels' work items; its tensor-core form takes 4 and 32 times as many
+    // visibilities, the other modes' defaults.
+    const int64_t scale = p->mode == P9IDG_MODE_FP32 ? 32 : 1;
+    p->tc.degrid_chunk = p->dchunk > 0 ? scale * p->dchunk : 16384;
+    p->tc.grid_chunk = p->mode == P9IDG_MODE_FP32 ? (p->gchunk > 0 ? 4 * static_cast<int64_t>(p->gchunk) : 4096) : 0;
     TRY(tc_prepare(p->tc, p->subs, p->lmn, p->c.subgrid_size, p->nch, p->dw_max, p->stream, g_last_error));
     tc_set_order(p->tc, p->mode, p->tc.want_order);
     return P9IDG_OK;
@@ -1118,13 +1117,16 @@ struct p9idg_batch {
     int32_t mode = P9IDG_MODE_FP32;
     cudaStream_t stream = nullptr;
     DevBuf d_gargs, d_dargs, d_aargs, d_sargs, d_tg, d_td;  // per-problem argument tables
-    DevBuf d_gitems, d_ditems, d_refs, d_done_init, d_done, d_finish, d_start;
+    DevBuf d_gitems, d_ditems, d_subs, d_refs, d_done_init, d_done, d_finish, d_start;
     int32_t ngitems = 0, nditems = 0, nrefs = 0;
     std::vector<WorkItem> h_gitems, h_ditems;  // merged work items of all problems, in launch order
-    // problems may mix subgrid sizes: the items and subgrid references are grouped by size,
-    // one launch per kernel stage and size (group k: items [g0, g0 + gn), [d0, d0 + dn), refs [r0, r0 + rn))
+    // problems may mix subgrid sizes, and FP32 ones the two forms of that mode: the items and subgrid
+    // references are grouped by size and form, one launch per kernel stage and group (group k: items
+    // [g0, g0 + gn), [d0, d0 + dn), refs [r0, r0 + rn))
     struct Group {
-        int32_t S, g0, gn, d0, dn, r0, rn;
+        int32_t key, S;
+        bool tc;
+        int32_t g0, gn, d0, dn, r0, rn;
     };
     std::vector<Group> groups;
     int tc_order = 1;  // tensor-core batches: 2 when any plan needs the second-order form
@@ -1138,6 +1140,10 @@ struct p9idg_batch {
 
 namespace {
 
+// Whether a plan's batch launches run on the tensor cores, and the group it belongs to.
+bool batch_tc(const p9idg_plan *p) { return use_tc(p) || use_fp32_tc(p, true); }
+int32_t group_key(const p9idg_plan *p) { return 2 * p->c.subgrid_size + (batch_tc(p) ? 1 : 0); }
+
 __global__ void stamp_kernel(unsigned long long *t) { *t = device_ns(); }
 
 p9idg_status batch_grid(p9idg_batch *b) {
@@ -1148,7 +1154,7 @@ p9idg_status batch_grid(p9idg_batch *b) {
         L.g.S = g.S;
         L.items = b->d_gitems.as<WorkItem>() + g.g0;
         L.nitems = g.gn;
-        if (b->mode == P9IDG_MODE_FP32) {
+        if (!g.tc) {
             if (g.gn > 0) CK(launch_gridder_fp32(L, b->stream, b->d_gargs.as<GridderArgs>()));
         } else {
             TRY(tc_grid_batch(b->d_tg.as<TcArgs>(), L.items, g.gn, b->mode, b->tc_order, b->stream, g_last_error));
@@ -1185,7 +1191,7 @@ p9idg_status batch_degrid(p9idg_batch *b) {
         L.g.S = g.S;
         L.items = b->d_ditems.as<WorkItem>() + g.d0;
         L.nitems = g.dn;
-        if (b->mode == P9IDG_MODE_FP32) {
+        if (!g.tc) {
             if (g.dn > 0) CK(launch_degridder_fp32(L, b->stream, b->d_dargs.as<GridderArgs>()));
         } else {
             TRY(tc_degrid_batch(b->d_td.as<TcArgs>(), L.items, g.dn, b->mode, b->tc_order, b->stream,
@@ -1214,26 +1220,26 @@ p9idg_status batch_order(p9idg_batch *b, int32_t schedule) {
             return pv[x.problem] != pv[y.problem] ? pv[x.problem] < pv[y.problem] : x.problem < y.problem;
         return item_vis(x) > item_vis(y);
     };
-    auto size_of = [&](const WorkItem &w) { return b->plans[w.problem]->c.subgrid_size; };
+    auto key_of = [&](const WorkItem &w) { return group_key(b->plans[w.problem]); };
     for (auto *v : {&b->h_gitems, &b->h_ditems}) {
         if (schedule == P9IDG_SCHEDULE_SMALL_FIRST)
             std::stable_sort(v->begin(), v->end(), small_first);
         else
             std::stable_sort(v->begin(), v->end(), throughput);
-        // one launch per subgrid size: the items of each size contiguous, in size order
+        // one launch per group: the items of each contiguous, in group order
         std::stable_sort(v->begin(), v->end(),
-                         [&](const WorkItem &x, const WorkItem &y) { return size_of(x) < size_of(y); });
+                         [&](const WorkItem &x, const WorkItem &y) { return key_of(x) < key_of(y); });
     }
     for (auto &g : b->groups) {
         g.g0 = g.gn = g.d0 = g.dn = 0;
         bool gs = false, ds = false;
         for (size_t k = 0; k < b->h_gitems.size(); k++)
-            if (size_of(b->h_gitems[k]) == g.S) {
+            if (key_of(b->h_gitems[k]) == g.key) {
                 if (!gs) g.g0 = static_cast<int32_t>(k), gs = true;
                 g.gn++;
             }
         for (size_t k = 0; k < b->h_ditems.size(); k++)
-            if (size_of(b->h_ditems[k]) == g.S) {
+            if (key_of(b->h_ditems[k]) == g.key) {
                 if (!ds) g.d0 = static_cast<int32_t>(k), ds = true;
                 g.dn++;
             }
@@ -1248,7 +1254,7 @@ void batch_release(p9idg_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     DevBuf *bufs[] = {&b->d_gargs, &b->d_dargs, &b->d_aargs, &b->d_sargs, &b->d_tg, &b->d_td, &b->d_gitems,
-                      &b->d_ditems, &b->d_refs, &b->d_done_init, &b->d_done, &b->d_finish, &b->d_start};
+                      &b->d_ditems, &b->d_subs, &b->d_refs, &b->d_done_init, &b->d_done, &b->d_finish, &b->d_start};
     for (DevBuf *x : bufs) x->release();
     if (b->stream) cudaStreamDestroy(b->stream);
 }
@@ -1717,14 +1723,7 @@ p9idg_status p9idg_plan_set_chunking(p9idg_plan *plan, int32_t gridder_max_vis, 
     plan->gchunk = gridder_max_vis;
     plan->dchunk = degridder_max_vis;
     build_gridder_items(plan);
-    if (plan->tc.ready) {
-        if (plan->dev_ready) {
-            CK(cudaSetDevice(plan->device));
-            CK(cudaStreamSynchronize(plan->stream));
-        }
-        tc_release(plan->tc);  // rebuilt (with the new degridder items) on the next tensor-core call
-    }
-    return P9IDG_OK;
+    return P9IDG_OK;  // the tensor-core items are rebuilt on the next tensor-core call (ensure_tc)
 }
 
 p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const void *const *d_vis,
@@ -1752,6 +1751,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     std::vector<SubgridOpArgs> aa(nplans), sa(nplans);
     std::vector<TcArgs> tg(nplans), td(nplans);
     std::vector<WorkItem> gitems, ditems;
+    std::vector<DevSubgrid> subs;
     std::vector<int2> refs;
     std::vector<int32_t> done(nplans, 0);
     // device-side completion tracking first: the argument tables point into it
@@ -1775,7 +1775,10 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     for (int i = 0; i < nplans; i++) {
         p9idg_plan *p = plans[i];
         const int S = p->c.subgrid_size;
-        cudaError_t e = p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->nslots));
+        const bool tc = batch_tc(p), fp32_tc = use_fp32_tc(p, true);
+        if (tc && (st = ensure_tc(p)) != P9IDG_OK) return bail(st);
+        cudaError_t e = p->d_partials.ensure(sizeof(float2) * S * S *
+                                             std::max<size_t>(1, fp32_tc ? p->tc.nslots : p->nslots));
         if (e == cudaSuccess) e = p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size()));
         if (e != cudaSuccess) return bail(cuda_fail(e, "plan buffers"));
         ga[i] = gridder_args(p);
@@ -1789,6 +1792,11 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         da[i].done = b->d_done.as<int32_t>() + i;
         da[i].finish_ns = b->d_finish.as<unsigned long long>() + i;
         aa[i] = subgrid_args(p);
+        // the subgrids with the slots of the items this batch runs: its own copy, as the plan's changes with
+        // its work-item sizes (an offset here, the address once all are known)
+        aa[i].subs = reinterpret_cast<const DevSubgrid *>(sizeof(DevSubgrid) * subs.size());
+        const std::vector<DevSubgrid> &slots = fp32_tc ? p->tc.gsubs_host : p->dsub;
+        subs.insert(subs.end(), slots.begin(), slots.end());
         aa[i].partials = p->d_partials.as<float2>();
         aa[i].layers = static_cast<float2 *>(d_layers[i]);
         aa[i].out_shifted = true;
@@ -1798,16 +1806,15 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         sa[i].grid_shifted = false;
         sa[i].subgrids = p->d_subgrids.as<float2>();
         sa[i].wstack = true;
-        const std::vector<WorkItem> *dsrc = &p->ditems;
-        if (b->mode != P9IDG_MODE_FP32) {
-            if ((st = ensure_tc(p)) != P9IDG_OK) return bail(st);
+        const std::vector<WorkItem> *dsrc = &p->ditems, *gsrc = fp32_tc ? &p->tc.gitems_host : &p->gitems;
+        if (tc) {
             b->tc_order = std::max(b->tc_order, p->tc.order);
             if ((st = tc_coefs(p->tc, ga[i], p->stream, g_last_error)) != P9IDG_OK) return bail(st);
             tc_fill_args(p->tc, ga[i], tg[i]);
             tc_fill_args(p->tc, da[i], td[i]);
             dsrc = &p->tc.ditems_host;
         }
-        for (WorkItem w : p->gitems) {
+        for (WorkItem w : *gsrc) {
             w.problem = i;
             gitems.push_back(w);
         }
@@ -1818,8 +1825,8 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         done[i] = static_cast<int32_t>(dsrc->size());
         for (size_t s = 0; s < p->dsub.size(); s++) refs.push_back(make_int2(i, static_cast<int>(s)));
         bool known = false;
-        for (const auto &g : b->groups) known |= g.S == S;
-        if (!known) b->groups.push_back({S, 0, 0, 0, 0, 0, 0});
+        for (const auto &g : b->groups) known |= g.key == group_key(p);
+        if (!known) b->groups.push_back({group_key(p), S, tc, 0, 0, 0, 0, 0, 0});
         b->layers.push_back(d_layers[i]);
         b->layer_bytes.push_back(sizeof(float2) * static_cast<size_t>(p->c.wlayer_count) * nn_of(p));
         b->vis_out.push_back(d_vis_out[i]);
@@ -1828,16 +1835,15 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         if (e2 != cudaSuccess) return bail(cuda_fail(e2, "plan preparation"));
     }
     std::sort(b->groups.begin(), b->groups.end(),
-              [](const p9idg_batch::Group &x, const p9idg_batch::Group &y) { return x.S < y.S; });
-    // subgrid references grouped by size (plan order inside a group)
-    std::stable_sort(refs.begin(), refs.end(), [&](const int2 &x, const int2 &y) {
-        return plans[x.x]->c.subgrid_size < plans[y.x]->c.subgrid_size;
-    });
+              [](const p9idg_batch::Group &x, const p9idg_batch::Group &y) { return x.key < y.key; });
+    // subgrid references grouped the same way (plan order inside a group)
+    std::stable_sort(refs.begin(), refs.end(),
+                     [&](const int2 &x, const int2 &y) { return group_key(plans[x.x]) < group_key(plans[y.x]); });
     for (auto &g : b->groups) {
         g.r0 = g.rn = 0;
         bool rs = false;
         for (size_t k = 0; k < refs.size(); k++)
-            if (plans[refs[k].x]->c.subgrid_size == g.S) {
+            if (group_key(plans[refs[k].x]) == g.key) {
                 if (!rs) g.r0 = static_cast<int32_t>(k), rs = true;
                 g.rn++;
             }
@@ -1849,6 +1855,9 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     b->ngitems = static_cast<int32_t>(b->h_gitems.size());
     b->nditems = static_cast<int32_t>(b->h_ditems.size());
     b->nrefs = static_cast<int32_t>(refs.size());
+    if ((st = upload(b->d_subs, subs)) != P9IDG_OK) return bail(st);
+    for (auto &x : aa)
+        x.subs = reinterpret_cast<const DevSubgrid *>(b->d_subs.as<char>() + reinterpret_cast<uintptr_t>(x.subs));
     if ((st = upload(b->d_gargs, ga)) != P9IDG_OK || (st = upload(b->d_dargs, da)) != P9IDG_OK ||
         (st = upload(b->d_aargs, aa)) != P9IDG_OK || (st = upload(b->d_sargs, sa)) != P9IDG_OK ||
         (st = upload(b->d_tg, tg)) != P9IDG_OK || (st = upload(b->d_td, td)) != P9IDG_OK ||

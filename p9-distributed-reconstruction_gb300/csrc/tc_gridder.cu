@@ -1305,16 +1305,55 @@ double tc_r_max(const std::vector<float> &lmn, int S) {
     return separable_tables(lmn, S, tabs);
 }
 
+// The work items for the sizes asked for: degridder items (whole time samples, up to degrid_chunk
+// visibilities each) and, with a grid_chunk, the FP32 mode's gridder items.
+static p9idg_status tc_items(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, int nch, cudaStream_t stream,
+                             std::string &err) {
+    if (st.items_degrid == st.degrid_chunk && (st.grid_chunk <= 0 || st.items_grid == st.grid_chunk)) return P9IDG_OK;
+    cudaError_t e = cudaStreamSynchronize(stream);  // launches in flight read the lists replaced here
+    for (void **q : {&st.ditems, &st.gitems, &st.gsubs}) {
+        if (*q) cudaFree(*q);
+        *q = nullptr;
+    }
+    st.items_degrid = st.items_grid = -1;
+    std::vector<DevSubgrid> dtmp;
+    build_work_items(subs, nch, st.degrid_chunk, dtmp, st.ditems_host);
+    st.gsubs_host.clear();
+    st.gitems_host.clear();
+    if (st.grid_chunk > 0) build_work_items(subs, nch, st.grid_chunk, st.gsubs_host, st.gitems_host);
+    const auto put = [&](void **dst, const auto &v) {
+        using T = typename std::decay<decltype(v)>::type::value_type;
+        if (e == cudaSuccess) e = device_alloc(dst, sizeof(T) * std::max<size_t>(1, v.size()));
+        if (e == cudaSuccess && !v.empty())
+            e = cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream);
+    };
+    put(&st.ditems, st.ditems_host);
+    if (st.grid_chunk > 0) {
+        put(&st.gitems, st.gitems_host);
+        put(&st.gsubs, st.gsubs_host);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) {
+        err = std::string("tensor-core work items: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
+    }
+    st.nditems = static_cast<int32_t>(st.ditems_host.size());
+    st.nslots = static_cast<int32_t>(st.gitems_host.size());
+    st.items_degrid = st.degrid_chunk;
+    st.items_grid = st.grid_chunk;
+    return P9IDG_OK;
+}
+
 p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn,
                         int S, int nch, double dw_max, cudaStream_t stream, std::string &err) {
-    if (st.ready) return P9IDG_OK;
+    if (st.ready) return tc_items(st, subs, nch, stream, err);
     if (!tc_subgrid_size_supported(S)) {
         err = "tensor-core kernels support subgrid sizes 8, 16, 24 and 32";
         return P9IDG_UNSUPPORTED;
     }
     std::vector<float> tabs;
     const double rmax = separable_tables(lmn, S, tabs);
-    // coefficient offsets per subgrid and the largest |dw|
+    // coefficient offsets per subgrid
     std::vector<int64_t> off(subs.size() + 1, 0);
     for (size_t i = 0; i < subs.size(); i++)
         off[i + 1] = off[i] + static_cast<int64_t>(subs[i].time_sample_count) * nch;
@@ -1333,46 +1372,25 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     };
     st.dw_scale = pow2_below(dw_max * 1.0001);
     st.r_scale = pow2_below(rmax);
-    // degridder work items: whole time samples, up to degrid_chunk visibilities each
-    std::vector<DevSubgrid> dtmp;
-    std::vector<WorkItem> ditems;
-    build_work_items(subs, nch, st.degrid_chunk, dtmp, ditems);
-    // gridder work items of the FP32 mode's form (the other modes use the plan's own)
-    std::vector<DevSubgrid> gsubs;
-    std::vector<WorkItem> gitems;
-    if (st.grid_chunk > 0) build_work_items(subs, nch, st.grid_chunk, gsubs, gitems);
     st.ncoef = off.back();
     cudaError_t e;
     if ((e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef))) != cudaSuccess ||
         (e = device_alloc(&st.coef_off, sizeof(int64_t) * off.size())) != cudaSuccess ||
         (e = device_alloc(&st.center, sizeof(float) * std::max<size_t>(1, subs.size()))) != cudaSuccess ||
-        (e = device_alloc(&st.tables, sizeof(float) * tabs.size())) != cudaSuccess ||
-        (e = device_alloc(&st.ditems, sizeof(WorkItem) * std::max<size_t>(1, ditems.size()))) != cudaSuccess ||
-        (st.grid_chunk > 0 && ((e = device_alloc(&st.gitems, sizeof(WorkItem) * std::max<size_t>(1, gitems.size()))) != cudaSuccess ||
-                               (e = device_alloc(&st.gsubs, sizeof(DevSubgrid) * std::max<size_t>(1, gsubs.size()))) != cudaSuccess))) {
+        (e = device_alloc(&st.tables, sizeof(float) * tabs.size())) != cudaSuccess) {
         err = std::string("tensor-core buffers: ") + cudaGetErrorString(e);
         tc_release(st);
         return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
     }
     cudaMemcpyAsync(st.coef_off, off.data(), sizeof(int64_t) * off.size(), cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(st.tables, tabs.data(), sizeof(float) * tabs.size(), cudaMemcpyHostToDevice, stream);
-    if (!ditems.empty())
-        cudaMemcpyAsync(st.ditems, ditems.data(), sizeof(WorkItem) * ditems.size(), cudaMemcpyHostToDevice, stream);
-    if (!gitems.empty()) {
-        cudaMemcpyAsync(st.gitems, gitems.data(), sizeof(WorkItem) * gitems.size(), cudaMemcpyHostToDevice, stream);
-        cudaMemcpyAsync(st.gsubs, gsubs.data(), sizeof(DevSubgrid) * gsubs.size(), cudaMemcpyHostToDevice, stream);
-    }
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) {
         err = std::string("tensor-core tables: ") + cudaGetErrorString(e);
         return P9IDG_CUDA_ERROR;
     }
-    st.nditems = static_cast<int32_t>(ditems.size());
-    st.ditems_host = ditems;
-    st.gitems_host = gitems;
-    st.nslots = static_cast<int32_t>(gitems.size());
     st.S = S;
     st.ready = true;
-    return P9IDG_OK;
+    return tc_items(st, subs, nch, stream, err);
 }
 
 // Per-visibility phase coefficients depend only on the plan and uvw: computed once and kept

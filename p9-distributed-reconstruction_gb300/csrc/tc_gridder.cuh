@@ -30,6 +30,8 @@ struct TcPlanState {
     int64_t grid_chunk = 0;
     void *gitems = nullptr, *gsubs = nullptr;
     std::vector<WorkItem> gitems_host;
+    std::vector<DevSubgrid> gsubs_host;
+    int64_t items_degrid = -1, items_grid = -1;  // the sizes the lists now on the device were made for
     int32_t nslots = 0;                 // partial-subgrid slots of those items (one each)
     int64_t degrid_chunk = 16384;       // visibilities per degridder work item (set before tc_prepare)
     double max_w_r = 0;           // max |dw| * max |r|: bound on the phase the form expands
@@ -99,7 +101,8 @@ int tc_order_for(double w_term, int want_order);
 // Selects the form of a prepared state for the plan's mode (no device work): the FP32 mode always
 // runs the first-order form about the subgrids' centres.
 void tc_set_order(TcPlanState &st, int mode, int want_order);
-// Builds the tables and uploads them (once per plan); dw_max = max |k| * max |w| of its samples.
+// Builds the tables and uploads them (once per plan), and the work items (again when degrid_chunk or
+// grid_chunk changed); dw_max = max |k| * max |w| of its samples.
 // The caller selects the form (tc_set_order) before it launches.
 p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, const std::vector<float> &lmn,
                         int S, int nch, double dw_max, cudaStream_t stream, std::string &err);
