@@ -71,16 +71,18 @@ struct DevBuf {
 };
 
 struct FftCache {
+    cufftType type;
     cufftHandle h = 0;
     int n = 0;
     cudaStream_t st = nullptr;
+    explicit FftCache(cufftType t = CUFFT_C2C) : type(t) {}
     p9idg_status get(int size, cudaStream_t stream, cufftHandle *out) {
         if (h && n != size) {
             cufftDestroy(h);
             h = 0;
         }
         if (!h) {
-            if (cufftPlan2d(&h, size, size, CUFFT_C2C) != CUFFT_SUCCESS) {
+            if (cufftPlan2d(&h, size, size, type) != CUFFT_SUCCESS) {
                 h = 0;
                 return fail(P9IDG_CUDA_ERROR, "cufftPlan2d failed");
             }
@@ -171,7 +173,7 @@ struct p9idg_plan {
     DevBuf d_partials, d_subgrids, d_vis_in, d_vis_out, d_layers, d_out128, d_grid128, d_grid128b, d_grid64,
         d_flags, d_image;
     TcPlanState tc;
-    FftCache fft;
+    FftCache fft, fft_real{CUFFT_C2R};
     // Host arrays used in place by the kernels (device reads/writes host memory through the host's
     // page tables, e.g. NVLink-C2C on Grace systems) instead of staged through device copies.
     bool host_direct = false;   // the device can access any host address
@@ -1079,6 +1081,37 @@ p9idg_status image_from_grid(p9idg_plan *p, float2 *d_grid, double norm, bool sh
     return P9IDG_OK;
 }
 
+// FFT.WStackIFFTFloat (and the caller's FFT.Shift when shift is set) of nlayers n x n layers, by a
+// complex-to-real transform of their sum's half plane where cuFFT has it in two passes (an even n with
+// no prime factor above 7) and can write the image itself (a count to divide by, an aligned address),
+// else by a complex transform and its real part.  8 layers of 3072^2: 0.280 ms complex, 0.220 ms real;
+// 689^2, where the real transform takes four passes: 0.051 against 0.058 ms.
+p9idg_status layers_to_image(const void *layers, bool c128, int nlayers, int n, int64_t vis_count, bool shift,
+                             FftCache &fft, FftCache &fft_real, DevBuf &grid, float *d_image, cudaStream_t st) {
+    int rest = n;
+    for (int p : {2, 3, 5, 7})
+        while (rest % p == 0) rest /= p;
+    const bool real = n % 2 == 0 && rest == 1 && vis_count != 0 && (reinterpret_cast<uintptr_t>(d_image) & 15) == 0;
+    const size_t nn = static_cast<size_t>(n) * n;
+    cufftHandle h;
+    if (real) {
+        CK(grid.ensure(sizeof(float2) * static_cast<size_t>(n) * (n / 2 + 1)));
+        CK(launch_layer_half(layers, c128, nlayers, n, 1.0 / static_cast<double>(vis_count), shift, grid.as<float2>(),
+                             st));
+        TRY(fft_real.get(n, st, &h));
+        if (cufftExecC2R(h, grid.as<cufftComplex>(), d_image) != CUFFT_SUCCESS)
+            return fail(P9IDG_CUDA_ERROR, "cufftExecC2R failed");
+        return P9IDG_OK;
+    }
+    CK(grid.ensure(sizeof(float2) * nn));
+    CK(launch_layer_sum(layers, c128, nlayers, static_cast<int64_t>(nn), grid.as<float2>(), st));
+    TRY(fft.get(n, st, &h));
+    if (cufftExecC2C(h, grid.as<cufftComplex>(), grid.as<cufftComplex>(), CUFFT_INVERSE) != CUFFT_SUCCESS)
+        return fail(P9IDG_CUDA_ERROR, "cufftExecC2C failed");
+    CK(launch_real_part(grid.as<float2>(), n, static_cast<double>(vis_count), shift, d_image, nullptr, st));
+    return P9IDG_OK;
+}
+
 // ---------- plan-less FFT helpers (FFT.cs entry points) ----------
 
 struct Standalone {
@@ -1087,7 +1120,7 @@ struct Standalone {
     int device = -1;
     cudaStream_t st = nullptr;
     DevBuf a, b, c;
-    FftCache fft;
+    FftCache fft, fft_real{CUFFT_C2R};
     p9idg_status init() {
         int count = 0;
         if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0)
@@ -1450,6 +1483,7 @@ void p9idg_plan_destroy(p9idg_plan *plan) {
         for (DevBuf *b : bufs) b->release();
         tc_release(plan->tc);
         plan->fft.release();
+        plan->fft_real.release();
         plan->d_gaps.release();
         plan->d_gitems_lyr.release();
         plan->d_sub_lyr.release();
@@ -1543,15 +1577,9 @@ p9idg_status p9idg_wstack_ifft_float(const double *layers, int32_t nlayers, int3
         return P9IDG_OK;
     }
     CK(s.a.ensure(sizeof(double2) * nn * nlayers));
-    CK(s.b.ensure(sizeof(float2) * nn));
     CK(s.c.ensure(sizeof(float) * nn));
     CK(cudaMemcpyAsync(s.a.p, layers, sizeof(double2) * nn * nlayers, cudaMemcpyHostToDevice, s.st));
-    CK(launch_layer_sum(s.a.p, true, nlayers, static_cast<int64_t>(nn), s.b.as<float2>(), s.st));
-    cufftHandle h;
-    TRY(s.fft.get(n, s.st, &h));
-    if (cufftExecC2C(h, s.b.as<cufftComplex>(), s.b.as<cufftComplex>(), CUFFT_INVERSE) != CUFFT_SUCCESS)
-        return fail(P9IDG_CUDA_ERROR, "cufftExecC2C failed");
-    CK(launch_real_part(s.b.as<float2>(), n, static_cast<double>(vis_count), false, s.c.as<float>(), nullptr, s.st));
+    TRY(layers_to_image(s.a.p, true, nlayers, n, vis_count, false, s.fft, s.fft_real, s.b, s.c.as<float>(), s.st));
     CK(cudaMemcpyAsync(image_out, s.c.p, sizeof(float) * nn, cudaMemcpyDeviceToHost, s.st));
     CK(cudaStreamSynchronize(s.st));
     return P9IDG_OK;
@@ -1637,14 +1665,9 @@ p9idg_status p9idg_degrid_device(p9idg_plan *plan, const void *d_grid, void *d_v
 p9idg_status p9idg_wstack_image_device(p9idg_plan *plan, const void *d_layers, float *d_image, int32_t shift) {
     if (!plan || !d_layers || !d_image) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(ensure_device(plan));
-    CK(plan->d_grid64.ensure(sizeof(float2) * nn_of(plan)));
-    {
-        StageScope t(plan, P9IDG_STAGE_LAYER_FFT);
-        CK(launch_layer_sum(d_layers, false, plan->c.wlayer_count, static_cast<int64_t>(nn_of(plan)),
-                            plan->d_grid64.as<float2>(), plan->stream));
-    }
-    return image_from_grid(plan, plan->d_grid64.as<float2>(), static_cast<double>(plan->c.vis_count), shift != 0,
-                           d_image, nullptr);
+    StageScope t(plan, P9IDG_STAGE_LAYER_FFT);
+    return layers_to_image(d_layers, false, plan->c.wlayer_count, plan->c.grid_size, plan->c.vis_count, shift != 0,
+                           plan->fft, plan->fft_real, plan->d_grid64, d_image, plan->stream);
 }
 
 p9idg_status p9idg_synchronize(p9idg_plan *plan) {

@@ -83,6 +83,48 @@ __global__ void layer_sum_kernel(const T *__restrict__ layers, int nlayers, int6
     }
 }
 
+// Half plane of the Hermitian part of the layers' sum, times scale: Re(IFFT(L)) is the
+// complex-to-real transform of H(k) = (L(k) + conj L(-k)) / 2, which needs half the work and traffic of
+// the complex one and no pass to take the real part.  alternate: times (-1)^(row + column), which moves
+// the image by n / 2 along both axes (FFT.Shift; n is even).  complex128 layers sum in FP64, complex64
+// layers in FP32 as in layer_sum_kernel; the scale is applied to FP32 values as hi + lo.
+// Bound by HBM: every layer is read once, a thread having two columns and their mirrors of each layer
+// in flight.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    layer_half_kernel(const T *__restrict__ layers, int nlayers, int n, double scale, bool alternate,
+                      float2 *__restrict__ out) {
+    using Acc = typename std::conditional<sizeof(T) == 16, double, float>::type;
+    const int r = blockIdx.x, c = 2 * (blockIdx.y * blockDim.x + threadIdx.x), nh = n / 2 + 1;
+    if (c >= nh) return;
+    const bool two = c + 1 < nh;
+    const int64_t nn = static_cast<int64_t>(n) * n;
+    const T *p = layers + static_cast<int64_t>(r) * n + c;
+    const T *q = layers + static_cast<int64_t>(r ? n - r : 0) * n;
+    const int q0 = c ? n - c : 0, q1 = n - c - 1;
+    Acc h[4] = {0, 0, 0, 0};  // the sums' real and imaginary parts at columns c and c + 1
+#pragma unroll 4
+    for (int k = 0; k < nlayers; k++) {
+        const T v0 = p[k * nn], w0 = q[k * nn + q0];
+        h[0] += v0.x + w0.x;
+        h[1] += v0.y - w0.y;
+        if (two) {
+            const T v1 = p[k * nn + 1], w1 = q[k * nn + q1];
+            h[2] += v1.x + w1.x;
+            h[3] += v1.y - w1.y;
+        }
+    }
+    float2 *dst = out + static_cast<int64_t>(r) * nh + c;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (j && !two) break;
+        const double sc = alternate && ((r + c + j) & 1) ? -0.5 * scale : 0.5 * scale;
+        const float sh = static_cast<float>(sc), sl = static_cast<float>(sc - static_cast<double>(sh));
+        const float re = static_cast<float>(h[2 * j]), im = static_cast<float>(h[2 * j + 1]);
+        dst[j] = make_float2(fmaf(re, sh, re * sl), fmaf(im, sh, im * sl));
+    }
+}
+
 // inv_norm = 1 / norm, made on the host: a multiply instead of an FP64 division per pixel
 __global__ void real_part_kernel(const float2 *__restrict__ in, int n, double inv_norm, bool shift,
                                  float *__restrict__ outf, double *__restrict__ outd) {
@@ -297,6 +339,18 @@ cudaError_t launch_layer_sum(const void *layers, bool c128, int nlayers, int64_t
     else
         layer_sum_kernel<float2><<<grid_blocks(nn, 256), 256, 0, st>>>(static_cast<const float2 *>(layers),
                                                                         nlayers, nn, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_layer_half(const void *layers, bool c128, int nlayers, int n, double scale, bool alternate,
+                              float2 *out, cudaStream_t st) {
+    const dim3 grid(n, (n / 2 + 1 + 511) / 512);
+    if (c128)
+        layer_half_kernel<double2><<<grid, 256, 0, st>>>(static_cast<const double2 *>(layers), nlayers, n, scale,
+                                                         alternate, out);
+    else
+        layer_half_kernel<float2><<<grid, 256, 0, st>>>(static_cast<const float2 *>(layers), nlayers, n, scale,
+                                                        alternate, out);
     return cudaGetLastError();
 }
 

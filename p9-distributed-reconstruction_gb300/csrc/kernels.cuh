@@ -120,6 +120,9 @@ cudaError_t launch_c128_to_c64(const double2 *in, int64_t count, float2 *out, cu
 cudaError_t launch_unit_vis(const uint8_t *flags, int64_t count, float2 *out, cudaStream_t st);
 // sum over layers (c64 or c128 input) -> c64 grid
 cudaError_t launch_layer_sum(const void *layers, bool c128, int nlayers, int64_t nn, float2 *out, cudaStream_t st);
+// half plane [n][n / 2 + 1] of the Hermitian part of that sum, times scale, for an even n
+cudaError_t launch_layer_half(const void *layers, bool c128, int nlayers, int n, double scale, bool alternate,
+                              float2 *out, cudaStream_t st);
 // real part / norm, optional FFT.Shift, to float or double
 cudaError_t launch_real_part(const float2 *in, int n, double norm, bool shift, float *outf, double *outd,
                              cudaStream_t st);
