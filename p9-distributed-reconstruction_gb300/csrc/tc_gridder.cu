@@ -41,14 +41,14 @@
 // (the mean of its samples' dw): the pixels are rotated by exp(-i dw0 r) in FP32 as the static
 // operand is made, and T1 is weighted by dw - dw0, which is an order smaller than dw (channels
 // and a short track).  FP16 hi + lo holds 22 bits, so what is left is the two phases' FP32
-// rounding and the hardware sincos, as in the sincos kernel: against FP64 7e-7 where that has
+// rounding and the hardware sincos, as in the sincos kernel: against FP64 6e-7 where that has
 // 8.5e-7 (2047^2, S = 24), and at most its error in every shape tested.  kFp32MaxDev: with
 // |dw - dw0| |r| <= 8e-4 the second-order term left out (3e-7 at most, 4e-8 rms over a subgrid's
 // samples and pixels) and the 11 bits of the first-order rows stay below that.
 // 8.0 M visibilities, S = 24: sincos kernel 2.04 ms (bound by the SFUs at 576 sincos per
 // visibility), this form 0.41 ms (48 useful of 64 sincos).  The gridder (EX) rotates its sums by
 // exp(i dw0 r) at the end and moves them out of the tensor core's accumulator every stage: 16.0 M
-// visibilities, S = 32, sincos kernel 6.75 ms, this form 1.05 ms, error 3.6e-7 -> 2.7e-7.
+// visibilities, S = 32, sincos kernel 6.75 ms, this form 1.05 ms, error 3.1e-7 -> 2.4e-7.
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -327,6 +327,15 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
         }
         if (y < S && x < S) out[shift_half(y, S) * S + shift_half(x, S)] = make_float2(re * tap, im * tap);
     }
+}
+
+// EX: what an accumulator of `valid` visibilities (at most a stage) is multiplied by.  Truncation toward zero
+// leaves it short by about 7e-8 of itself per K step of 16 (measured over 3072^2 to 287^2 grids, point
+// sources in noise: 2.4e-7 to 3.3e-7 after 4 steps, where the sincos kernel's sums are short by
+// 0.4e-7 to 1.4e-7), which 1 + 2^-22 undoes to within 1e-7.
+__device__ __forceinline__ float stage_gain(int valid) {
+    const int steps = (valid + 15) >> 4;
+    return steps >= 3 ? 1.f + 2.384185791015625e-7f : steps == 2 ? 1.f + 1.1920928955078125e-7f : 1.f;
 }
 
 // O2: the second-order form (|dw r| up to P9IDG_TC_MAX_W_TERM2): y rows 192-255 carry
@@ -632,6 +641,8 @@ __global__ void __launch_bounds__(kGThreads, 2)
                     break;
                 }
                 tc_fence_after();
+                const float gain = stage_gain(kGVps);
+                const float2 gain2 = make_float2(gain, gain);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     uint32_t bh[16], bl[16], sum[16];
@@ -644,7 +655,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) {
                         auto two = [j](const uint32_t *t) { return make_float2(__uint_as_float(t[j]), __uint_as_float(t[j + 1])); };
-                        const float2 v = __fadd2_rn(two(sum), __fadd2_rn(two(bh), two(bl)));
+                        const float2 v = __ffma2_rn(__fadd2_rn(two(bh), two(bl)), gain2, two(sum));
                         sum[j] = __float_as_uint(v.x);
                         sum[j + 1] = __float_as_uint(v.y);
                     }
@@ -677,10 +688,11 @@ __global__ void __launch_bounds__(kGThreads, 2)
 #pragma unroll
             for (int j = 0; j < 32; j++) e0[j * 33] += __uint_as_float(r[j]);
             if (EX) {
+                const float gain = stage_gain(nvis - (nstages - 1) * kGVps);
                 tmem_ld32(tq + 192, r);  // the earlier stages
                 tmem_ld_wait(r);
 #pragma unroll
-                for (int j = 0; j < 32; j++) e0[j * 33] += __uint_as_float(r[j]);
+                for (int j = 0; j < 32; j++) e0[j * 33] = fmaf(e0[j * 33], gain, __uint_as_float(r[j]));
             }
             float *e1 = E + (8 + 2 * q + u) * 1056 + lane;
             tmem_ld32(tq + 64, r);  // B1_u
@@ -856,8 +868,8 @@ __global__ void __launch_bounds__(kDThreads, 2)
                     st_shared_v4(addr, im_row(w[0]), im_row(w[1]), im_row(w[2]), im_row(w[3]));
             }
         };
-        put(0, lo);
-        put(1, hi);
+        put(kCentred ? 1 : 0, lo);
+        put(kCentred ? 0 : 1, hi);
         put(2, r1);
         if (O2) put(3, r2);
         fence_proxy_async();
@@ -885,8 +897,22 @@ __global__ void __launch_bounds__(kDThreads, 2)
                 tc_fence_after();
                 const uint32_t ahi = ts + b * kDTileBytes, alo = ahi + kDTileHalf;
                 const uint32_t acc = tmem + static_cast<uint32_t>(cb * 128);
+                if (kCentred) {
+                    // the small products first, so that the accumulator's truncation toward zero counts at
+                    // its full size for the four hi x hi steps only: [T0 lo | T1 (| T2)], then A_lo, then hi
 #pragma unroll
-                for (int kc = 0; kc < 4; kc++) {
+                    for (int kc = 0; kc < 4; kc++)
+                        mma_f16(acc, smem_desc(ahi + kc * 256, 128, 1024), smem_desc(bs + 8 * 1024 + kc * 256, 128, 1024),
+                                id1, kc > 0 ? 1u : 0u);
+#pragma unroll
+                    for (int kc = 0; kc < 4; kc++)
+                        mma_f16(acc, smem_desc(alo + kc * 256, 128, 1024), smem_desc(bs + kc * 256, 128, 1024), id64, 1u);
+#pragma unroll
+                    for (int kc = 0; kc < 4; kc++)
+                        mma_f16(acc, smem_desc(ahi + kc * 256, 128, 1024), smem_desc(bs + kc * 256, 128, 1024), id64, 1u);
+                }
+#pragma unroll
+                for (int kc = 0; kc < (kCentred ? 0 : 4); kc++) {
                     const uint64_t dahi = smem_desc(ahi + kc * 256, 128, 1024);
                     mma_f16(acc, dahi, smem_desc(bs + 8 * 1024 + kc * 256, 128, 1024), id1, kc > 0 ? 1u : 0u);
                     mma_f16(acc, dahi, smem_desc(bs + kc * 256, 128, 1024), id64, 1u);
