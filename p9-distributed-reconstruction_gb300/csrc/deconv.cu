@@ -18,7 +18,7 @@
 // (|change| bits << 32) | (0xFFFFFFFF - pixel index), so the largest key is the largest change
 // and, among equal changes, the first pixel, which is the order in which GetAbsMax
 // (FastSerialCD.cs:135-170) keeps its winner.  Iterations are launched from a captured CUDA
-// graph, 256 at a time, each chained to the previous by programmatic dependent launch; a launch
+// graph, 32 at a time, each chained to the previous by programmatic dependent launch; a launch
 // after the stopping iteration does nothing, so the iteration count and result equal the
 // reference's loop.
 
@@ -124,7 +124,11 @@ constexpr int kNT = 512, kWarps = kNT / 32;  // image reductions
 // the 152, each evaluating 5,120 pixels; 32 x 128 tiles of 512 threads need 175 CTAs, two on some
 // SMs, and the 3072^2 major cycle's coordinate descent ran 19 % slower with them.
 constexpr int kTY = 40, kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32, kCdBlocksPerSM = 1;
-constexpr int kGraphIters = 256;  // even: every replay ends on state buffer 0
+// Even: every replay ends on state buffer 0.  Launches past the stopping one are spent for nothing, up
+// to two replays' worth (the rest of its own and the one in flight); 1000 iterations at 3072^2 took
+// 7.33 ms with 256 a replay and one replay too many, and take 6.50 ms with 16 or 32 a replay (6.69
+// with 8, 6.76 to 6.79 with 64 to 256).
+constexpr int kGraphIters = 32;
 
 struct CdCtl {  // the state one launch hands to the next
     int32_t iter, done, converged, error;
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const CdParams *pp, unsi
 // per-call fields (images, lambda, alpha, eps, iteration cap) come from pp, which only the host
 // writes before the graph is launched.
 __global__ void __launch_bounds__(kCdNT, kCdBlocksPerSM)
-    cd_iter_kernel(const __grid_constant__ CdParams F, const CdParams *pp, int parity) {
+    cd_iter_kernel(const __grid_constant__ CdParams F, const CdParams *pp, int parity, CdCtl *report) {
     __shared__ unsigned long long sm_in[kCdWarps], sm_out[kCdWarps];
     __shared__ CdCtl c;
     CdParams P = F;
@@ -320,23 +324,28 @@ __global__ void __launch_bounds__(kCdNT, kCdBlocksPerSM)
     const CdCtl *cin = P.ctl + parity;
     CdCtl *cout = P.ctl + (1 - parity);
     if (threadIdx.x == 0) c = *cin;
+    // the last launch of a replay hands the state it leaves to the host (pinned memory; null otherwise)
+    const auto leave = [&](const CdCtl &v) {
+        *cout = v;
+        if (report) *report = v;
+    };
     const unsigned long long key = reduce_tiles(kin, ntiles, sm_in);  // its barrier publishes c
     const bool lead = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
     if (c.done) {
-        if (lead) *cout = c;
+        if (lead) leave(c);
         return;
     }
     if (c.iter >= P.max_iter) {  // while (!converged & iter < iterations)
-        if (lead) *cout = CdCtl{c.iter, 1, 0, 0};
+        if (lead) leave(CdCtl{c.iter, 1, 0, 0});
         return;
     }
     const float diff = __uint_as_float(static_cast<uint32_t>(key >> 32));
     if (diff < P.eps) {  // converged = maxPixel.PixelMaxDiff < epsilon
-        if (lead) *cout = CdCtl{c.iter, 1, 1, 0};
+        if (lead) leave(CdCtl{c.iter, 1, 1, 0});
         return;
     }
     if (key == 0ull) {  // the reference would index pixel (-1, -1)
-        if (lead) *cout = CdCtl{c.iter, 1, 0, 1};
+        if (lead) leave(CdCtl{c.iter, 1, 0, 1});
         return;
     }
     Window w;
@@ -362,7 +371,7 @@ __global__ void __launch_bounds__(kCdNT, kCdBlocksPerSM)
     const float2 *sel_val = vin + static_cast<int>(w.py / kTY) * P.tiles_x + static_cast<int>(w.px / kTX);
     const int ty = ty0 + static_cast<int>(blockIdx.y), tx = tx0 + static_cast<int>(blockIdx.x);
     if (ty <= ty1 && tx <= tx1) eval_tile<true>(P, P.lambda, P.alpha, ty, tx, w, sel_val, kout, vout, sm_out);
-    if (lead) *cout = CdCtl{c.iter + 1, 0, 0, 0};
+    if (lead) leave(CdCtl{c.iter + 1, 0, 0, 0});
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next iteration may launch
 }
 
@@ -981,7 +990,7 @@ p9idg_status cd_capture(p9idg_cd *cd) {
     cudaError_t le = cudaSuccess;
     for (int k = 0; k < kGraphIters && le == cudaSuccess; k++)
         le = cudaLaunchKernelEx(&cfg, cd_iter_kernel, cd->hp, static_cast<const CdParams *>(cd->params.as<CdParams>()),
-                                k & 1);
+                                k & 1, k + 1 == kGraphIters ? cd->h_ctl : static_cast<CdCtl *>(nullptr));
     cudaGraph_t gph = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(cd->own, &gph);
     if (le != cudaSuccess || ce != cudaSuccess) {
@@ -1014,17 +1023,17 @@ p9idg_status cd_run(p9idg_cd *cd, float *d_x, float *d_g, float lambda, float al
     TRY(cd_upload_params(cd));
     TRY(cd_scan(cd, lambda, alpha));
     TRY(cd_capture(cd));
-    // One replay stays in flight while the host reads the control word the previous one left: the
-    // copy after replay r is enqueued before replay r + 1, so the GPU never waits on the host.  A
-    // replay launched after the stopping one does nothing (every launch sees the done flag).
-    const int64_t max_replays = static_cast<int64_t>(std::max(max_iter, 0)) / kGraphIters + 2;
+    // One replay stays in flight while the host looks at the state the previous one left, so the GPU
+    // never waits on the host; a replay launched after the stopping one does nothing (every launch sees
+    // the done flag).  max_iter + 1 launches are enough: the one past the last iteration stops.
+    const int64_t max_replays = (static_cast<int64_t>(std::max(max_iter, 0)) + kGraphIters) / kGraphIters;
+    *cd->h_ctl = CdCtl{};
     CK(cudaGraphLaunch(cd->exec, cd->stream));
     for (int64_t r = 0; r < max_replays; r++) {
-        CK(cudaMemcpyAsync(cd->h_ctl, cd->ctl.p, sizeof(CdCtl), cudaMemcpyDeviceToHost, cd->stream));
         CK(cudaEventRecord(cd->ev_ctl, cd->stream));
         if (r + 1 < max_replays) CK(cudaGraphLaunch(cd->exec, cd->stream));
         CK(cudaEventSynchronize(cd->ev_ctl));
-        if (cd->h_ctl->done) break;
+        if (static_cast<volatile CdCtl *>(cd->h_ctl)->done) break;
     }
     CK(cudaStreamSynchronize(cd->stream));  // the replay in flight, if any
     if (!cd->h_ctl->done) return fail(P9IDG_DEVICE_CHECK_FAILED, "coordinate descent did not stop");
