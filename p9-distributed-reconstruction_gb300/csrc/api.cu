@@ -181,7 +181,8 @@ struct p9idg_plan {
     std::vector<int64_t> gaps;  // (start, count) ranges of visibilities no subgrid covers
     std::vector<char> layer_used;  // w layers some subgrid adds into
     bool gaps_ready = false;
-    DevBuf d_gaps;
+    DevBuf d_gaps;        // the gaps, then the same ranges in pieces of at most kZeroPiece words
+    int64_t gap_words = 0, gap_pieces = 0;
     cudaStream_t side = nullptr;  // the D2H copy of DeGrid's shifted grid runs here, beside the degridder
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mid = nullptr;
     // Zero-fills beside the gridder and degridder (ZeroSide): a high-priority stream, so that its few
@@ -572,10 +573,14 @@ struct ZeroSide {
     }
 };
 
+// Whether nitems tensor-core work items' loader warps can zero that many 8-byte words without lengthening
+// the kernel: up to 128 KB each, of the 20 us and more that an item takes.
+bool zero_in_kernel(int64_t words, int64_t nitems) { return words > 0 && words <= nitems * 16384; }
+
 // Gridder over nitems work items (all of the plan's, or a group of them) into their partial slots.
 // fp32_tc: the items are the FP32 mode's tensor-core form's.
 p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const WorkItem *d_items, int32_t nitems,
-                        bool fp32_tc = false) {
+                        bool fp32_tc = false, const ZeroFill &zero = {}) {
     const int S = p->c.subgrid_size;
     const int32_t nslots = fp32_tc ? p->tc.nslots : p->nslots;
     CK(p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, nslots)));
@@ -586,6 +591,7 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
     a.vis = d_vis;
     a.vis_c128 = vis_c128;
     a.partials = p->d_partials.as<float2>();
+    a.zero = zero;
     if (use_tc(p) || fp32_tc) {
         TRY(ensure_tc(p));
         TRY(tc_grid(p->tc, a, p->mode, p->stream, g_last_error));
@@ -613,8 +619,10 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
     return P9IDG_OK;
 }
 
-// The layers are zeroed beside the gridder (a 604 MB fill at 3072^2 with 8 layers, 0.09 ms of the
-// adder's stage when it ran there).
+// The layers are zeroed by the tensor-core gridder's loader warps, which idle once a work item's last
+// stage is on its way, or, where there is too much to zero for the items there are and for the sincos
+// kernels, beside the gridder (a 604 MB fill at 3072^2 with 8 layers, 0.09 ms of the adder's stage when
+// it ran there).  A small call saves the launch and the two stream dependencies.
 p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d_layers, bool wstack,
                       bool device_call = false) {
     const int nl = wstack ? p->c.wlayer_count : 1;
@@ -626,11 +634,18 @@ p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d
         items = static_cast<const WorkItem *>(p->tc.gitems);
         nitems = static_cast<int32_t>(p->tc.gitems_host.size());
     }
-    ZeroSide z{p};
-    TRY(z.fork());
-    TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc));
-    CK(launch_zero_c64_beside(d_layers, static_cast<int64_t>(nl) * static_cast<int64_t>(nn_of(p)), p->zside));
-    TRY(z.join());
+    const int64_t words = static_cast<int64_t>(nl) * static_cast<int64_t>(nn_of(p));
+    if ((use_tc(p) || fp32_tc) && zero_in_kernel(words, nitems)) {
+        const ZeroFill zero{reinterpret_cast<uint2 *>(d_layers), nullptr, words, (words + kZeroPiece - 1) / kZeroPiece,
+                            kZeroPiece, 0};
+        TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc, zero));
+    } else {
+        ZeroSide z{p};
+        TRY(z.fork());
+        TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc));
+        CK(launch_zero_c64_beside(d_layers, words, p->zside));
+        TRY(z.join());
+    }
     return add_subgrids(p, d_layers, wstack, nullptr, 0, fp32_tc);
 }
 
@@ -639,17 +654,21 @@ p9idg_status ensure_gaps(p9idg_plan *p);
 
 // The degridder writes every visibility some subgrid covers; only the others (quirk P1's drops,
 // baselines without subgrids) are zeroed apart.  Output in host memory (out_in_host): before the
-// degridder, on the plan's stream.  Output in device memory: beside the splitter and degridder, on
-// the zeroing stream, as the two write disjoint visibilities (the whole output, 516 MB at 3072^2,
-// was zeroed before the degridder, 0.08 ms of its stage).
+// degridder, on the plan's stream.  Output in device memory: by the tensor-core degridder's loader
+// warps (complex64), else beside the splitter and degridder, on the zeroing stream, as the two write
+// disjoint visibilities (the whole output, 516 MB at 3072^2, was zeroed before the degridder, 0.08 ms
+// of its stage).
 p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, void *d_vis, bool out_c128,
                         bool wstack, bool out_in_host = false) {
     const int S = p->c.subgrid_size;
     CK(p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size())));
     TRY(ensure_gaps(p));
     const int64_t ngaps = static_cast<int64_t>(p->gaps.size() / 2);
+    const bool tc = use_tc(p) || use_fp32_tc(p, !out_c128);
+    if (tc) TRY(ensure_tc(p));
+    const bool fused = tc && !out_c128 && (ngaps == 0 || zero_in_kernel(p->gap_words, p->tc.nditems));
     ZeroSide z{p};
-    if (!out_in_host) TRY(z.fork());
+    if (!out_in_host && !fused) TRY(z.fork());
     {
         StageScope t(p, P9IDG_STAGE_SPLIT_SUBGRID_FFT);
         SubgridOpArgs a = subgrid_args(p);
@@ -659,7 +678,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.wstack = wstack;
         CK(launch_split_subgrid_fft(a, p->stream));
     }
-    if (!out_in_host) CK(launch_zero_ranges_beside(d_vis, out_c128, p->d_gaps.as<int64_t>(), ngaps, p->zside));
+    if (!out_in_host && !fused) CK(launch_zero_ranges_beside(d_vis, out_c128, p->d_gaps.as<int64_t>(), ngaps, p->zside));
     {
         StageScope t(p, P9IDG_STAGE_DEGRIDDER);
         if (out_in_host) CK(launch_zero_ranges(d_vis, out_c128, p->d_gaps.as<int64_t>(), ngaps, p->stream));
@@ -669,14 +688,15 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.subgrids = p->d_subgrids.as<float2>();
         a.vis_out = d_vis;
         a.out_c128 = out_c128;
-        if (use_tc(p) || use_fp32_tc(p, !out_c128)) {
-            TRY(ensure_tc(p));
+        if (tc) {
+            if (fused)
+                a.zero = {static_cast<uint2 *>(d_vis), p->d_gaps.as<int64_t>() + 2 * ngaps, 0, p->gap_pieces, 0, 0};
             TRY(tc_degrid(p->tc, a, p->mode, p->stream, g_last_error));
         } else {
             CK(launch_degridder_fp32(a, p->stream));
         }
     }
-    if (!out_in_host) TRY(z.join());
+    if (!out_in_host && !fused) TRY(z.join());
     return P9IDG_OK;
 }
 
@@ -740,10 +760,19 @@ p9idg_status ensure_gaps(p9idg_plan *p) {
         }
         if (sx >= 1 && sx < N - S && sy >= 1 && sy < N - S && sw >= 0 && sw < W) p->layer_used[sw] = 1;
     }
-    CK(p->d_gaps.ensure(sizeof(int64_t) * std::max<size_t>(2, p->gaps.size())));
-    if (!p->gaps.empty())
-        CK(cudaMemcpyAsync(p->d_gaps.p, p->gaps.data(), sizeof(int64_t) * p->gaps.size(), cudaMemcpyHostToDevice,
-                           p->stream));
+    std::vector<int64_t> all(p->gaps);
+    p->gap_words = 0;
+    for (size_t k = 0; k < p->gaps.size(); k += 2) {
+        p->gap_words += p->gaps[k + 1];
+        for (int64_t j = 0; j < p->gaps[k + 1]; j += kZeroPiece) {
+            all.push_back(p->gaps[k] + j);
+            all.push_back(std::min<int64_t>(kZeroPiece, p->gaps[k + 1] - j));
+        }
+    }
+    p->gap_pieces = static_cast<int64_t>((all.size() - p->gaps.size()) / 2);
+    CK(p->d_gaps.ensure(sizeof(int64_t) * std::max<size_t>(2, all.size())));
+    if (!all.empty())
+        CK(cudaMemcpyAsync(p->d_gaps.p, all.data(), sizeof(int64_t) * all.size(), cudaMemcpyHostToDevice, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     p->gaps_ready = true;
     return P9IDG_OK;
@@ -1165,8 +1194,9 @@ struct p9idg_batch {
     int tc_order = 1;  // tensor-core batches: 2 when any plan needs the second-order form
     std::vector<int64_t> prob_vis;             // visibilities per problem (for the schedules)
     int32_t schedule = P9IDG_SCHEDULE_THROUGHPUT;
-    std::vector<void *> layers, vis_out;
-    std::vector<size_t> layer_bytes, vis_bytes;
+    // The w layers and the visibilities no subgrid covers, as ranges from address 0
+    DevBuf d_zgrid, d_zvis;
+    int64_t nzgrid = 0, nzvis = 0, zgrid_words = 0, zvis_words = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -1177,12 +1207,37 @@ namespace {
 bool batch_tc(const p9idg_plan *p) { return use_tc(p) || use_fp32_tc(p, true); }
 int32_t group_key(const p9idg_plan *p) { return 2 * p->c.subgrid_size + (batch_tc(p) ? 1 : 0); }
 
-__global__ void stamp_kernel(unsigned long long *t) { *t = device_ns(); }
+// Start of a degrid phase: its time, and each problem's work-item countdown and completion time.
+__global__ void batch_start_kernel(unsigned long long *start, const int32_t *done_init, int32_t *done,
+                                   unsigned long long *finish, int n) {
+    if (threadIdx.x == 0) *start = device_ns();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        done[i] = done_init[i];
+        finish[i] = 0;
+    }
+}
 
+// The zero-fill a stage's first tensor-core launch does (there is one with enough items), or all of it
+// now, in one launch.
+p9idg_status batch_zero(p9idg_batch *b, const DevBuf &ranges, int64_t n, int64_t words, bool degrid, int &in_group,
+                        ZeroFill &zero) {
+    zero = {nullptr, ranges.as<int64_t>(), 0, n, 0, 0};
+    in_group = -1;
+    for (size_t k = 0; k < b->groups.size() && in_group < 0; k++)
+        if (b->groups[k].tc && zero_in_kernel(words, degrid ? b->groups[k].dn : b->groups[k].gn))
+            in_group = static_cast<int>(k);
+    if (in_group < 0) CK(launch_zero_fill(zero, b->stream));
+    return P9IDG_OK;
+}
+
+// The layers are zeroed in the gridder kernels, the uncovered visibilities in the degridder, or each in
+// one launch before them (12 problems of 512^2 to 1024^2: 24 memsets took 0.08 of 1.15 ms a pass).
 p9idg_status batch_grid(p9idg_batch *b) {
-    for (size_t i = 0; i < b->plans.size(); i++)
-        CK(cudaMemsetAsync(b->layers[i], 0, b->layer_bytes[i], b->stream));
-    for (const auto &g : b->groups) {
+    int zk;
+    ZeroFill zero;
+    TRY(batch_zero(b, b->d_zgrid, b->nzgrid, b->zgrid_words, false, zk, zero));
+    for (size_t k = 0; k < b->groups.size(); k++) {
+        const auto &g = b->groups[k];
         GridderArgs L{};
         L.g.S = g.S;
         L.items = b->d_gitems.as<WorkItem>() + g.g0;
@@ -1190,7 +1245,8 @@ p9idg_status batch_grid(p9idg_batch *b) {
         if (!g.tc) {
             if (g.gn > 0) CK(launch_gridder_fp32(L, b->stream, b->d_gargs.as<GridderArgs>()));
         } else {
-            TRY(tc_grid_batch(b->d_tg.as<TcArgs>(), L.items, g.gn, b->mode, b->tc_order, b->stream, g_last_error));
+            TRY(tc_grid_batch(b->d_tg.as<TcArgs>(), L.items, g.gn, static_cast<int>(k) == zk ? zero : ZeroFill{}, b->mode,
+                              b->tc_order, b->stream, g_last_error));
         }
     }
     for (const auto &g : b->groups) {
@@ -1205,11 +1261,13 @@ p9idg_status batch_grid(p9idg_batch *b) {
 }
 
 p9idg_status batch_degrid(p9idg_batch *b) {
-    const size_t n = b->plans.size();
-    stamp_kernel<<<1, 1, 0, b->stream>>>(b->d_start.as<unsigned long long>());
+    const int n = static_cast<int>(b->plans.size());
+    batch_start_kernel<<<1, 128, 0, b->stream>>>(b->d_start.as<unsigned long long>(), b->d_done_init.as<int32_t>(),
+                                                 b->d_done.as<int32_t>(), b->d_finish.as<unsigned long long>(), n);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(b->d_done.p, b->d_done_init.p, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, b->stream));
-    CK(cudaMemsetAsync(b->d_finish.p, 0, sizeof(unsigned long long) * n, b->stream));
+    int zk;
+    ZeroFill zero;
+    TRY(batch_zero(b, b->d_zvis, b->nzvis, b->zvis_words, true, zk, zero));
     for (const auto &g : b->groups) {
         SubgridOpArgs A{};
         A.g.S = g.S;
@@ -1218,8 +1276,8 @@ p9idg_status batch_degrid(p9idg_batch *b) {
         A.wstack = true;
         if (g.rn > 0) CK(launch_split_subgrid_fft(A, b->stream, b->d_sargs.as<SubgridOpArgs>()));
     }
-    for (size_t i = 0; i < n; i++) CK(cudaMemsetAsync(b->vis_out[i], 0, b->vis_bytes[i], b->stream));
-    for (const auto &g : b->groups) {
+    for (size_t k = 0; k < b->groups.size(); k++) {
+        const auto &g = b->groups[k];
         GridderArgs L{};
         L.g.S = g.S;
         L.items = b->d_ditems.as<WorkItem>() + g.d0;
@@ -1227,8 +1285,8 @@ p9idg_status batch_degrid(p9idg_batch *b) {
         if (!g.tc) {
             if (g.dn > 0) CK(launch_degridder_fp32(L, b->stream, b->d_dargs.as<GridderArgs>()));
         } else {
-            TRY(tc_degrid_batch(b->d_td.as<TcArgs>(), L.items, g.dn, b->mode, b->tc_order, b->stream,
-                                g_last_error));
+            TRY(tc_degrid_batch(b->d_td.as<TcArgs>(), L.items, g.dn, static_cast<int>(k) == zk ? zero : ZeroFill{},
+                                b->mode, b->tc_order, b->stream, g_last_error));
         }
     }
     return P9IDG_OK;
@@ -1287,7 +1345,7 @@ void batch_release(p9idg_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     DevBuf *bufs[] = {&b->d_gargs, &b->d_dargs, &b->d_aargs, &b->d_sargs, &b->d_tg, &b->d_td, &b->d_gitems,
-                      &b->d_ditems, &b->d_subs, &b->d_refs, &b->d_done_init, &b->d_done, &b->d_finish, &b->d_start};
+                      &b->d_zgrid, &b->d_zvis, &b->d_ditems, &b->d_subs, &b->d_refs, &b->d_done_init, &b->d_done, &b->d_finish, &b->d_start};
     for (DevBuf *x : bufs) x->release();
     if (b->stream) cudaStreamDestroy(b->stream);
 }
@@ -1776,6 +1834,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     std::vector<WorkItem> gitems, ditems;
     std::vector<DevSubgrid> subs;
     std::vector<int2> refs;
+    std::vector<int64_t> zgrid, zvis;
     std::vector<int32_t> done(nplans, 0);
     // device-side completion tracking first: the argument tables point into it
     p9idg_status st;
@@ -1850,10 +1909,18 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         bool known = false;
         for (const auto &g : b->groups) known |= g.key == group_key(p);
         if (!known) b->groups.push_back({group_key(p), S, tc, 0, 0, 0, 0, 0, 0});
-        b->layers.push_back(d_layers[i]);
-        b->layer_bytes.push_back(sizeof(float2) * static_cast<size_t>(p->c.wlayer_count) * nn_of(p));
-        b->vis_out.push_back(d_vis_out[i]);
-        b->vis_bytes.push_back(sizeof(float2) * vis_count_of(p));
+        if ((st = ensure_gaps(p)) != P9IDG_OK) return bail(st);
+        const auto zero = [](std::vector<int64_t> &v, int64_t &total, void *base, int64_t first, int64_t words) {
+            const int64_t at = static_cast<int64_t>(reinterpret_cast<uintptr_t>(base) / 8) + first;
+            for (int64_t k = 0; k < words; k += kZeroPiece) {
+                v.push_back(at + k);
+                v.push_back(std::min<int64_t>(kZeroPiece, words - k));
+            }
+            total += words;
+        };
+        zero(zgrid, b->zgrid_words, d_layers[i], 0,
+             static_cast<int64_t>(p->c.wlayer_count) * static_cast<int64_t>(nn_of(p)));
+        for (size_t k = 0; k < p->gaps.size(); k += 2) zero(zvis, b->zvis_words, d_vis_out[i], p->gaps[k], p->gaps[k + 1]);
         cudaError_t e2 = cudaStreamSynchronize(p->stream);
         if (e2 != cudaSuccess) return bail(cuda_fail(e2, "plan preparation"));
     }
@@ -1878,7 +1945,11 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     b->ngitems = static_cast<int32_t>(b->h_gitems.size());
     b->nditems = static_cast<int32_t>(b->h_ditems.size());
     b->nrefs = static_cast<int32_t>(refs.size());
-    if ((st = upload(b->d_subs, subs)) != P9IDG_OK) return bail(st);
+    b->nzgrid = static_cast<int64_t>(zgrid.size() / 2);
+    b->nzvis = static_cast<int64_t>(zvis.size() / 2);
+    if ((st = upload(b->d_zgrid, zgrid)) != P9IDG_OK || (st = upload(b->d_zvis, zvis)) != P9IDG_OK ||
+        (st = upload(b->d_subs, subs)) != P9IDG_OK)
+        return bail(st);
     for (auto &x : aa)
         x.subs = reinterpret_cast<const DevSubgrid *>(b->d_subs.as<char>() + reinterpret_cast<uintptr_t>(x.subs));
     if ((st = upload(b->d_gargs, ga)) != P9IDG_OK || (st = upload(b->d_dargs, da)) != P9IDG_OK ||
@@ -1951,6 +2022,7 @@ p9idg_status p9idg_batch_capture_graph(p9idg_batch *b) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
     b->graph = g;
     CK(cudaGraphInstantiate(&b->exec, b->graph, 0));
+    CK(cudaGraphUpload(b->exec, b->stream));
     return P9IDG_OK;
 }
 

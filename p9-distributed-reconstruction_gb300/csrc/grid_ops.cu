@@ -248,6 +248,10 @@ __global__ void zero_words_kernel(uint2 *__restrict__ out, int64_t n8) {
     }
 }
 
+__global__ void zero_fill_kernel(const ZeroFill z) {
+    for (int64_t p = blockIdx.x; p < z.count; p += gridDim.x) zero_piece(z, p, threadIdx.x, blockDim.x);
+}
+
 __global__ void zero_c128_kernel(double2 *__restrict__ out, int64_t count) {
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < count;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x)
@@ -305,6 +309,12 @@ cudaError_t launch_zero_ranges_beside(void *out, bool c128, const int64_t *range
         zero_ranges_kernel<double2><<<blocks, 128, 0, st>>>(static_cast<double2 *>(out), ranges, nranges);
     else
         zero_ranges_kernel<float2><<<blocks, 128, 0, st>>>(static_cast<float2 *>(out), ranges, nranges);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_zero_fill(const ZeroFill &z, cudaStream_t st) {
+    if (z.count == 0) return cudaSuccess;
+    zero_fill_kernel<<<static_cast<unsigned>(std::min<int64_t>(z.count, sm_count() * 8)), 256, 0, st>>>(z);
     return cudaGetLastError();
 }
 

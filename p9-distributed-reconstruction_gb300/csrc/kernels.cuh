@@ -39,6 +39,40 @@ __device__ inline float2 load_vis(const double2 *v, int64_t i) {
 __device__ inline void store_vis(float2 *v, int64_t i, float2 x) { v[i] = x; }
 __device__ inline void store_vis(double2 *v, int64_t i, float2 x) { v[i] = make_double2(x.x, x.y); }
 
+// A zero-fill in pieces of 8-byte words: of `total` words from base on, `piece` at a time, or (ranges
+// given) of ranges[2 i + 1] words from word ranges[2 i] on, counted from base (null: from address 0).
+// The tensor-core kernels' loader warps do it in the time they would idle: block b takes the pieces
+// b, b + gridDim.x, ...
+struct ZeroFill {
+    uint2 *base;
+    const int64_t *ranges;
+    int64_t total, count;  // words (without ranges), pieces
+    int32_t piece, pad;
+};
+constexpr int32_t kZeroPiece = 2048;  // words: 16 KB
+
+__device__ __forceinline__ void zero_piece(const ZeroFill &z, int64_t p, int thread, int nthreads) {
+    uint2 *out;
+    int64_t n8;
+    if (z.ranges) {
+        out = reinterpret_cast<uint2 *>(reinterpret_cast<uintptr_t>(z.base) + 8 * z.ranges[2 * p]);
+        n8 = z.ranges[2 * p + 1];
+    } else {
+        out = z.base + p * z.piece;
+        n8 = z.total - p * z.piece;
+        n8 = n8 < z.piece ? n8 : z.piece;
+    }
+    // 16-byte stores from the first 16-byte boundary on
+    const int64_t head = (reinterpret_cast<uintptr_t>(out) & 15) != 0 && n8 > 0 ? 1 : 0;
+    const int64_t n16 = (n8 - head) / 2;
+    uint4 *body = reinterpret_cast<uint4 *>(out + head);
+    for (int64_t i = thread; i < n16; i += nthreads) body[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (thread == 0) {
+        if (head) out[0] = make_uint2(0u, 0u);
+        if ((n8 - head) & 1) out[n8 - 1] = make_uint2(0u, 0u);
+    }
+}
+
 // ---- launchers (gridder_fp32.cu) ----
 struct GridderArgs {
     Geometry g;
@@ -57,6 +91,7 @@ struct GridderArgs {
     bool out_c128;
     int32_t nsub;              // subgrids in `subs`
     int32_t *status;           // device status word
+    ZeroFill zero;             // tensor-core kernels: what their loader warps zero (count 0: nothing)
     // batched launches: work items left in this problem; the CTA finishing the last one
     // records the GPU time (ns) in *finish_ns.  Null when not tracked.
     int32_t *done;
@@ -113,6 +148,8 @@ cudaError_t launch_zero_ranges(void *out, bool c128, const int64_t *ranges, int6
 // zero-fills to run beside a tensor-core gridder or degridder: CTAs of 128 threads, at most one per SM
 cudaError_t launch_zero_ranges_beside(void *out, bool c128, const int64_t *ranges, int64_t nranges, cudaStream_t st);
 cudaError_t launch_zero_c64_beside(float2 *out, int64_t count, cudaStream_t st);
+// the pieces of a ZeroFill, on their own
+cudaError_t launch_zero_fill(const ZeroFill &z, cudaStream_t st);
 cudaError_t launch_zero_c128(double2 *out, int64_t count, cudaStream_t st);
 // *flag (int32, device) = whether two device arrays of nwords 64-bit words differ anywhere
 cudaError_t launch_words_differ(const void *a, const void *b, int64_t nwords, int32_t *flag, cudaStream_t st);

@@ -472,6 +472,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
             }
             issued = i + 1;
         }
+        for (int64_t p = blockIdx.x; p < L.zero.count; p += gridDim.x) zero_piece(L.zero, p, lane, 32);
         // tiles still in flight land before the CTA can exit (consumed ones have completed)
         if (lane == 0) {
             volatile int never = 0;
@@ -505,6 +506,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
             }
             cp_async_arrive(&in_full[slot]);
         }
+        for (int64_t p = blockIdx.x; p < L.zero.count; p += gridDim.x) zero_piece(L.zero, p, lane, 32);
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ---- producers
@@ -930,8 +932,8 @@ __global__ void __launch_bounds__(kDThreads, 2)
     } else if (warp == kDLoaderWarp && TMA) {
         // ---- loader (TMA): tile i's 128 coefficients as one 2-D tile -> ring slot i % kDRing; rows
         // past the item's end belong to the next item and only feed visibilities never stored
+        int issued = 0;
         if (lane == 0) {
-            int issued = 0;
             for (int i = 0; i < ntiles; i++) {
                 const int slot = i % kDRing;
                 const uint32_t ph = (i / kDRing) & 1;
@@ -949,6 +951,10 @@ __global__ void __launch_bounds__(kDThreads, 2)
                             &in_full[slot]);
                 issued = i + 1;
             }
+        }
+        __syncwarp();
+        for (int64_t p = blockIdx.x; p < L.zero.count; p += gridDim.x) zero_piece(L.zero, p, lane, 32);
+        if (lane == 0) {
             volatile int never = 0;
             for (int i = issued > kDRing ? issued - kDRing : 0; i < issued; i++)
                 if (!mbar_wait(&in_full[i % kDRing], (i / kDRing) & 1, &never, a.wait_ns)) atomicOr(a.status, kStatusWait);
@@ -976,6 +982,7 @@ __global__ void __launch_bounds__(kDThreads, 2)
             }
             cp_async_arrive(&in_full[slot]);
         }
+        for (int64_t p = blockIdx.x; p < L.zero.count; p += gridDim.x) zero_piece(L.zero, p, lane, 32);
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp < 4) {
         // ---- producers: A tile, hi and lo.  Thread t writes the 16-byte chunks cc = t + 128 u
@@ -1602,6 +1609,7 @@ void tc_fill_args(const TcPlanState &st, const GridderArgs &a, TcArgs &t) {
     t.status = a.status;
     t.done = a.done;
     t.finish_ns = a.finish_ns;
+    t.zero = a.zero;
 }
 
 p9idg_status tc_coefs(TcPlanState &st, const GridderArgs &a, cudaStream_t stream, std::string &err) {
@@ -1641,18 +1649,20 @@ p9idg_status tc_degrid(TcPlanState &st, const GridderArgs &a, int mode, cudaStre
                                                              tma ? &maps : nullptr, stream, err);
 }
 
-p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, int mode, int order,
-                           cudaStream_t stream, std::string &err) {
+p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero, int mode,
+                           int order, cudaStream_t stream, std::string &err) {
     TcArgs t{};
     t.items = items;
+    t.zero = zero;
     return order == 2 ? launch_tc_gridder<true, true>(t, probs, nitems, false, mode, nullptr, stream, err)
                       : launch_tc_gridder<true, false>(t, probs, nitems, false, mode, nullptr, stream, err);
 }
 
-p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, int mode, int order,
-                             cudaStream_t stream, std::string &err) {
+p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero,
+                             int mode, int order, cudaStream_t stream, std::string &err) {
     TcArgs t{};
     t.items = items;
+    t.zero = zero;
     return order == 2 ? launch_tc_degridder<true, true>(t, probs, nitems, false, mode, nullptr, stream, err)
                       : launch_tc_degridder<true, false>(t, probs, nitems, false, mode, nullptr, stream, err);
 }

@@ -69,6 +69,7 @@ struct TcArgs {
     int32_t *done;   // batched launches: completion count / time (see GridderArgs)
     unsigned long long *finish_ns;
     uint64_t wait_ns;          // limit of every pipeline wait before the kernel gives up (2 s)
+    ZeroFill zero;             // launch-wide, also in batches
     int32_t debug_skip_stage;  // fault injection: the loader never delivers this stage (-1: off)
 };
 
@@ -91,10 +92,10 @@ p9idg_status tc_coefs(TcPlanState &st, const GridderArgs &a, cudaStream_t stream
 // indexed by WorkItem::problem.
 // order: 2 when any problem of the batch needs the second-order form (it serves first-order
 // problems as well, a little more accurately).
-p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, int mode, int order,
-                           cudaStream_t stream, std::string &err);
-p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, int mode, int order,
-                             cudaStream_t stream, std::string &err);
+p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero, int mode,
+                           int order, cudaStream_t stream, std::string &err);
+p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero,
+                             int mode, int order, cudaStream_t stream, std::string &err);
 // The form (1 or 2) a plan with this w term runs for a requested order (0 = automatic), or 0 when
 // neither bound holds (the plan then keeps the FP32 kernels).
 int tc_order_for(double w_term, int want_order);
