@@ -151,6 +151,7 @@ struct p9idg_plan {
     // hi + lo: see fp32_on_tensor_cores.  The host-array calls, whose results keep to the last bit and
     // which may pass a uvw of their own, run the sincos kernels.
     bool fp32_tc = false;
+    int64_t wave_grid = 0, wave_degrid = 0;  // default tensor-core work-item sizes (0: not worked out yet)
     std::vector<double> freq, wn, uvw;
     std::vector<p9idg_subgrid> subs;
     std::vector<DevSubgrid> dsub;
@@ -488,14 +489,44 @@ GridderArgs gridder_args(p9idg_plan *p) {
     return a;
 }
 
+// Visibilities per tensor-core work item: the most there may be (hi), or, where that leaves room in the
+// first wave of two items per SM, the fewest (a multiple of 128) that still make one wave: an item takes
+// about 6 us before and after its visibilities and 15 ns for each, so fewer and longer items, and items
+// left for a second wave, are slower (341^2, 66 baselines: gridder call 57 -> 32 us; splitting to V / slots
+// without counting the items instead made a call of 23 us 25 us).
+int64_t wave_chunk(const p9idg_plan *p, int64_t hi) {
+    const int64_t slots = 2 * static_cast<int64_t>(sm_count());
+    const auto items = [&](int64_t c) {
+        const int64_t times = std::max<int64_t>(1, c / std::max(1, p->nch));
+        int64_t n = 0;
+        for (const auto &s : p->subs) n += (s.time_sample_count + times - 1) / times;
+        return n;
+    };
+    if (static_cast<int64_t>(p->subs.size()) >= slots || items(hi) >= slots) return hi;
+    int64_t lo = 0, up = hi / 128;  // items(128 lo) > slots >= items(128 up)
+    while (up - lo > 1) {
+        const int64_t mid = (lo + up) / 2;
+        (items(128 * mid) > slots ? lo : up) = mid;
+    }
+    return 128 * up;
+}
+
 p9idg_status ensure_tc(p9idg_plan *p) {
     // degridder items do not accumulate across visibilities: 16384 measured 1.6 % faster than 8192
     // (32768 the same as 16384), 8192 3.5 % faster than 4096.  The FP32 mode's sizes (1024 and 512 by
     // default) are its sincos kernels' work items; its tensor-core form takes 4 and 32 times as many
     // visibilities, the other modes' defaults.
-    const int64_t scale = p->mode == P9IDG_MODE_FP32 ? 32 : 1;
-    p->tc.degrid_chunk = p->dchunk > 0 ? scale * p->dchunk : 16384;
-    p->tc.grid_chunk = p->mode == P9IDG_MODE_FP32 ? (p->gchunk > 0 ? 4 * static_cast<int64_t>(p->gchunk) : 4096) : 0;
+    const bool fp32 = p->mode == P9IDG_MODE_FP32;
+    if (p->wave_grid == 0) {
+        p->wave_grid = wave_chunk(p, 4096);
+        p->wave_degrid = wave_chunk(p, 16384);
+    }
+    p->tc.degrid_chunk = p->dchunk > 0 ? (fp32 ? 32 : 1) * static_cast<int64_t>(p->dchunk) : p->wave_degrid;
+    // (a BF16x3 or FP16x3 item is one accumulation in tensor memory, whose rounding depends on its length:
+    // those keep the length that host calls and batches use)
+    p->tc.grid_chunk = p->gchunk > 0 ? (fp32 ? 4 : 1) * static_cast<int64_t>(p->gchunk)
+                       : fp32        ? p->wave_grid
+                                     : 4096;
     TRY(tc_prepare(p->tc, p->subs, p->lmn, p->c.subgrid_size, p->nch, p->dw_max, p->stream, g_last_error));
     tc_set_order(p->tc, p->mode, p->tc.want_order);
     return P9IDG_OK;
@@ -573,16 +604,25 @@ struct ZeroSide {
     }
 };
 
-// Whether nitems tensor-core work items' loader warps can zero that many 8-byte words without lengthening
-// the kernel: up to 128 KB each, of the 20 us and more that an item takes.
+// Whether nitems tensor-core work items' loader warps should zero that many 8-byte words: up to 128 KB
+// each, stores that the item's last stages and epilogue cover (1402^2, 792 items of 99 KB: a call of 38 us
+// against 51 us with the fill beside it; the batch of 12 small problems 1.03 against 1.08 ms).
 bool zero_in_kernel(int64_t words, int64_t nitems) { return words > 0 && words <= nitems * 16384; }
 
+// Whether a fill beside the gridder should take all the bandwidth it can instead of a few CTAs' worth: when
+// those few (about 2.4 TB/s) would still be filling after the gridder is done.
+bool fill_outlasts_gridder(const p9idg_plan *p, int64_t words, bool tc) {
+    const double v = static_cast<double>(p->gridded_vis), s2 = p->c.subgrid_size * p->c.subgrid_size;
+    const double gridder = tc ? 1e-5 + v * 50e-12 : v * s2 / 2.4e12;
+    return static_cast<double>(words) * 8 / 2.4e12 > gridder;
+}
+
 // Gridder over nitems work items (all of the plan's, or a group of them) into their partial slots.
-// fp32_tc: the items are the FP32 mode's tensor-core form's.
+// dev_tc: a device call on the tensor cores, whose items are the tensor-core state's.
 p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const WorkItem *d_items, int32_t nitems,
-                        bool fp32_tc = false, const ZeroFill &zero = {}) {
+                        bool dev_tc = false, const ZeroFill &zero = {}) {
     const int S = p->c.subgrid_size;
-    const int32_t nslots = fp32_tc ? p->tc.nslots : p->nslots;
+    const int32_t nslots = dev_tc ? p->tc.nslots : p->nslots;
     CK(p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, nslots)));
     StageScope t(p, P9IDG_STAGE_GRIDDER);
     GridderArgs a = gridder_args(p);
@@ -592,7 +632,7 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
     a.vis_c128 = vis_c128;
     a.partials = p->d_partials.as<float2>();
     a.zero = zero;
-    if (use_tc(p) || fp32_tc) {
+    if (use_tc(p) || dev_tc) {
         TRY(ensure_tc(p));
         TRY(tc_grid(p->tc, a, p->mode, p->stream, g_last_error));
     } else {
@@ -603,10 +643,10 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
 
 // Subgrid IFFT + adder of nsub subgrids (all, or the subgrid list d_list) into the layers.
 p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const int32_t *d_list, int32_t nsub,
-                          bool fp32_tc = false) {
+                          bool dev_tc = false) {
     StageScope t(p, P9IDG_STAGE_SUBGRID_IFFT_ADD);
     SubgridOpArgs a = subgrid_args(p);
-    if (fp32_tc) a.subs = static_cast<const DevSubgrid *>(p->tc.gsubs);
+    if (dev_tc) a.subs = static_cast<const DevSubgrid *>(p->tc.gsubs);
     a.partials = p->d_partials.as<float2>();
     a.layers = d_layers;
     a.out_shifted = true;  // IDG.cs:17,37
@@ -626,27 +666,27 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
 p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d_layers, bool wstack,
                       bool device_call = false) {
     const int nl = wstack ? p->c.wlayer_count : 1;
-    const bool fp32_tc = use_fp32_tc(p, device_call);
+    const bool dev_tc = device_call && (use_tc(p) || use_fp32_tc(p, true));
     const WorkItem *items = p->d_gitems.as<WorkItem>();
     int32_t nitems = static_cast<int32_t>(p->gitems.size());
-    if (fp32_tc) {
+    if (dev_tc) {
         TRY(ensure_tc(p));
         items = static_cast<const WorkItem *>(p->tc.gitems);
-        nitems = static_cast<int32_t>(p->tc.gitems_host.size());
+        nitems = p->tc.ngitems;
     }
     const int64_t words = static_cast<int64_t>(nl) * static_cast<int64_t>(nn_of(p));
-    if ((use_tc(p) || fp32_tc) && zero_in_kernel(words, nitems)) {
+    if (dev_tc && zero_in_kernel(words, nitems)) {
         const ZeroFill zero{reinterpret_cast<uint2 *>(d_layers), nullptr, words, (words + kZeroPiece - 1) / kZeroPiece,
                             kZeroPiece, 0};
-        TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc, zero));
+        TRY(grid_items(p, d_vis, vis_c128, items, nitems, dev_tc, zero));
     } else {
         ZeroSide z{p};
         TRY(z.fork());
-        TRY(grid_items(p, d_vis, vis_c128, items, nitems, fp32_tc));
-        CK(launch_zero_c64_beside(d_layers, words, p->zside));
+        TRY(grid_items(p, d_vis, vis_c128, items, nitems, dev_tc));
+        CK(launch_zero_c64_beside(d_layers, words, fill_outlasts_gridder(p, words, dev_tc || use_tc(p)), p->zside));
         TRY(z.join());
     }
-    return add_subgrids(p, d_layers, wstack, nullptr, 0, fp32_tc);
+    return add_subgrids(p, d_layers, wstack, nullptr, 0, dev_tc);
 }
 
 // grid (device complex64) -> vis (device, complex64 or complex128); uncovered samples are 0
@@ -1000,7 +1040,7 @@ p9idg_status host_grid_common(p9idg_plan *p, const double *vis, const double *uv
             TRY(z.fork());
             auto zero_layers = [&]() -> p9idg_status {
                 if (z.joined) return P9IDG_OK;
-                CK(launch_zero_c64_beside(layers, static_cast<int64_t>(nl * nn), p->zside));
+                CK(launch_zero_c64_beside(layers, static_cast<int64_t>(nl * nn), false, p->zside));
                 return z.join();
             };
             if (nmi > 0 || nms > 0) {
@@ -1857,10 +1897,22 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     for (int i = 0; i < nplans; i++) {
         p9idg_plan *p = plans[i];
         const int S = p->c.subgrid_size;
-        const bool tc = batch_tc(p), fp32_tc = use_fp32_tc(p, true);
+        const bool tc = batch_tc(p), fp32 = p->mode == P9IDG_MODE_FP32;
         if (tc && (st = ensure_tc(p)) != P9IDG_OK) return bail(st);
-        cudaError_t e = p->d_partials.ensure(sizeof(float2) * S * S *
-                                             std::max<size_t>(1, fp32_tc ? p->tc.nslots : p->nslots));
+        // the whole batch shares the GPU, so its tensor-core items are full-sized however small a plan is
+        std::vector<DevSubgrid> gslots, dslots;
+        std::vector<WorkItem> gwork, dwork;
+        if (tc) {
+            build_work_items(p->subs, p->nch, p->gchunk > 0 ? (fp32 ? 4 : 1) * static_cast<int64_t>(p->gchunk) : 4096,
+                             gslots, gwork);
+            build_work_items(p->subs, p->nch, p->dchunk > 0 ? (fp32 ? 32 : 1) * static_cast<int64_t>(p->dchunk) : 16384,
+                             dslots, dwork);
+        }
+        const std::vector<WorkItem> &gsrc = tc ? gwork : p->gitems, &dsrc = tc ? dwork : p->ditems;
+        // (and room for the plan's own calls, which must not move the buffer under the batch)
+        const size_t slots_max = std::max({gsrc.size(), static_cast<size_t>(p->nslots),
+                                           static_cast<size_t>(tc ? p->tc.nslots : 0), size_t(1)});
+        cudaError_t e = p->d_partials.ensure(sizeof(float2) * S * S * slots_max);
         if (e == cudaSuccess) e = p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size()));
         if (e != cudaSuccess) return bail(cuda_fail(e, "plan buffers"));
         ga[i] = gridder_args(p);
@@ -1877,7 +1929,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         // the subgrids with the slots of the items this batch runs: its own copy, as the plan's changes with
         // its work-item sizes (an offset here, the address once all are known)
         aa[i].subs = reinterpret_cast<const DevSubgrid *>(sizeof(DevSubgrid) * subs.size());
-        const std::vector<DevSubgrid> &slots = fp32_tc ? p->tc.gsubs_host : p->dsub;
+        const std::vector<DevSubgrid> &slots = tc ? gslots : p->dsub;
         subs.insert(subs.end(), slots.begin(), slots.end());
         aa[i].partials = p->d_partials.as<float2>();
         aa[i].layers = static_cast<float2 *>(d_layers[i]);
@@ -1888,23 +1940,21 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         sa[i].grid_shifted = false;
         sa[i].subgrids = p->d_subgrids.as<float2>();
         sa[i].wstack = true;
-        const std::vector<WorkItem> *dsrc = &p->ditems, *gsrc = fp32_tc ? &p->tc.gitems_host : &p->gitems;
         if (tc) {
             b->tc_order = std::max(b->tc_order, p->tc.order);
             if ((st = tc_coefs(p->tc, ga[i], p->stream, g_last_error)) != P9IDG_OK) return bail(st);
             tc_fill_args(p->tc, ga[i], tg[i]);
             tc_fill_args(p->tc, da[i], td[i]);
-            dsrc = &p->tc.ditems_host;
         }
-        for (WorkItem w : *gsrc) {
+        for (WorkItem w : gsrc) {
             w.problem = i;
             gitems.push_back(w);
         }
-        for (WorkItem w : *dsrc) {
+        for (WorkItem w : dsrc) {
             w.problem = i;
             ditems.push_back(w);
         }
-        done[i] = static_cast<int32_t>(dsrc->size());
+        done[i] = static_cast<int32_t>(dsrc.size());
         for (size_t s = 0; s < p->dsub.size(); s++) refs.push_back(make_int2(i, static_cast<int>(s)));
         bool known = false;
         for (const auto &g : b->groups) known |= g.key == group_key(p);

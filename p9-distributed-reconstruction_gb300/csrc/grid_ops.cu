@@ -12,8 +12,6 @@
 
 namespace p9idg {
 
-namespace {
-
 int sm_count() {
     static int sms = 0;
     if (sms == 0) {
@@ -24,6 +22,8 @@ int sm_count() {
     }
     return sms;
 }
+
+namespace {
 
 int grid_blocks(int64_t n, int threads) {
     const int sms = sm_count();
@@ -318,9 +318,10 @@ cudaError_t launch_zero_fill(const ZeroFill &z, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_zero_c64_beside(float2 *out, int64_t count, cudaStream_t st) {
+cudaError_t launch_zero_c64_beside(float2 *out, int64_t count, bool wide, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
-    zero_words_kernel<<<std::max(1, sm_count() / 4), 128, 0, st>>>(reinterpret_cast<uint2 *>(out), count);
+    zero_words_kernel<<<std::max(1, wide ? sm_count() * 8 : sm_count() / 4), 128, 0, st>>>(
+        reinterpret_cast<uint2 *>(out), count);
     return cudaGetLastError();
 }
 

@@ -140,6 +140,7 @@ cudaError_t launch_subgrid_ifft_add(const SubgridOpArgs &a, cudaStream_t st, con
 cudaError_t launch_split_subgrid_fft(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);
 
 // ---- launchers (grid_ops.cu) ----
+int sm_count();  // of the current device
 // c128 (unshifted, host layout) -> c64 shifted copy and, when out128 != null, c128 shifted copy.
 cudaError_t launch_shift_convert(const double2 *in, int n, float2 *out64, double2 *out128, cudaStream_t st);
 cudaError_t launch_c64_to_c128(const float2 *in, int64_t count, double2 *out, cudaStream_t st);
@@ -147,7 +148,8 @@ cudaError_t launch_c64_to_c128(const float2 *in, int64_t count, double2 *out, cu
 cudaError_t launch_zero_ranges(void *out, bool c128, const int64_t *ranges, int64_t nranges, cudaStream_t st);
 // zero-fills to run beside a tensor-core gridder or degridder: CTAs of 128 threads, at most one per SM
 cudaError_t launch_zero_ranges_beside(void *out, bool c128, const int64_t *ranges, int64_t nranges, cudaStream_t st);
-cudaError_t launch_zero_c64_beside(float2 *out, int64_t count, cudaStream_t st);
+// (wide: 8 per SM, for a fill that would outlast the gridder)
+cudaError_t launch_zero_c64_beside(float2 *out, int64_t count, bool wide, cudaStream_t st);
 // the pieces of a ZeroFill, on their own
 cudaError_t launch_zero_fill(const ZeroFill &z, cudaStream_t st);
 cudaError_t launch_zero_c128(double2 *out, int64_t count, cudaStream_t st);

@@ -1338,40 +1338,37 @@ double tc_r_max(const std::vector<float> &lmn, int S) {
     return separable_tables(lmn, S, tabs);
 }
 
-// The work items for the sizes asked for: degridder items (whole time samples, up to degrid_chunk
-// visibilities each) and, with a grid_chunk, the FP32 mode's gridder items.
+// The work items for the sizes asked for: degridder and gridder items (whole time samples, up to
+// degrid_chunk and grid_chunk visibilities each).
 static p9idg_status tc_items(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, int nch, cudaStream_t stream,
                              std::string &err) {
-    if (st.items_degrid == st.degrid_chunk && (st.grid_chunk <= 0 || st.items_grid == st.grid_chunk)) return P9IDG_OK;
+    if (st.items_degrid == st.degrid_chunk && st.items_grid == st.grid_chunk) return P9IDG_OK;
     cudaError_t e = cudaStreamSynchronize(stream);  // launches in flight read the lists replaced here
     for (void **q : {&st.ditems, &st.gitems, &st.gsubs}) {
         if (*q) cudaFree(*q);
         *q = nullptr;
     }
     st.items_degrid = st.items_grid = -1;
-    std::vector<DevSubgrid> dtmp;
-    build_work_items(subs, nch, st.degrid_chunk, dtmp, st.ditems_host);
-    st.gsubs_host.clear();
-    st.gitems_host.clear();
-    if (st.grid_chunk > 0) build_work_items(subs, nch, st.grid_chunk, st.gsubs_host, st.gitems_host);
+    std::vector<DevSubgrid> dtmp, gsubs;
+    std::vector<WorkItem> ditems, gitems;
+    build_work_items(subs, nch, st.degrid_chunk, dtmp, ditems);
+    build_work_items(subs, nch, st.grid_chunk, gsubs, gitems);
     const auto put = [&](void **dst, const auto &v) {
         using T = typename std::decay<decltype(v)>::type::value_type;
         if (e == cudaSuccess) e = device_alloc(dst, sizeof(T) * std::max<size_t>(1, v.size()));
         if (e == cudaSuccess && !v.empty())
             e = cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream);
     };
-    put(&st.ditems, st.ditems_host);
-    if (st.grid_chunk > 0) {
-        put(&st.gitems, st.gitems_host);
-        put(&st.gsubs, st.gsubs_host);
-    }
+    put(&st.ditems, ditems);
+    put(&st.gitems, gitems);
+    put(&st.gsubs, gsubs);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
         err = std::string("tensor-core work items: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
     }
-    st.nditems = static_cast<int32_t>(st.ditems_host.size());
-    st.nslots = static_cast<int32_t>(st.gitems_host.size());
+    st.nditems = static_cast<int32_t>(ditems.size());
+    st.ngitems = st.nslots = static_cast<int32_t>(gitems.size());
     st.items_degrid = st.degrid_chunk;
     st.items_grid = st.grid_chunk;
     return P9IDG_OK;

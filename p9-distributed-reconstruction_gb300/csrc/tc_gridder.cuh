@@ -24,13 +24,11 @@ struct TcPlanState {
                                   // zero past the plan's S
     void *ditems = nullptr;       // degridder work items (<= degrid_chunk visibilities)
     int32_t nditems = 0;
-    std::vector<WorkItem> ditems_host;  // the same list on the host (batches merge them)
-    // FP32 mode: its own gridder work items (<= grid_chunk visibilities; 0: none) and the subgrid list
-    // that records their slots
+    // gridder work items of the device calls (<= grid_chunk visibilities; host calls use the plan's), and
+    // the subgrid list that records their slots
     int64_t grid_chunk = 0;
     void *gitems = nullptr, *gsubs = nullptr;
-    std::vector<WorkItem> gitems_host;
-    std::vector<DevSubgrid> gsubs_host;
+    int32_t ngitems = 0;
     int64_t items_degrid = -1, items_grid = -1;  // the sizes the lists now on the device were made for
     int32_t nslots = 0;                 // partial-subgrid slots of those items (one each)
     int64_t degrid_chunk = 16384;       // visibilities per degridder work item (set before tc_prepare)
