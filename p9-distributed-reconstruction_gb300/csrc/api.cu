@@ -643,7 +643,7 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
 
 // Subgrid IFFT + adder of nsub subgrids (all, or the subgrid list d_list) into the layers.
 p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const int32_t *d_list, int32_t nsub,
-                          bool dev_tc = false) {
+                          bool dev_tc = false, bool device_call = false) {
     StageScope t(p, P9IDG_STAGE_SUBGRID_IFFT_ADD);
     SubgridOpArgs a = subgrid_args(p);
     if (dev_tc) a.subs = static_cast<const DevSubgrid *>(p->tc.gsubs);
@@ -651,6 +651,7 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
     a.layers = d_layers;
     a.out_shifted = true;  // IDG.cs:17,37
     a.wstack = wstack;
+    a.keep_bits = !device_call;
     if (d_list) {
         a.sub_list = d_list;
         a.nsub = nsub;
@@ -686,7 +687,7 @@ p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d
         CK(launch_zero_c64_beside(d_layers, words, fill_outlasts_gridder(p, words, dev_tc || use_tc(p)), p->zside));
         TRY(z.join());
     }
-    return add_subgrids(p, d_layers, wstack, nullptr, 0, dev_tc);
+    return add_subgrids(p, d_layers, wstack, nullptr, 0, dev_tc, device_call);
 }
 
 // grid (device complex64) -> vis (device, complex64 or complex128); uncovered samples are 0
@@ -716,6 +717,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.grid_shifted = grid_shifted;
         a.subgrids = p->d_subgrids.as<float2>();
         a.wstack = wstack;
+        a.keep_bits = out_c128;
         CK(launch_split_subgrid_fft(a, p->stream));
     }
     if (!out_in_host && !fused) CK(launch_zero_ranges_beside(d_vis, out_c128, p->d_gaps.as<int64_t>(), ngaps, p->zside));

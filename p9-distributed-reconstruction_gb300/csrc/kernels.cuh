@@ -134,7 +134,8 @@ struct SubgridOpArgs {
     int32_t *status;
     const int2 *refs;          // batched launches: (problem, subgrid) per block; nsub = count
     const int32_t *sub_list;   // own launches: subgrid index per block (null: the block index)
-    const float2 *twiddles;    // exp(+2 pi i j / S), j < S, made in FP64 (null: the kernels make them)
+    const float2 *twiddles;    // exp(+2 pi i j / S), j < S, made in FP64 (null, with keep_bits: made there)
+    bool keep_bits;            // host-array calls: the form whose results those keep
 };
 cudaError_t launch_subgrid_ifft_add(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);
 cudaError_t launch_split_subgrid_fft(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);
