@@ -10,17 +10,13 @@
 //
 // Coordinate descent.  One iteration of FastSerialCD picks the pixel whose proximal update
 // changes it most (a scan of the whole image), sets it, and adds the scaled PSF^2 to the
-// gradient map in a window around it.  Only pixels in that window change, so the GPU keeps
-// the best candidate of every 40 x 128 tile and, per iteration, re-evaluates only the tiles
-// the window touches: one launch reduces the tile candidates the previous launch left to the
-// selected pixel (every CTA does this itself), updates the window's gradients and writes those
-// tiles' new candidates into the other of two state buffers.  A candidate is one 64-bit key,
-// (|change| bits << 32) | (0xFFFFFFFF - pixel index), so the largest key is the largest change
-// and, among equal changes, the first pixel, which is the order in which GetAbsMax
-// (FastSerialCD.cs:135-170) keeps its winner.  Iterations are launched from a captured CUDA
-// graph, 32 at a time, each chained to the previous by programmatic dependent launch; a launch
-// after the stopping iteration does nothing, so the iteration count and result equal the
-// reference's loop.
+// gradient map in a window around it.  Only pixels in that window change, so the GPU keeps the
+// best candidate of every 40 x 128 tile (one for each warp's rows of it) and re-evaluates only the
+// rows that the window touches.  A candidate is ordered by one 64-bit key, (|change| bits << 32) |
+// (0xFFFFFFFF - pixel index), so the largest key is the largest change and, among equal changes,
+// the first pixel, which is the order in which GetAbsMax (FastSerialCD.cs:135-170) keeps its
+// winner.  The iterations run inside one cooperative launch whose CTAs own fixed tiles and
+// exchange nothing but their best candidates (cd_run_kernel).
 
 #include <cuda_runtime.h>
 #include <cufft.h>
@@ -111,268 +107,468 @@ __device__ __forceinline__ float cs_maxf(float a, float b) {
     return signbit(b) ? a : b;
 }
 
-// ElasticNet.ProximalOperator (Common.cs:28-29), un-fused.
-__device__ __forceinline__ float prox(float x, float lipschitz, float lambda, float alpha) {
-    const float num = cs_maxf(__fsub_rn(x, __fmul_rn(lambda, alpha)), 0.0f);
-    const float den = __fadd_rn(lipschitz, __fmul_rn(lambda, __fsub_rn(1.0f, alpha)));
-    return __fdiv_rn(num, den);
+// ElasticNet.ProximalOperator (Common.cs:28-29), un-fused: thr = lambda * alpha and slope = lambda *
+// (1 - alpha), each rounded as the reference rounds it.  max(v, 0) is Math.Max
+// as above: NaN stays, -0 becomes +0.  Most pixels of a sparse model are held at zero by the
+// threshold, and 0 / den is +0 for every positive den, so a warp of such pixels makes no division.
+__device__ __forceinline__ float prox(float x, float lipschitz, float thr, float slope) {
+    const float v = __fsub_rn(x, thr);
+    const float den = __fadd_rn(lipschitz, slope);
+    if (v <= 0.0f && den > 0.0f) return 0.0f;
+    return __fdiv_rn(v <= 0.0f ? 0.0f : v, den);
 }
 
 constexpr int kNT = 512, kWarps = kNT / 32;  // image reductions
-// Coordinate descent: tiles of kTY x kTX pixels, one CTA of kCdNT threads per tile (8 pixels a
-// thread).  A 768^2 update window (a 384^2 PSF) spans 21 x 7 = 147 such tiles, one CTA per SM of
-// the 152, each evaluating 5,120 pixels; 32 x 128 tiles of 512 threads need 175 CTAs, two on some
-// SMs, and the 3072^2 major cycle's coordinate descent ran 19 % slower with them.
-constexpr int kTY = 40, kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32, kCdBlocksPerSM = 1;
-// Even: every replay ends on state buffer 0.  Launches past the stopping one are spent for nothing, up
-// to two replays' worth (the rest of its own and the one in flight); 1000 iterations at 3072^2 took
-// 7.33 ms with 256 a replay and one replay too many, and take 6.50 ms with 16 or 32 a replay (6.69
-// with 8, 6.76 to 6.79 with 64 to 256).
-constexpr int kGraphIters = 32;
+// Coordinate descent: tiles of kTY x kTX pixels, CTAs of kCdNT threads, each warp two rows of a tile.
+// A 768^2 update window (a 384^2 PSF) spans 21 x 7 = 147 such tiles, one for each CTA of the 152 SMs.
+constexpr int kTY = 40, kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32;
+constexpr int kCdRows = kTY / kCdWarps, kCdCols = kTX / 32;  // pixels a thread: rows x columns
+// Slots of the exchange, three for each lane of the polling warp; pairs of CTAs share one from
+// kCdPairFrom CTAs on.  Measured for the exchange alone: 1270 clocks with 30 CTAs, each polling every
+// slot, 3500 with 147 (the polls of one line queue up), 2490 with 74 pairs; pairs of 30 take 2040.
+constexpr int kCdPoll = 3, kCdSlots = 32 * kCdPoll, kCdPairFrom = 56;
+// Iterations of one launch: few enough that other streams' kernels wait milliseconds for the SMs, not
+// for a whole deconvolution, and enough that a launch does not show.
+constexpr int kCdLaunchIters = 512;
+// Clocks (about 4 s) after which a CTA gives up waiting for another.  All CTAs of a cooperative launch are
+// resident, so this is only met if one of them cannot run.
+constexpr long long kCdPatience = 8000000000ll;
 
 struct CdCtl {  // the state one launch hands to the next
     int32_t iter, done, converged, error;
 };
 
-struct CdParams {  // device-resident, read by every launch (so one captured graph serves all calls)
+// A candidate: x = |change| bits, y = 0xFFFFFFFF - (row << 16 | column), z = new value, w = current value;
+// all zero for "none".  (x, y) is the key, larger is better: the largest change, and of equal changes the
+// first pixel in row-major order.
+using CdCand = uint4;
+
+struct CdParams {
     float *x, *g;
     const float *a, *psf2;
-    unsigned long long *tile_key;  // [2][ntiles]: best key of each tile (double-buffered by launch parity)
-    float2 *tile_val;              // [2][ntiles]: (new value, current value) of each tile's best pixel
-    CdCtl *ctl;                    // [2]
+    CdCand *cand;                  // [tile][warp]
+    unsigned long long *tile_key;  // best key of each tile, left by the scan
+    uint4 *slots;                  // [2][kCdSlots]: (epoch, candidate's y, z, w)
+    CdCtl *ctl;
+    CdCtl *report;  // pinned: [0] the state a launch leaves, [1].error set by a CTA that gave up
     int32_t n, ph, pw, tiles_x, tiles_y, max_iter;
+    int32_t ax, ay;              // tile (ty, tx) belongs to CTA (ty % ay) * ax + tx % ax
+    uint32_t inv_ax, inv_ay;     // ceil(2^31 / ax): q / ax = q * inv_ax >> 31 for q below 2^11
+    int32_t local_x, local_tiles;  // tiles of one CTA: in a row, in all (at most)
     float lambda, alpha, eps;
-    int32_t pad;
 };
 
-// Max of a 64-bit key over the warp as two 32-bit hardware reductions: the high words, then the
-// low words of the lanes holding the highest one (the same lexicographic maximum).
-__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
-    const unsigned hi = static_cast<unsigned>(v >> 32);
+// Max of a 64-bit key (hi, lo) over the warp as two 32-bit hardware reductions: the high words, then
+// the low words of the lanes holding the highest one (the same lexicographic maximum).
+__device__ __forceinline__ uint2 warp_max(unsigned hi, unsigned lo) {
     const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? static_cast<unsigned>(v) : 0u);
-    return (static_cast<unsigned long long>(mh) << 32) | ml;
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return make_uint2(mh, ml);
 }
 
-// Block-wide max with one barrier: every warp reduces the per-warp results itself.  sm[kCdWarps]
-// must not be reused by the same CTA afterwards (each call site has its own array).
-__device__ unsigned long long block_max(unsigned long long v, unsigned long long *sm) {
-    static_assert(kCdWarps <= 32, "one warp reduces the per-warp results");
-    v = warp_max(v);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+__device__ __forceinline__ CdCand better(const CdCand &a, const CdCand &b) {
+    return a.x > b.x || (a.x == b.x && a.y > b.y) ? a : b;
+}
+
+// The lane that holds the warp's best candidate (pixels are unique; of lanes without any, the first).
+__device__ __forceinline__ int best_lane(const CdCand &c) {
+    const uint2 m = warp_max(c.x, c.y);
+    return __ffs(__ballot_sync(0xffffffffu, c.x == m.x && c.y == m.y)) - 1;
+}
+
+// One 16-byte access that no other can split: a packet carries its own epoch, so a reader that finds
+// the epoch it waits for has the packet's other words too, without a fence.
+__device__ __forceinline__ void st_packet(uint4 *p, const uint4 &v) {
+    const unsigned long long lo = v.x | (static_cast<unsigned long long>(v.y) << 32),
+                             hi = v.z | (static_cast<unsigned long long>(v.w) << 32);
+    asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(p), "l"(lo), "l"(hi)
+                 : "memory");
+}
+
+__device__ __forceinline__ uint4 ld_packet(const uint4 *p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n.reg .b128 q;\nld.relaxed.gpu.global.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}\n" : "=l"(lo), "=l"(hi) : "l"(p)
+                 : "memory");
+    return make_uint4(static_cast<unsigned>(lo), static_cast<unsigned>(lo >> 32), static_cast<unsigned>(hi),
+                      static_cast<unsigned>(hi >> 32));
+}
+
+__device__ __forceinline__ uint32_t cd_shared(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+__device__ __forceinline__ uint32_t cd_peer(uint32_t addr, unsigned rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
+// 16 bytes into another CTA's shared memory; they count towards that CTA's barrier when they are there.
+__device__ __forceinline__ void cd_st_peer(uint32_t dst, uint32_t bar, const uint4 &v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(v.x),
+                 "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cd_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void cd_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase) {
+    long long t0 = 0;
+    while (true) {
+        uint32_t done;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(phase)
+            : "memory");
+        if (done) return true;
+        const long long t = clock64();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kCdPatience) return false;
+    }
+}
+
+__device__ __forceinline__ void cd_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct Window {
+    int py, px, y0, y1, x0, x1;
+    float xnew, xdiff;
+};
+
+// Evaluates (and with UPDATE first updates) this warp's rows of one tile; returns this thread's best
+// candidate.  All of a thread's loads are issued before any is used (predicated, no early exits), so
+// the rows cost one memory latency rather than one per pixel.
+template <bool UPDATE>
+__device__ __forceinline__ CdCand eval_rows(const CdParams &P, float thr, float slope, int ty, int tx, const Window &w) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int yb = ty * kTY + warp * kCdRows, xb = tx * kTX + lane;
+    bool in[kCdRows][kCdCols], upd[kCdRows][kCdCols];
+    float gv[kCdRows][kCdCols], xv[kCdRows][kCdCols], av[kCdRows][kCdCols], pv[kCdRows][kCdCols];
+    float *gp[kCdRows];
+#pragma unroll
+    for (int r = 0; r < kCdRows; r++) {
+        const int y = yb + r;
+        const size_t i0 = static_cast<size_t>(y) * P.n + xb;
+        gp[r] = P.g + i0;
+        const float *xp = P.x + i0, *ap = P.a + i0;
+        const float *pp = P.psf2 + (static_cast<int64_t>(y + P.ph / 2 - w.py) * P.pw + (xb + P.pw / 2 - w.px));
+#pragma unroll
+        for (int k = 0; k < kCdCols; k++) {
+            const int xc = xb + 32 * k;
+            in[r][k] = y < P.n && xc < P.n;
+            upd[r][k] = UPDATE && y >= w.y0 && y < w.y1 && xc >= w.x0 && xc < w.x1;
+            gv[r][k] = in[r][k] ? gp[r][32 * k] : 0.0f;
+            xv[r][k] = in[r][k] ? xp[32 * k] : 0.0f;
+            av[r][k] = in[r][k] ? __ldg(ap + 32 * k) : 1.0f;
+            pv[r][k] = upd[r][k] ? __ldg(pp + 32 * k) : 0.0f;
+        }
+        if (UPDATE && y == w.py) {  // the selected pixel takes its new value
+#pragma unroll
+            for (int k = 0; k < kCdCols; k++)
+                if (xb + 32 * k == w.px) {
+                    xv[r][k] = w.xnew;
+                    P.x[i0 + 32 * k] = w.xnew;
+                }
+        }
+    }
+    float bd = 0.0f, bnew = 0.0f, bold = 0.0f;
+    uint32_t bi = 0xFFFFFFFFu;
+#pragma unroll
+    for (int r = 0; r < kCdRows; r++) {
+#pragma unroll
+        for (int k = 0; k < kCdCols; k++) {
+            float g = gv[r][k];
+            if (UPDATE && upd[r][k]) {
+                g = __fadd_rn(g, __fmul_rn(pv[r][k], w.xdiff));  // gradients[i, j] += psf2 * xDiff
+                gp[r][32 * k] = g;
+            }
+            const float a = av[r][k], old = xv[r][k];
+            const float xt = prox(__fadd_rn(__fmul_rn(old, a), g), a, thr, slope);
+            const float d = fabsf(__fsub_rn(old, xt));
+            if (in[r][k] && d > bd) {  // pixels in index order: the first of equal changes stays
+                bd = d;
+                bnew = xt;
+                bold = old;
+                bi = (static_cast<uint32_t>(yb + r) << 16) | static_cast<uint32_t>(xb + 32 * k);
+            }
+        }
+    }
+    return make_uint4(__float_as_uint(bd), 0xFFFFFFFFu - bi, __float_as_uint(bnew), __float_as_uint(bold));
+}
+
+// Full scan (GetAbsMax over the whole image): every warp's candidate of every tile, and each tile's best key.
+__global__ void __launch_bounds__(kCdNT) cd_scan_kernel(const __grid_constant__ CdParams P) {
+    __shared__ uint2 sm[kCdWarps];
+    const float thr = __fmul_rn(P.lambda, P.alpha), slope = __fmul_rn(P.lambda, __fsub_rn(1.0f, P.alpha));
+    const Window w{};
+    const CdCand c = eval_rows<false>(P, thr, slope, blockIdx.y, blockIdx.x, w);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.y * P.tiles_x + blockIdx.x;
+    if (lane == best_lane(c)) {
+        P.cand[t * static_cast<int64_t>(kCdWarps) + warp] = c;
+        sm[warp] = make_uint2(c.x, c.y);
+    }
     __syncthreads();
-    const unsigned lane = threadIdx.x & 31;
-    return warp_max(lane < kCdWarps ? sm[lane] : 0ull);
+    if (warp == 0) {
+        const uint2 v = lane < kCdWarps ? sm[lane] : make_uint2(0u, 0u);
+        const uint2 m = warp_max(v.x, v.y);
+        if (lane == 0) P.tile_key[t] = (static_cast<unsigned long long>(m.x) << 32) | m.y;
+    }
+    if (t == 0) {
+        if (threadIdx.x == 0) *P.ctl = CdCtl{0, 0, 0, 0};
+        if (threadIdx.x < 2 * kCdSlots) P.slots[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
-// The best key over all tiles of one buffer (8 loads in flight per thread: one round up to
-// 4096 tiles, e.g. a 4096^2 image).
-__device__ unsigned long long reduce_tiles(const unsigned long long *keys, int ntiles, unsigned long long *sm) {
+// The largest key of the scan (GetAbsMax's result), for the host.
+__global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const unsigned long long *keys, int ntiles, unsigned long long *out) {
+    __shared__ uint2 sm[kCdWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned long long best = 0;
     for (int base = 0; base < ntiles; base += 8 * kCdNT) {
         unsigned long long v[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const int t = base + j * kCdNT + static_cast<int>(threadIdx.x);
-            v[j] = t < ntiles ? __ldcg(keys + t) : 0ull;
+            v[j] = t < ntiles ? keys[t] : 0ull;
         }
 #pragma unroll
         for (int j = 0; j < 8; j++) best = v[j] > best ? v[j] : best;
     }
-    return block_max(best, sm);
-}
-
-struct Window {
-    uint32_t sel;  // selected pixel index
-    int py, px, y0, y1, x0, x1, yh, xh;
-};
-
-// Evaluates (and with UPDATE first updates) one tile; writes its best key and values.  All of a
-// thread's loads are issued before any is used (predicated, no early exits), so a tile costs one
-// memory latency rather than one per pixel.
-template <bool UPDATE>
-__device__ void eval_tile(const CdParams &P, float lambda, float alpha, int ty, int tx, const Window &w,
-                          const float2 *sel_val, unsigned long long *key_out, float2 *val_out,
-                          unsigned long long *sm) {
-    constexpr int R = kTY / kCdWarps, K = kTX / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int yb = ty * kTY + warp * R, xb = tx * kTX + lane;
-    // the selected pixel's (new, current) values: every thread loads them beside its pixels (one
-    // request per warp), so no block barrier is needed to share them
-    float2 sv = make_float2(0.0f, 0.0f);
-    if (UPDATE) sv = __ldcg(sel_val);
-    float gv[R][K], xv[R][K], av[R][K], pv[R][K];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const int y = yb + r, xc = xb + 32 * k;
-            const bool in = y < P.n && xc < P.n;
-            const uint32_t i = static_cast<uint32_t>(y) * static_cast<uint32_t>(P.n) + static_cast<uint32_t>(xc);
-            gv[r][k] = 0.0f;
-            xv[r][k] = 0.0f;
-            av[r][k] = 1.0f;
-            pv[r][k] = 0.0f;
-            if (in) {
-                gv[r][k] = P.g[i];
-                xv[r][k] = P.x[i];
-                av[r][k] = __ldg(P.a + i);
-            }
-            if (UPDATE && in && y >= w.y0 && y < w.y1 && xc >= w.x0 && xc < w.x1)
-                pv[r][k] = __ldg(P.psf2 + static_cast<int64_t>(y + w.yh - w.py) * P.pw + (xc + w.xh - w.px));
-        }
-    }
-    float xnew = 0.0f, xdiff = 0.0f;
-    if (UPDATE) {
-        xnew = sv.x;
-        xdiff = __fsub_rn(sv.y, sv.x);  // pixelOld - maxPixel.PixelNew
-    }
-    unsigned long long best = 0;
-    float bnew = 0.0f, bold = 0.0f;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const int y = yb + r, xc = xb + 32 * k;
-            if (y >= P.n || xc >= P.n) continue;
-            const uint32_t i = static_cast<uint32_t>(y) * static_cast<uint32_t>(P.n) + static_cast<uint32_t>(xc);
-            float g = gv[r][k], old = xv[r][k];
-            if (UPDATE) {
-                if (y >= w.y0 && y < w.y1 && xc >= w.x0 && xc < w.x1) {
-                    g = __fadd_rn(g, __fmul_rn(pv[r][k], xdiff));  // gradients[i, j] += psf2 * xDiff
-                    P.g[i] = g;
-                }
-                if (i == w.sel) {
-                    old = xnew;
-                    P.x[i] = xnew;
-                }
-            }
-            const float a = av[r][k];
-            const float xt = prox(__fadd_rn(__fmul_rn(old, a), g), a, lambda, alpha);
-            const float d = fabsf(__fsub_rn(old, xt));
-            const unsigned long long key =
-                (0.0f < d) ? ((static_cast<unsigned long long>(__float_as_uint(d)) << 32) | (0xFFFFFFFFu - i)) : 0ull;
-            if (key > best) {
-                best = key;
-                bnew = xt;
-                bold = old;
-            }
-        }
-    }
-    const unsigned long long m = block_max(best, sm);
-    const int t = ty * P.tiles_x + tx;
-    if (threadIdx.x == 0) key_out[t] = m;
-    if (m != 0ull && best == m) val_out[t] = make_float2(bnew, bold);
-}
-
-// Full scan into state buffer 0: the candidate of every tile (GetAbsMax over the whole image).
-__global__ void __launch_bounds__(kCdNT) cd_scan_kernel(const CdParams *pp, float lambda, float alpha) {
-    __shared__ unsigned long long sm[kCdWarps];
-    const CdParams P = *pp;
-    Window w{};
-    eval_tile<false>(P, lambda, alpha, blockIdx.y, blockIdx.x, w, nullptr, P.tile_key, P.tile_val, sm);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) P.ctl[0] = CdCtl{0, 0, 0, 0};
-}
-
-// The selected pixel's key and values of state buffer 0 (GetAbsMax's result), for the host.
-__global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const CdParams *pp, unsigned long long *out_key, float2 *out_val) {
-    __shared__ unsigned long long sm[kCdWarps];
-    const CdParams P = *pp;
-    const unsigned long long best = reduce_tiles(P.tile_key, P.tiles_x * P.tiles_y, sm);
-    if (threadIdx.x == 0) {
-        *out_key = best;
-        float2 v = make_float2(0.0f, 0.0f);
-        if (best) {
-            const uint32_t idx = 0xFFFFFFFFu - static_cast<uint32_t>(best);
-            v = P.tile_val[static_cast<int>((idx / P.n) / kTY) * P.tiles_x + static_cast<int>((idx % P.n) / kTX)];
-        }
-        *out_val = v;
+    const uint2 m = warp_max(static_cast<unsigned>(best >> 32), static_cast<unsigned>(best));
+    if (lane == 0) sm[warp] = m;
+    __syncthreads();
+    if (warp == 0) {
+        const uint2 v = lane < kCdWarps ? sm[lane] : make_uint2(0u, 0u);
+        const uint2 a = warp_max(v.x, v.y);
+        if (lane == 0) *out = (static_cast<unsigned long long>(a.x) << 32) | a.y;
     }
 }
 
-// One coordinate-descent iteration (FastSerialCD.cs:83-98).  Launch k reads state buffer k % 2
-// (tile candidates and control) and writes buffer (k + 1) % 2: the window's tiles re-evaluated,
-// every other tile's candidate copied.  Each CTA finds the selected pixel itself from the input
-// buffer, so a launch needs no grid-wide synchronisation.
+// Up to kCdLaunchIters coordinate-descent iterations (FastSerialCD.cs:83-98) in one cooperative launch.
 //
-// The fixed fields (state buffers, maps, sizes) are a kernel parameter captured with the graph,
-// so the first loads of a launch (the tile keys) need no pointer loaded from memory first; the
-// per-call fields (images, lambda, alpha, eps, iteration cap) come from pp, which only the host
-// writes before the graph is launched.
-__global__ void __launch_bounds__(kCdNT, kCdBlocksPerSM)
-    cd_iter_kernel(const __grid_constant__ CdParams F, const CdParams *pp, int parity, CdCtl *report) {
-    __shared__ unsigned long long sm_in[kCdWarps], sm_out[kCdWarps];
-    __shared__ CdCtl c;
-    CdParams P = F;
-    P.x = pp->x;
-    P.g = pp->g;
-    P.lambda = pp->lambda;
-    P.alpha = pp->alpha;
-    P.eps = pp->eps;
-    P.max_iter = pp->max_iter;
-    // Programmatic dependent launch: this grid is launched while the previous iteration finishes
-    // (each CTA of that grid releases it as its last step) and waits here until that grid has
-    // completed and its candidates and control are visible.  Nothing the previous grid writes is
-    // read before the wait.  Releasing at the end rather than the start measured faster: early
-    // waiting CTAs cost ~2 us per iteration when most of the window lies outside the image.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int ntiles = P.tiles_x * P.tiles_y;
-    const unsigned long long *kin = P.tile_key + static_cast<int64_t>(parity) * ntiles;
-    const float2 *vin = P.tile_val + static_cast<int64_t>(parity) * ntiles;
-    unsigned long long *kout = P.tile_key + static_cast<int64_t>(1 - parity) * ntiles;
-    float2 *vout = P.tile_val + static_cast<int64_t>(1 - parity) * ntiles;
-    const CdCtl *cin = P.ctl + parity;
-    CdCtl *cout = P.ctl + (1 - parity);
-    if (threadIdx.x == 0) c = *cin;
-    // the last launch of a replay hands the state it leaves to the host (pinned memory; null otherwise)
-    const auto leave = [&](const CdCtl &v) {
-        *cout = v;
-        if (report) *report = v;
-    };
-    const unsigned long long key = reduce_tiles(kin, ntiles, sm_in);  // its barrier publishes c
-    const bool lead = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
-    if (c.done) {
-        if (lead) leave(c);
+// An iteration is a latency chain: agree on the pixel, load the window, update and re-evaluate it, find
+// the new candidates.  The only thing that CTAs need of each other is the best candidate, so a tile
+// belongs to the same CTA (and a pixel to the same thread) throughout, the tiles dealt out as a torus of
+// ay x ax CTAs: a window of at most that many tiles gives no CTA two of them.
+//
+// The exchange: every warp puts its best candidate into its cluster's first CTA (a cluster is one CTA or
+// a pair), whose first warp posts the best of them as one 16-byte packet that carries the iteration's
+// number, reads every cluster's packet until all carry it, and hands the best to the cluster's warps.  No
+// fence, atomic or grid-wide counter is needed, and gradients and model stay out of it.  Buffers and
+// slots alternate between two sets: a slot is overwritten only after every cluster has posted the
+// iteration after it, hence read it.
+//
+// A lane keeps in registers the candidate of its warp's rows of local tile `lane`; images of more than 32
+// tiles a CTA (4864 tiles, about 5000^2) keep them in P.cand, which only this warp touches.
+__global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant__ CdParams P) {
+    __shared__ CdCand sm_in[2][2 * kCdWarps];  // candidates of the cluster's warps (first CTA)
+    __shared__ CdCand sm_sel[2];               // the selected candidate
+    __shared__ unsigned long long bar_in[2], bar_sel[2];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const CdCtl c0 = *P.ctl;
+    if (c0.done) {  // the same for all CTAs: an earlier launch wrote it
+        if (blockIdx.x == 0 && threadIdx.x == 0) P.report[0] = c0;
         return;
     }
-    if (c.iter >= P.max_iter) {  // while (!converged & iter < iterations)
-        if (lead) leave(CdCtl{c.iter, 1, 0, 0});
-        return;
-    }
-    const float diff = __uint_as_float(static_cast<uint32_t>(key >> 32));
-    if (diff < P.eps) {  // converged = maxPixel.PixelMaxDiff < epsilon
-        if (lead) leave(CdCtl{c.iter, 1, 1, 0});
-        return;
-    }
-    if (key == 0ull) {  // the reference would index pixel (-1, -1)
-        if (lead) leave(CdCtl{c.iter, 1, 0, 1});
-        return;
-    }
-    Window w;
-    w.sel = 0xFFFFFFFFu - static_cast<uint32_t>(key);
-    w.py = static_cast<int>(w.sel / P.n);
-    w.px = static_cast<int>(w.sel % P.n);
-    w.yh = P.ph / 2;
-    w.xh = P.pw / 2;
-    w.y0 = max(w.py - w.yh, 0);
-    w.x0 = max(w.px - w.xh, 0);
-    w.y1 = min(w.py - w.yh + P.ph, P.n);
-    w.x1 = min(w.px - w.xh + P.pw, P.n);
-    const int ty0 = w.y0 / kTY, ty1 = (w.y1 - 1) / kTY, tx0 = w.x0 / kTX, tx1 = (w.x1 - 1) / kTX;
-    // candidates of the tiles outside the window carry over unchanged
-    const int nb = gridDim.x * gridDim.y, b = blockIdx.y * gridDim.x + blockIdx.x;
-    for (int t = b + nb * static_cast<int>(threadIdx.x); t < ntiles; t += nb * kCdNT) {
-        const int tty = t / P.tiles_x, ttx = t % P.tiles_x;
-        if (tty < ty0 || tty > ty1 || ttx < tx0 || ttx > tx1) {
-            kout[t] = __ldcg(kin + t);
-            vout[t] = __ldcg(vin + t);
+    unsigned rank, csize;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+    const bool pair = csize == 2;
+    const int nslots = static_cast<int>(gridDim.x / csize), slot = static_cast<int>(blockIdx.x / csize);
+    const uint32_t in_bar = cd_shared(bar_in), sel_bar = cd_shared(bar_sel);
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < 2; b++) {
+            // candidates: an arrival of each warp here, and in a pair the bytes of the other CTA's warps
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(in_bar + 8 * b), "r"(kCdWarps + (pair ? 1 : 0)));
+            // selection: an arrival of the first warp, or the bytes that it sends to the second CTA
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sel_bar + 8 * b));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int b = 0; b < 2; b++) {
+            if (pair && rank == 0) cd_expect(in_bar + 8 * b, kCdWarps * sizeof(CdCand));
+            if (rank == 1) cd_expect(sel_bar + 8 * b, sizeof(CdCand));
         }
     }
-    const float2 *sel_val = vin + static_cast<int>(w.py / kTY) * P.tiles_x + static_cast<int>(w.px / kTX);
-    const int ty = ty0 + static_cast<int>(blockIdx.y), tx = tx0 + static_cast<int>(blockIdx.x);
-    if (ty <= ty1 && tx <= tx1) eval_tile<true>(P, P.lambda, P.alpha, ty, tx, w, sel_val, kout, vout, sm_out);
-    if (lead) leave(CdCtl{c.iter + 1, 0, 0, 0});
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the next iteration may launch
+    if (pair)
+        cd_cluster_sync();
+    else
+        __syncthreads();
+
+    const int cta = blockIdx.x, cy = static_cast<int>(static_cast<uint32_t>(cta) / static_cast<uint32_t>(P.ax)), cx = cta - cy * P.ax;
+    const bool owner = cy < P.ay;  // the last CTA of an odd number in pairs owns nothing
+    const bool in_regs = P.local_tiles <= 32;
+    const CdCand none = make_uint4(0u, 0u, 0u, 0u);
+    // this warp's candidate of local tile l = (ty / ay) * local_x + tx / ax; null past the image
+    const auto at = [&](int l) -> CdCand * {
+        const int q = l / P.local_x, ty = cy + q * P.ay, tx = cx + (l - q * P.local_x) * P.ax;
+        return owner && l < P.local_tiles && ty < P.tiles_y && tx < P.tiles_x
+                   ? P.cand + (static_cast<int64_t>(ty) * P.tiles_x + tx) * kCdWarps + warp
+                   : nullptr;
+    };
+    const auto scan_held = [&]() {
+        CdCand h = none;
+        for (int l = lane; l < P.local_tiles; l += 32)
+            if (const CdCand *p = at(l)) h = better(*p, h);
+        return h;
+    };
+    CdCand held = scan_held();  // best of the local tiles l = lane mod 32
+    CdCand best = held;         // what this thread has to offer
+    CdCand fresh = none;        // its candidate of local tile fresh_tile, not yet in held
+    int fresh_tile = -1;
+    const auto settle = [&]() {
+        if (fresh_tile < 0) return;
+        const int o = best_lane(fresh);
+        const CdCand t = make_uint4(__shfl_sync(0xffffffffu, fresh.x, o), __shfl_sync(0xffffffffu, fresh.y, o),
+                                    __shfl_sync(0xffffffffu, fresh.z, o), __shfl_sync(0xffffffffu, fresh.w, o));
+        if (lane == fresh_tile) held = t;
+        fresh_tile = -1;
+    };
+    const float thr = __fmul_rn(P.lambda, P.alpha), slope = __fmul_rn(P.lambda, __fsub_rn(1.0f, P.alpha));
+    CdCtl c{c0.iter, 0, 0, 0};
+    for (int step = 0;; step++) {
+        if (c.iter >= P.max_iter) {  // while (!converged & iter < iterations)
+            c.done = 1;
+            break;
+        }
+        if (step == kCdLaunchIters) break;
+        const int b = step & 1;
+        const uint32_t phase = (step >> 1) & 1, in_b = in_bar + 8 * b, sel_b = sel_bar + 8 * b;
+        bool ok = true;
+        if (lane == best_lane(best)) {
+            if (rank == 0) {
+                sm_in[b][warp] = best;
+                cd_arrive(in_b);
+            } else {
+                cd_st_peer(cd_peer(cd_shared(&sm_in[b][kCdWarps + warp]), 0), cd_peer(in_b, 0), best);
+            }
+        }
+        if (rank == 0 && warp == 0) {
+            ok = __all_sync(0xffffffffu, cd_wait(in_b, phase));
+            if (ok) {
+                uint4 *slots = P.slots + (c.iter & 1) * kCdSlots;
+                const unsigned epoch = static_cast<unsigned>(c.iter) + 1u;
+                CdCand v = lane < kCdWarps ? sm_in[b][lane] : none;
+                if (pair) {
+                    if (lane < kCdWarps) v = better(v, sm_in[b][kCdWarps + lane]);
+                    if (lane == 0) cd_expect(in_b, kCdWarps * sizeof(CdCand));
+                }
+                if (lane == best_lane(v)) st_packet(slots + slot, make_uint4(epoch, v.y, v.z, v.w));
+                v = none;
+                unsigned want = 0;
+#pragma unroll
+                for (int j = 0; j < kCdPoll; j++) want |= lane + 32 * j < nslots ? 1u << j : 0u;
+                const long long t0 = clock64();
+                while (true) {
+                    uint4 q[kCdPoll];
+#pragma unroll
+                    for (int j = 0; j < kCdPoll; j++)
+                        q[j] = (want >> j) & 1u ? ld_packet(slots + lane + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                    for (int j = 0; j < kCdPoll; j++) {
+                        if (q[j].x != epoch) continue;  // epochs start at 1
+                        want &= ~(1u << j);
+                        // |change| is not sent: it is the difference of the two values
+                        q[j].x = __float_as_uint(fabsf(__fsub_rn(__uint_as_float(q[j].w), __uint_as_float(q[j].z))));
+                        v = better(q[j], v);
+                    }
+                    if (!__any_sync(0xffffffffu, want != 0u)) break;
+                    if (__any_sync(0xffffffffu, clock64() - t0 > kCdPatience)) {
+                        ok = false;
+                        break;
+                    }
+                }
+                if (ok && lane == best_lane(v)) {
+                    if (pair) cd_st_peer(cd_peer(cd_shared(&sm_sel[b]), 1), cd_peer(sel_b, 1), v);
+                    sm_sel[b] = v;
+                    cd_arrive(sel_b);
+                }
+            }
+        }
+        settle();  // while the exchange is under way
+        ok = __all_sync(0xffffffffu, ok && cd_wait(sel_b, phase));
+        if (!ok) {
+            c = CdCtl{c.iter, 1, 0, 2};
+            if (lane == 0) P.report[1].error = 2;
+            break;
+        }
+        if (rank == 1 && threadIdx.x == 0) cd_expect(sel_b, sizeof(CdCand));
+        const CdCand s = sm_sel[b];
+        if (__uint_as_float(s.x) < P.eps) {  // converged = maxPixel.PixelMaxDiff < epsilon
+            c = CdCtl{c.iter, 1, 1, 0};
+            break;
+        }
+        if (s.y == 0u) {  // none: the reference would index pixel (-1, -1)
+            c = CdCtl{c.iter, 1, 0, 1};
+            break;
+        }
+        c.iter++;
+        if (!owner) continue;
+        Window w;
+        w.py = static_cast<int>((0xFFFFFFFFu - s.y) >> 16);
+        w.px = static_cast<int>((0xFFFFFFFFu - s.y) & 0xFFFFu);
+        w.y0 = max(w.py - P.ph / 2, 0);
+        w.x0 = max(w.px - P.pw / 2, 0);
+        w.y1 = min(w.py - P.ph / 2 + P.ph, P.n);
+        w.x1 = min(w.px - P.pw / 2 + P.pw, P.n);
+        w.xnew = __uint_as_float(s.z);
+        w.xdiff = __fsub_rn(__uint_as_float(s.w), w.xnew);  // pixelOld - maxPixel.PixelNew
+        // the first tile row and column of this CTA at or after the window's
+        const auto first = [](int q, uint32_t d, uint32_t inv) {
+            return q > 0 ? static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(q) + d - 1u) * inv) >> 31) : 0;
+        };
+        const int ly0 = first(w.y0 / kTY - cy, P.ay, P.inv_ay), lx0 = first(w.x0 / kTX - cx, P.ax, P.inv_ax);
+        const int ty1 = (w.y1 - 1) / kTY, tx1 = (w.x1 - 1) / kTX;
+        const int ty0 = cy + ly0 * P.ay, tx0 = cx + lx0 * P.ax;
+        best = held;
+        if (ty0 > ty1 || tx0 > tx1) continue;
+        if (in_regs && ty0 + P.ay > ty1 && tx0 + P.ax > tx1) {
+            // one tile: its pixels are offered at once, in place of the candidate held of it
+            const int yb = ty0 * kTY + warp * kCdRows;
+            if (yb + kCdRows <= w.y0 || yb >= w.y1) continue;  // none of this warp's rows
+            const int l = ly0 * P.local_x + lx0;
+            fresh = eval_rows<true>(P, thr, slope, ty0, tx0, w);
+            fresh_tile = l;
+            best = better(fresh, lane == l ? none : held);
+            continue;
+        }
+        bool rescan = false;
+        for (int ly = ly0, ty = ty0; ty <= ty1; ly++, ty += P.ay) {
+            const int yb = ty * kTY + warp * kCdRows;
+            if (yb + kCdRows <= w.y0 || yb >= w.y1) continue;
+            for (int lx = lx0, tx = tx0; tx <= tx1; lx++, tx += P.ax) {
+                const int l = ly * P.local_x + lx;
+                const CdCand v = eval_rows<true>(P, thr, slope, ty, tx, w);
+                const int o = best_lane(v);
+                if (in_regs) {
+                    const CdCand t = make_uint4(__shfl_sync(0xffffffffu, v.x, o), __shfl_sync(0xffffffffu, v.y, o),
+                                                __shfl_sync(0xffffffffu, v.z, o), __shfl_sync(0xffffffffu, v.w, o));
+                    if (lane == l) held = t;
+                } else {
+                    if (lane == o) *at(l) = v;
+                    rescan = true;
+                }
+            }
+        }
+        if (rescan) {
+            __syncwarp();
+            held = scan_held();
+        }
+        best = held;
+    }
+    settle();
+    if (in_regs)
+        if (CdCand *p = at(lane)) *p = held;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *P.ctl = c;
+        P.report[0] = c;
+    }
+    if (pair) cd_cluster_sync();  // no CTA leaves while the other may still write to it
 }
 
 // ------------------------------------------------------------------------------------------
@@ -896,15 +1092,12 @@ struct p9idg_cd {
     int n = 0, ph = 0, pw = 0;  // image size, psf2 size
     int tiles_x = 0, tiles_y = 0;
     float max_lipschitz = 0.0f;
-    Buf x, g, amap, psf2, tile_key, tile_val, params, ctl, pick, word, partial, sq0, sq1, psf_tmp;
+    Buf x, g, amap, psf2, tile_key, cand, slots, ctl, pick, word, partial, sq0, sq1, psf_tmp;
     Z2Z fft;
     CdParams hp{};
-    CdParams captured{};                   // hp as the iteration graph was captured with
-    CdCtl *h_ctl = nullptr;                // pinned
+    CdCtl *h_ctl = nullptr;                // pinned [2]
     unsigned long long *h_pick = nullptr;  // pinned: selected key
-    cudaEvent_t ev_ctl = nullptr;          // the control word of a replay has reached h_ctl
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    cudaEvent_t ev_ctl = nullptr;          // the control word of a launch has reached h_ctl
 };
 
 namespace {
@@ -946,66 +1139,60 @@ p9idg_status cd_set_maps(p9idg_cd *cd, const float *h_psf, int h, int w) {
     return P9IDG_OK;
 }
 
-p9idg_status cd_upload_params(p9idg_cd *cd) {
-    CK(cudaMemcpyAsync(cd->params.p, &cd->hp, sizeof(CdParams), cudaMemcpyHostToDevice, cd->stream));
-    return P9IDG_OK;
-}
-
-dim3 cd_window_grid(const p9idg_cd *cd) {
-    const int wy = std::min(cd->tiles_y, (cd->ph + kTY - 1) / kTY + 1);
-    const int wx = std::min(cd->tiles_x, (cd->pw + kTX - 1) / kTX + 1);
-    return dim3(static_cast<unsigned>(wx), static_cast<unsigned>(wy));
-}
-
-// The fields the iteration kernels take from their captured parameter (the rest come from the
-// device copy of the parameters on every launch).
-bool same_fixed_params(const CdParams &a, const CdParams &b) {
-    return a.a == b.a && a.psf2 == b.psf2 && a.tile_key == b.tile_key && a.tile_val == b.tile_val && a.ctl == b.ctl &&
-           a.n == b.n && a.ph == b.ph && a.pw == b.pw && a.tiles_x == b.tiles_x && a.tiles_y == b.tiles_y;
-}
-
-p9idg_status cd_capture(p9idg_cd *cd) {
-    if (cd->exec) {
-        if (same_fixed_params(cd->captured, cd->hp)) return P9IDG_OK;
-        cudaGraphExecDestroy(cd->exec);
-        cudaGraphDestroy(cd->graph);
-        cd->exec = nullptr;
-        cd->graph = nullptr;
-    }
-    // captured on the deconvolver's own stream (never the legacy stream); replayed on cd->stream
-    const dim3 grid = cd_window_grid(cd);
-    // every launch allows programmatic serialisation with the one before it (the kernel waits on
-    // it with griddepcontrol.wait before reading its results)
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+// Launch of the run kernel: nctas CTAs, in pairs from kCdPairFrom on.
+struct CdLaunch {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kCdNT);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = cd->own;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CK(cudaStreamBeginCapture(cd->own, cudaStreamCaptureModeThreadLocal));
-    cudaError_t le = cudaSuccess;
-    for (int k = 0; k < kGraphIters && le == cudaSuccess; k++)
-        le = cudaLaunchKernelEx(&cfg, cd_iter_kernel, cd->hp, static_cast<const CdParams *>(cd->params.as<CdParams>()),
-                                k & 1, k + 1 == kGraphIters ? cd->h_ctl : static_cast<CdCtl *>(nullptr));
-    cudaGraph_t gph = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(cd->own, &gph);
-    if (le != cudaSuccess || ce != cudaSuccess) {
-        if (gph) cudaGraphDestroy(gph);
-        return cuda_fail(le != cudaSuccess ? le : ce, "capturing the coordinate-descent graph");
+    cudaLaunchAttribute attr[2];
+    explicit CdLaunch(int nctas, cudaStream_t stream) {
+        const unsigned c = nctas >= kCdPairFrom ? 2 : 1;
+        cfg.gridDim = dim3((static_cast<unsigned>(nctas) + c - 1) / c * c);
+        cfg.blockDim = dim3(kCdNT);
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeCooperative;
+        attr[1].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
     }
-    cd->graph = gph;
-    CK(cudaGraphInstantiate(&cd->exec, cd->graph, 0));
-    cd->captured = cd->hp;
+};
+
+// Deals the tiles out to the CTAs of the run kernel: the ay x ax torus that leaves the fewest tiles of a
+// whole window to one CTA and then the fewest tiles in all (more CTAs).
+p9idg_status cd_layout(p9idg_cd *cd) {
+    CdParams &p = cd->hp;
+    int coop = 0, pairs = 0;
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, cd->device));
+    CdLaunch two(kCdPairFrom, cd->stream);
+    two.cfg.numAttrs = 1;
+    CK(cudaOccupancyMaxActiveClusters(&pairs, cd_run_kernel, &two.cfg));
+    const int most = 2 * std::min(pairs, kCdSlots);
+    if (!coop || most < 2) return fail(P9IDG_UNSUPPORTED, "the device cannot run the coordinate-descent kernel");
+    const auto div = [](int a, int b) { return (a + b - 1) / b; };
+    const int wy = std::min(cd->tiles_y, div(cd->ph, kTY) + 1), wx = std::min(cd->tiles_x, div(cd->pw, kTX) + 1);
+    int64_t best = INT64_MAX;
+    for (int ax = 1; ax <= std::min(cd->tiles_x, most); ax++)
+        for (int ay = 1; ay <= std::min(cd->tiles_y, most / ax); ay++) {
+            const int64_t window = static_cast<int64_t>(div(wy, ay)) * div(wx, ax),
+                          all = static_cast<int64_t>(div(cd->tiles_y, ay)) * div(cd->tiles_x, ax);
+            const int64_t cost = (window << 32) + all;
+            if (cost < best) {
+                best = cost;
+                p.ax = ax;
+                p.ay = ay;
+            }
+        }
+    p.inv_ax = static_cast<uint32_t>(((1ull << 31) + p.ax - 1) / p.ax);
+    p.inv_ay = static_cast<uint32_t>(((1ull << 31) + p.ay - 1) / p.ay);
+    p.local_x = div(cd->tiles_x, p.ax);
+    p.local_tiles = div(cd->tiles_y, p.ay) * p.local_x;
     return P9IDG_OK;
 }
 
-// Candidates of every tile with (lambda, alpha) into state buffer 0, control reset.
-p9idg_status cd_scan(p9idg_cd *cd, float lambda, float alpha) {
-    cd_scan_kernel<<<dim3(cd->tiles_x, cd->tiles_y), kCdNT, 0, cd->stream>>>(cd->params.as<CdParams>(), lambda, alpha);
+// Candidates of every tile with the parameters' lambda and alpha, control reset.
+p9idg_status cd_scan(p9idg_cd *cd) {
+    cd_scan_kernel<<<dim3(cd->tiles_x, cd->tiles_y), kCdNT, 0, cd->stream>>>(cd->hp);
     CK(cudaGetLastError());
     return P9IDG_OK;
 }
@@ -1020,29 +1207,31 @@ p9idg_status cd_run(p9idg_cd *cd, float *d_x, float *d_g, float lambda, float al
     cd->hp.alpha = alpha;
     cd->hp.eps = eps;
     cd->hp.max_iter = max_iter;
-    TRY(cd_upload_params(cd));
-    TRY(cd_scan(cd, lambda, alpha));
-    TRY(cd_capture(cd));
-    // One replay stays in flight while the host looks at the state the previous one left, so the GPU
-    // never waits on the host; a replay launched after the stopping one does nothing (every launch sees
-    // the done flag).  max_iter + 1 launches are enough: the one past the last iteration stops.
-    const int64_t max_replays = (static_cast<int64_t>(std::max(max_iter, 0)) + kGraphIters) / kGraphIters;
-    *cd->h_ctl = CdCtl{};
-    CK(cudaGraphLaunch(cd->exec, cd->stream));
-    for (int64_t r = 0; r < max_replays; r++) {
+    TRY(cd_scan(cd));
+    cd->h_ctl[0] = cd->h_ctl[1] = CdCtl{};
+    if (max_iter <= 0) {
+        CK(cudaStreamSynchronize(cd->stream));
+        cd->h_ctl[0].done = 1;
+    }
+    // One launch stays in flight while the host looks at the state the previous one left, so the GPU never
+    // waits on the host; a launch after the stopping one does nothing (it sees the done flag).
+    const int64_t launches = (static_cast<int64_t>(std::max(max_iter, 0)) + kCdLaunchIters - 1) / kCdLaunchIters;
+    CdLaunch run(cd->hp.ax * cd->hp.ay, cd->stream);
+    if (launches > 0) CK(cudaLaunchKernelEx(&run.cfg, cd_run_kernel, cd->hp));
+    for (int64_t r = 0; r < launches; r++) {
         CK(cudaEventRecord(cd->ev_ctl, cd->stream));
-        if (r + 1 < max_replays) CK(cudaGraphLaunch(cd->exec, cd->stream));
+        if (r + 1 < launches) CK(cudaLaunchKernelEx(&run.cfg, cd_run_kernel, cd->hp));
         CK(cudaEventSynchronize(cd->ev_ctl));
         if (static_cast<volatile CdCtl *>(cd->h_ctl)->done) break;
     }
-    CK(cudaStreamSynchronize(cd->stream));  // the replay in flight, if any
-    if (!cd->h_ctl->done) return fail(P9IDG_DEVICE_CHECK_FAILED, "coordinate descent did not stop");
-    if (cd->h_ctl->error)
+    CK(cudaStreamSynchronize(cd->stream));  // the launch in flight, if any
+    if (!cd->h_ctl[0].done || cd->h_ctl[1].error) return fail(P9IDG_DEVICE_CHECK_FAILED, "coordinate descent did not stop");
+    if (cd->h_ctl[0].error)
         return fail(P9IDG_INVALID_ARGUMENT,
                     "no pixel changes and epsilon <= 0: the reference would index pixel (-1, -1)");
     if (res) {
-        res->converged = cd->h_ctl->converged;
-        res->iterations = cd->h_ctl->iter;
+        res->converged = cd->h_ctl[0].converged;
+        res->iterations = cd->h_ctl[0].iter;
         res->elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
     return P9IDG_OK;
@@ -1051,10 +1240,10 @@ p9idg_status cd_run(p9idg_cd *cd, float *d_x, float *d_g, float lambda, float al
 p9idg_status cd_abs_max(p9idg_cd *cd, const float *d_x, const float *d_g, float lambda, float alpha, float *out) {
     cd->hp.x = const_cast<float *>(d_x);
     cd->hp.g = const_cast<float *>(d_g);
-    TRY(cd_upload_params(cd));
-    TRY(cd_scan(cd, lambda, alpha));
-    cd_pick_kernel<<<1, kCdNT, 0, cd->stream>>>(cd->params.as<CdParams>(), cd->pick.as<unsigned long long>(),
-                                             reinterpret_cast<float2 *>(cd->pick.as<unsigned long long>() + 1));
+    cd->hp.lambda = lambda;
+    cd->hp.alpha = alpha;
+    TRY(cd_scan(cd));
+    cd_pick_kernel<<<1, kCdNT, 0, cd->stream>>>(cd->hp.tile_key, cd->tiles_x * cd->tiles_y, cd->pick.as<unsigned long long>());
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(cd->h_pick, cd->pick.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, cd->stream));
     CK(cudaStreamSynchronize(cd->stream));
@@ -1066,9 +1255,7 @@ p9idg_status cd_abs_max(p9idg_cd *cd, const float *d_x, const float *d_g, float 
 void cd_release(p9idg_cd *cd) {
     if (cd->stream) cudaStreamSynchronize(cd->stream);
     if (cd->ev_ctl) cudaEventDestroy(cd->ev_ctl);
-    if (cd->exec) cudaGraphExecDestroy(cd->exec);
-    if (cd->graph) cudaGraphDestroy(cd->graph);
-    Buf *bufs[] = {&cd->x, &cd->g, &cd->amap, &cd->psf2, &cd->tile_key, &cd->tile_val, &cd->params, &cd->ctl,
+    Buf *bufs[] = {&cd->x, &cd->g, &cd->amap, &cd->psf2, &cd->tile_key, &cd->cand, &cd->slots, &cd->ctl,
                    &cd->pick, &cd->word, &cd->partial, &cd->sq0, &cd->sq1, &cd->psf_tmp};
     for (Buf *b : bufs) b->release();
     cd->fft.release();
@@ -1081,7 +1268,7 @@ p9idg_status cd_init(p9idg_cd *cd, int n, const float *psf, int h, int w) {
     CK(cudaGetDevice(&cd->device));
     CK(cudaStreamCreateWithFlags(&cd->own, cudaStreamNonBlocking));
     cd->stream = cd->own;
-    CK(cudaMallocHost(reinterpret_cast<void **>(&cd->h_ctl), sizeof(CdCtl)));
+    CK(cudaMallocHost(reinterpret_cast<void **>(&cd->h_ctl), 2 * sizeof(CdCtl)));
     CK(cudaMallocHost(reinterpret_cast<void **>(&cd->h_pick), sizeof(unsigned long long)));
     CK(cudaEventCreateWithFlags(&cd->ev_ctl, cudaEventDisableTiming));
     cd->n = n;
@@ -1089,25 +1276,27 @@ p9idg_status cd_init(p9idg_cd *cd, int n, const float *psf, int h, int w) {
     cd->tiles_y = (n + kTY - 1) / kTY;
     const size_t nn = static_cast<size_t>(n) * n, nt = static_cast<size_t>(cd->tiles_x) * cd->tiles_y;
     CK(cd->amap.ensure(sizeof(float) * nn));
-    CK(cd->tile_key.ensure(sizeof(unsigned long long) * 2 * nt));
-    CK(cd->tile_val.ensure(sizeof(float2) * 2 * nt));
-    CK(cd->params.ensure(sizeof(CdParams)));
-    CK(cd->ctl.ensure(sizeof(CdCtl) * 2));
-    CK(cd->pick.ensure(sizeof(unsigned long long) + sizeof(float2)));
+    CK(cd->tile_key.ensure(sizeof(unsigned long long) * nt));
+    CK(cd->cand.ensure(sizeof(CdCand) * kCdWarps * nt));
+    CK(cd->slots.ensure(sizeof(uint4) * 2 * kCdSlots));
+    CK(cd->ctl.ensure(sizeof(CdCtl)));
+    CK(cd->pick.ensure(sizeof(unsigned long long)));
     CK(cd->word.ensure(sizeof(unsigned int)));
     TRY(cd_set_maps(cd, psf, h, w));
     cd->hp = CdParams{};
     cd->hp.a = cd->amap.as<float>();
     cd->hp.psf2 = cd->psf2.as<float>();
+    cd->hp.cand = cd->cand.as<CdCand>();
     cd->hp.tile_key = cd->tile_key.as<unsigned long long>();
-    cd->hp.tile_val = cd->tile_val.as<float2>();
+    cd->hp.slots = cd->slots.as<uint4>();
     cd->hp.ctl = cd->ctl.as<CdCtl>();
+    cd->hp.report = cd->h_ctl;
     cd->hp.n = n;
     cd->hp.ph = cd->ph;
     cd->hp.pw = cd->pw;
     cd->hp.tiles_x = cd->tiles_x;
     cd->hp.tiles_y = cd->tiles_y;
-    return P9IDG_OK;
+    return cd_layout(cd);
 }
 
 p9idg_status check_cd_args(int32_t n, const float *psf, int32_t h, int32_t w) {
