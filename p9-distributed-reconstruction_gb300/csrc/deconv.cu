@@ -20,6 +20,7 @@
 
 #include <cuda_runtime.h>
 #include <cufft.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <chrono>
@@ -119,10 +120,10 @@ __device__ __forceinline__ float prox(float x, float lipschitz, float thr, float
 }
 
 constexpr int kNT = 512, kWarps = kNT / 32;  // image reductions
-// Coordinate descent: tiles of kTY x kTX pixels, CTAs of kCdNT threads, each warp two rows of a tile.
-// A 768^2 update window (a 384^2 PSF) spans 21 x 7 = 147 such tiles, one for each CTA of the 152 SMs.
-constexpr int kTY = 40, kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32;
-constexpr int kCdRows = kTY / kCdWarps, kCdCols = kTX / 32;  // pixels a thread: rows x columns
+// Coordinate descent: CTAs of kCdNT threads, tiles of kTX columns in which each warp has R = 1 or 2 rows.  A
+// 768^2 update window (a 384^2 PSF) spans 21 x 7 = 147 tiles of two rows a warp, one for each CTA of the 152
+// SMs.  Windows of few tiles take one row (cd_layout).
+constexpr int kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32, kCdCols = kTX / 32;
 // Slots of the exchange, three for each lane of the polling warp; pairs of CTAs share one from
 // kCdPairFrom CTAs on.  Measured for the exchange alone: 1270 clocks with 30 CTAs, each polling every
 // slot, 3500 with 147 (the polls of one line queue up), 2490 with 74 pairs; pairs of 30 take 2040.
@@ -130,6 +131,9 @@ constexpr int kCdPoll = 3, kCdSlots = 32 * kCdPoll, kCdPairFrom = 56;
 // Iterations of one launch: few enough that other streams' kernels wait milliseconds for the SMs, not
 // for a whole deconvolution, and enough that a launch does not show.
 constexpr int kCdLaunchIters = 512;
+// q / d = q * ceil(2^36 / d) >> 36 for q * d < 2^36; here q < 2^17, d < 2^15 and d >= 20, so the factor
+// fits 32 bits.
+constexpr int kCdInvBits = 36;
 // Clocks (about 4 s) after which a CTA gives up waiting for another.  All CTAs of a cooperative launch are
 // resident, so this is only met if one of them cannot run.
 constexpr long long kCdPatience = 8000000000ll;
@@ -152,8 +156,9 @@ struct CdParams {
     CdCtl *ctl;
     CdCtl *report;  // pinned: [0] the state a launch leaves, [1].error set by a CTA that gave up
     int32_t n, ph, pw, tiles_x, tiles_y, max_iter;
-    int32_t ax, ay;              // tile (ty, tx) belongs to CTA (ty % ay) * ax + tx % ax
-    uint32_t inv_ax, inv_ay;     // ceil(2^31 / ax): q / ax = q * inv_ax >> 31 for q below 2^11
+    int32_t rows;                  // R
+    int32_t ax, ay;                // tile (ty, tx) belongs to CTA (ty % ay) * ax + tx % ax
+    uint32_t inv_row, inv_col;     // ceil(2^kCdInvBits / tile rows of a period), .. / tile columns
     int32_t local_x, local_tiles;  // tiles of one CTA: in a row, in all (at most)
     float lambda, alpha, eps;
 };
@@ -216,12 +221,14 @@ __device__ __forceinline__ void cd_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+// CTA scope: what st.async delivers is in shared memory when its bytes are counted.  Acquiring at cluster
+// scope empties L1 each time, and the tiles' pixels then come from L2 in every iteration.
 __device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase) {
     long long t0 = 0;
     while (true) {
         uint32_t done;
         asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
             : "r"(bar), "r"(phase)
             : "memory");
@@ -237,78 +244,144 @@ __device__ __forceinline__ void cd_cluster_sync() {
 }
 
 struct Window {
-    int py, px, y0, y1, x0, x1;
+    int py, px;          // selected pixel
+    int yq, xq;          // of the update window's first pixel, which may lie outside the image
+    int y0, y1, x0, x1;  // its part inside
     float xnew, xdiff;
 };
 
-// Evaluates (and with UPDATE first updates) this warp's rows of one tile; returns this thread's best
-// candidate.  All of a thread's loads are issued before any is used (predicated, no early exits), so
-// the rows cost one memory latency rather than one per pixel.
-template <bool UPDATE>
-__device__ __forceinline__ CdCand eval_rows(const CdParams &P, float thr, float slope, int ty, int tx, const Window &w) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int yb = ty * kTY + warp * kCdRows, xb = tx * kTX + lane;
-    bool in[kCdRows][kCdCols], upd[kCdRows][kCdCols];
-    float gv[kCdRows][kCdCols], xv[kCdRows][kCdCols], av[kCdRows][kCdCols], pv[kCdRows][kCdCols];
-    float *gp[kCdRows];
+// Two additions an instruction, rounded as __fadd_rn.  Products stay scalar: a packed mul.rn and the packed
+// add.rn after it came out fused.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float rcp_approx(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+// Evaluates (and with UPDATE first updates) the warp's R rows from yb of the tile at column xb; returns
+// this thread's best candidate, which is the exact one wherever it is the warp's best.  COVER: what is known
+// of the rows' pixels: nothing, that all lie in the image, or that all lie in the update window.  All of a
+// thread's loads are issued before any is used, so the rows cost one memory latency rather than one per pixel.
+//
+// The kernel around this waits for what its warps issue here (five warps a scheduler), and most of it would
+// be divisions for pixels that cannot win.  So the changes are first approximated with a reciprocal good to an
+// ulp: for den in (1e-30, 1e30), quotient and change are off by at most Q 2^-22 + D 2^-23 (Q bounds the warp's
+// quotients, D is its largest change), so the pixel with the largest change is among those within twice that
+// of D, and only these (usually one in the warp) are evaluated as the reference does; rows whose pixels are
+// all zero and held there by the threshold are left at once.  NaN and infinities fail the comparisons that
+// leave a pixel out.
+enum Cover { kAny, kImage, kWindow };
+
+template <int R, bool UPDATE, Cover COVER>
+__device__ __forceinline__ CdCand eval_rows(const CdParams &P, float thr, float slope, int yb, int xb, const Window &w) {
+    const int x = xb + static_cast<int>(threadIdx.x & 31);
+    constexpr int J = R * kCdCols;
+    float gv[J], xv[J], av[J], pv[J], d[J];
+    bool in[J], upd[J];
+    const size_t i0 = static_cast<size_t>(yb) * P.n + x;
+    float *gp = P.g + i0, *xp = P.x + i0;
+    const float *ap = P.a + i0;
+    const float *pp = P.psf2 + (static_cast<int64_t>(yb - w.yq) * P.pw + (x - w.xq));
+    const auto off = [&](int j) { return (j / kCdCols) * P.n + 32 * (j % kCdCols); };
 #pragma unroll
-    for (int r = 0; r < kCdRows; r++) {
-        const int y = yb + r;
-        const size_t i0 = static_cast<size_t>(y) * P.n + xb;
-        gp[r] = P.g + i0;
-        const float *xp = P.x + i0, *ap = P.a + i0;
-        const float *pp = P.psf2 + (static_cast<int64_t>(y + P.ph / 2 - w.py) * P.pw + (xb + P.pw / 2 - w.px));
-#pragma unroll
-        for (int k = 0; k < kCdCols; k++) {
-            const int xc = xb + 32 * k;
-            in[r][k] = y < P.n && xc < P.n;
-            upd[r][k] = UPDATE && y >= w.y0 && y < w.y1 && xc >= w.x0 && xc < w.x1;
-            gv[r][k] = in[r][k] ? gp[r][32 * k] : 0.0f;
-            xv[r][k] = in[r][k] ? xp[32 * k] : 0.0f;
-            av[r][k] = in[r][k] ? __ldg(ap + 32 * k) : 1.0f;
-            pv[r][k] = upd[r][k] ? __ldg(pp + 32 * k) : 0.0f;
-        }
-        if (UPDATE && y == w.py) {  // the selected pixel takes its new value
-#pragma unroll
-            for (int k = 0; k < kCdCols; k++)
-                if (xb + 32 * k == w.px) {
-                    xv[r][k] = w.xnew;
-                    P.x[i0 + 32 * k] = w.xnew;
-                }
-        }
+    for (int j = 0; j < J; j++) {
+        const int r = j / kCdCols, k = j % kCdCols, y = yb + r, xc = x + 32 * k;
+        in[j] = COVER != kAny || (y < P.n && xc < P.n);
+        upd[j] = UPDATE && (COVER == kWindow || (y >= w.y0 && y < w.y1 && xc >= w.x0 && xc < w.x1));
+        gv[j] = in[j] ? gp[off(j)] : 0.0f;
+        xv[j] = in[j] ? xp[off(j)] : 0.0f;
+        av[j] = in[j] ? __ldg(ap + off(j)) : 1.0f;
+        pv[j] = upd[j] ? __ldg(pp + (r * P.pw + 32 * k)) : 0.0f;
     }
-    float bd = 0.0f, bnew = 0.0f, bold = 0.0f;
-    uint32_t bi = 0xFFFFFFFFu;
+    if (UPDATE && w.py - yb < R && w.py >= yb) {  // the selected pixel takes its new value
 #pragma unroll
-    for (int r = 0; r < kCdRows; r++) {
-#pragma unroll
-        for (int k = 0; k < kCdCols; k++) {
-            float g = gv[r][k];
-            if (UPDATE && upd[r][k]) {
-                g = __fadd_rn(g, __fmul_rn(pv[r][k], w.xdiff));  // gradients[i, j] += psf2 * xDiff
-                gp[r][32 * k] = g;
+        for (int j = 0; j < J; j++)
+            if (w.py == yb + j / kCdCols && w.px == x + 32 * (j % kCdCols)) {
+                xv[j] = w.xnew;
+                xp[off(j)] = w.xnew;
             }
-            const float a = av[r][k], old = xv[r][k];
-            const float xt = prox(__fadd_rn(__fmul_rn(old, a), g), a, thr, slope);
-            const float d = fabsf(__fsub_rn(old, xt));
-            if (in[r][k] && d > bd) {  // pixels in index order: the first of equal changes stays
-                bd = d;
-                bnew = xt;
-                bold = old;
-                bi = (static_cast<uint32_t>(yb + r) << 16) | static_cast<uint32_t>(xb + 32 * k);
-            }
-        }
     }
-    return make_uint4(__float_as_uint(bd), 0xFFFFFFFFu - bi, __float_as_uint(bnew), __float_as_uint(bold));
+    const F2 thr2 = f2(-thr, -thr), slope2 = f2(slope, slope);
+    float dmax = 0.0f, vmax = 0.0f, den_lo = 1e30f, den_hi = 0.0f;
+#pragma unroll
+    for (int j = 0; j < J; j += 2) {
+        if (UPDATE) {  // gradients[i, j] += psf2 * xDiff
+            const float2 g = f2_get(
+                f2_add(f2(gv[j], gv[j + 1]), f2(__fmul_rn(pv[j], w.xdiff), __fmul_rn(pv[j + 1], w.xdiff))));
+            if (upd[j]) gp[off(j)] = gv[j] = g.x;
+            if (upd[j + 1]) gp[off(j + 1)] = gv[j + 1] = g.y;
+        }
+        const F2 xa = f2(__fmul_rn(xv[j], av[j]), __fmul_rn(xv[j + 1], av[j + 1]));
+        const float2 v = f2_get(f2_add(f2_add(xa, f2(gv[j], gv[j + 1])), thr2));
+        const float2 den = f2_get(f2_add(f2(av[j], av[j + 1]), slope2));
+        const float va = max_nan(v.x, 0.0f), vb = max_nan(v.y, 0.0f);
+        d[j] = fabsf(__fsub_rn(xv[j], __fmul_rn(va, rcp_approx(den.x))));
+        d[j + 1] = fabsf(__fsub_rn(xv[j + 1], __fmul_rn(vb, rcp_approx(den.y))));
+        if (COVER == kAny) {
+            d[j] = in[j] ? d[j] : 0.0f;
+            d[j + 1] = in[j + 1] ? d[j + 1] : 0.0f;
+        }
+        dmax = fmaxf(dmax, fmaxf(d[j], d[j + 1]));
+        vmax = max_nan(vmax, max_nan(va, vb));
+        den_lo = fminf(den_lo, fminf(den.x, den.y));
+        den_hi = fmaxf(den_hi, fmaxf(den.x, den.y));
+    }
+    const float q = den_lo > 1e-30f && den_hi < 1e30f ? __fmul_rn(vmax, 1.0001f * rcp_approx(den_lo)) : CUDART_NAN_F;
+    const float D = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dmax)));
+    const float Q = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(q)));  // a NaN is the largest
+    CdCand best = make_uint4(0u, 0u, 0u, 0u);
+    if (D == 0.0f && __all_sync(0xffffffffu, vmax == 0.0f)) return best;
+    const float least = D - (D + Q) * 0x1p-20f - 1e-37f;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        if (d[j] < least || !in[j]) continue;
+        const float xt = prox(__fadd_rn(__fmul_rn(xv[j], av[j]), gv[j]), av[j], thr, slope);
+        const float e = fabsf(__fsub_rn(xv[j], xt));
+        if (e > __uint_as_float(best.x))  // pixels in index order: the first of equal changes stays
+            best = make_uint4(__float_as_uint(e),
+                              0xFFFFFFFFu - ((static_cast<uint32_t>(yb + j / kCdCols) << 16) | static_cast<uint32_t>(x + 32 * (j % kCdCols))),
+                              __float_as_uint(xt), __float_as_uint(xv[j]));
+    }
+    return best;
+}
+
+// The same for an update, by what the window and the image cover.
+template <int R>
+__device__ __forceinline__ CdCand update_rows(const CdParams &P, float thr, float slope, int yb, int xb, const Window &w) {
+    if (yb >= w.y0 && yb + R <= w.y1 && xb >= w.x0 && xb + kTX <= w.x1) return eval_rows<R, true, kWindow>(P, thr, slope, yb, xb, w);
+    if (yb + R <= P.n && xb + kTX <= P.n) return eval_rows<R, true, kImage>(P, thr, slope, yb, xb, w);
+    return eval_rows<R, true, kAny>(P, thr, slope, yb, xb, w);
 }
 
 // Full scan (GetAbsMax over the whole image): every warp's candidate of every tile, and each tile's best key.
+template <int R>
 __global__ void __launch_bounds__(kCdNT) cd_scan_kernel(const __grid_constant__ CdParams P) {
     __shared__ uint2 sm[kCdWarps];
     const float thr = __fmul_rn(P.lambda, P.alpha), slope = __fmul_rn(P.lambda, __fsub_rn(1.0f, P.alpha));
     const Window w{};
-    const CdCand c = eval_rows<false>(P, thr, slope, blockIdx.y, blockIdx.x, w);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.y * P.tiles_x + blockIdx.x;
+    const CdCand c = eval_rows<R, false, kAny>(P, thr, slope, (blockIdx.y * kCdWarps + warp) * R, blockIdx.x * kTX, w);
     if (lane == best_lane(c)) {
         P.cand[t * static_cast<int64_t>(kCdWarps) + warp] = c;
         sm[warp] = make_uint2(c.x, c.y);
@@ -364,8 +437,14 @@ __global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const unsigned long long
 // slots alternate between two sets: a slot is overwritten only after every cluster has posted the
 // iteration after it, hence read it.
 //
+// Measured for 1000 iterations at 3072^2 with a 768^2 window: 4.5 us an iteration, against 6.5 us for a
+// launch per iteration (graph replays with programmatic dependent launches, every CTA reducing all tile
+// keys).  Of the 4.5 us about 1.3 are the exchange and its two hops within a pair, 1.5 a warp's loads and
+// evaluation, and the rest the wait for the slowest of 147 CTAs.
+//
 // A lane keeps in registers the candidate of its warp's rows of local tile `lane`; images of more than 32
-// tiles a CTA (4864 tiles, about 5000^2) keep them in P.cand, which only this warp touches.
+// tiles a CTA (4864 tiles, 5000^2 with two rows a warp) keep them in P.cand, which only this warp touches.
+template <int R>
 __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant__ CdParams P) {
     __shared__ CdCand sm_in[2][2 * kCdWarps];  // candidates of the cluster's warps (first CTA)
     __shared__ CdCand sm_sel[2];               // the selected candidate
@@ -417,6 +496,7 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
             if (const CdCand *p = at(l)) h = better(*p, h);
         return h;
     };
+    const int row0 = (cy * kCdWarps + warp) * R, row_step = P.ay * kCdWarps * R, col0 = cx * kTX, col_step = P.ax * kTX;
     CdCand held = scan_held();  // best of the local tiles l = lane mod 32
     CdCand best = held;         // what this thread has to offer
     CdCand fresh = none;        // its candidate of local tile fresh_tile, not yet in held
@@ -512,50 +592,41 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
         Window w;
         w.py = static_cast<int>((0xFFFFFFFFu - s.y) >> 16);
         w.px = static_cast<int>((0xFFFFFFFFu - s.y) & 0xFFFFu);
-        w.y0 = max(w.py - P.ph / 2, 0);
-        w.x0 = max(w.px - P.pw / 2, 0);
-        w.y1 = min(w.py - P.ph / 2 + P.ph, P.n);
-        w.x1 = min(w.px - P.pw / 2 + P.pw, P.n);
+        w.yq = w.py - P.ph / 2;
+        w.xq = w.px - P.pw / 2;
+        w.y0 = max(w.yq, 0);
+        w.x0 = max(w.xq, 0);
+        w.y1 = min(w.yq + P.ph, P.n);
+        w.x1 = min(w.xq + P.pw, P.n);
         w.xnew = __uint_as_float(s.z);
         w.xdiff = __fsub_rn(__uint_as_float(s.w), w.xnew);  // pixelOld - maxPixel.PixelNew
-        // the first tile row and column of this CTA at or after the window's
-        const auto first = [](int q, uint32_t d, uint32_t inv) {
-            return q > 0 ? static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(q) + d - 1u) * inv) >> 31) : 0;
+        // this warp's first rows and this CTA's first tile column that reach into the window
+        const auto first = [](int q, int d, uint32_t inv) {
+            return static_cast<int>(__umulhi(static_cast<uint32_t>(max(q, 0) + d - 1), inv) >> (kCdInvBits - 32));
         };
-        const int ly0 = first(w.y0 / kTY - cy, P.ay, P.inv_ay), lx0 = first(w.x0 / kTX - cx, P.ax, P.inv_ax);
-        const int ty1 = (w.y1 - 1) / kTY, tx1 = (w.x1 - 1) / kTX;
-        const int ty0 = cy + ly0 * P.ay, tx0 = cx + lx0 * P.ax;
+        const int ly0 = first(w.y0 - (R - 1) - row0, row_step, P.inv_row), yb0 = row0 + ly0 * row_step;
+        const int lx0 = first(w.x0 - (kTX - 1) - col0, col_step, P.inv_col), xb0 = col0 + lx0 * col_step;
         best = held;
-        if (ty0 > ty1 || tx0 > tx1) continue;
-        if (in_regs && ty0 + P.ay > ty1 && tx0 + P.ax > tx1) {
+        if (yb0 >= w.y1 || xb0 >= w.x1) continue;
+        if (in_regs && yb0 + row_step >= w.y1 && xb0 + col_step >= w.x1) {
             // one tile: its pixels are offered at once, in place of the candidate held of it
-            const int yb = ty0 * kTY + warp * kCdRows;
-            if (yb + kCdRows <= w.y0 || yb >= w.y1) continue;  // none of this warp's rows
-            const int l = ly0 * P.local_x + lx0;
-            fresh = eval_rows<true>(P, thr, slope, ty0, tx0, w);
-            fresh_tile = l;
-            best = better(fresh, lane == l ? none : held);
+            fresh_tile = ly0 * P.local_x + lx0;
+            fresh = update_rows<R>(P, thr, slope, yb0, xb0, w);
+            best = better(fresh, lane == fresh_tile ? none : held);
             continue;
         }
-        bool rescan = false;
-        for (int ly = ly0, ty = ty0; ty <= ty1; ly++, ty += P.ay) {
-            const int yb = ty * kTY + warp * kCdRows;
-            if (yb + kCdRows <= w.y0 || yb >= w.y1) continue;
-            for (int lx = lx0, tx = tx0; tx <= tx1; lx++, tx += P.ax) {
-                const int l = ly * P.local_x + lx;
-                const CdCand v = eval_rows<true>(P, thr, slope, ty, tx, w);
-                const int o = best_lane(v);
+        for (int ly = ly0, yb = yb0; yb < w.y1; ly++, yb += row_step)
+            for (int lx = lx0, xb = xb0; xb < w.x1; lx++, xb += col_step) {
+                fresh_tile = ly * P.local_x + lx;
+                fresh = update_rows<R>(P, thr, slope, yb, xb, w);
                 if (in_regs) {
-                    const CdCand t = make_uint4(__shfl_sync(0xffffffffu, v.x, o), __shfl_sync(0xffffffffu, v.y, o),
-                                                __shfl_sync(0xffffffffu, v.z, o), __shfl_sync(0xffffffffu, v.w, o));
-                    if (lane == l) held = t;
+                    settle();
                 } else {
-                    if (lane == o) *at(l) = v;
-                    rescan = true;
+                    if (lane == best_lane(fresh)) *at(fresh_tile) = fresh;
+                    fresh_tile = -1;
                 }
             }
-        }
-        if (rescan) {
+        if (!in_regs) {
             __syncwarp();
             held = scan_held();
         }
@@ -1143,7 +1214,7 @@ p9idg_status cd_set_maps(p9idg_cd *cd, const float *h_psf, int h, int w) {
 struct CdLaunch {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    explicit CdLaunch(int nctas, cudaStream_t stream) {
+    CdLaunch(int nctas, cudaStream_t stream) {
         const unsigned c = nctas >= kCdPairFrom ? 2 : 1;
         cfg.gridDim = dim3((static_cast<unsigned>(nctas) + c - 1) / c * c);
         cfg.blockDim = dim3(kCdNT);
@@ -1159,40 +1230,63 @@ struct CdLaunch {
 };
 
 // Deals the tiles out to the CTAs of the run kernel: the ay x ax torus that leaves the fewest tiles of a
-// whole window to one CTA and then the fewest tiles in all (more CTAs).
+// whole window to one CTA.  Of several, the one of the fewest CTAs that keep their candidates in registers
+// (at most 32 tiles each), since the exchange grows with them (1024^2 with a 256^2 window: 24 CTAs 2.97 ms a
+// 1000 iterations, 104 CTAs 3.20 ms); if none does, the one of the fewest tiles a CTA.
 p9idg_status cd_layout(p9idg_cd *cd) {
     CdParams &p = cd->hp;
     int coop = 0, pairs = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, cd->device));
     CdLaunch two(kCdPairFrom, cd->stream);
     two.cfg.numAttrs = 1;
-    CK(cudaOccupancyMaxActiveClusters(&pairs, cd_run_kernel, &two.cfg));
+    CK(cudaOccupancyMaxActiveClusters(&pairs, cd_run_kernel<2>, &two.cfg));
     const int most = 2 * std::min(pairs, kCdSlots);
     if (!coop || most < 2) return fail(P9IDG_UNSUPPORTED, "the device cannot run the coordinate-descent kernel");
     const auto div = [](int a, int b) { return (a + b - 1) / b; };
-    const int wy = std::min(cd->tiles_y, div(cd->ph, kTY) + 1), wx = std::min(cd->tiles_x, div(cd->pw, kTX) + 1);
+    // One row a warp halves the evaluation, which is about half of an iteration, and doubles the CTAs that
+    // exchange candidates.  1000 iterations at 376^2 with an 80^2 window: 2.30 ms with one row (10 tiles),
+    // 2.85 with two; at 1024^2 with a 256^2 window: 3.29 ms with one row (42 tiles), 2.97 with two.
+    p.rows = 1;
+    const auto window_rows = [&]() { return std::min(div(cd->n, kCdWarps * p.rows), div(cd->ph, kCdWarps * p.rows) + 1); };
+    cd->tiles_x = div(cd->n, kTX);
+    const int wx = std::min(cd->tiles_x, div(cd->pw, kTX) + 1);
+    if (window_rows() * wx > std::min(32, most)) p.rows = 2;
+    cd->tiles_y = div(cd->n, kCdWarps * p.rows);
+    const int wy = window_rows();
     int64_t best = INT64_MAX;
     for (int ax = 1; ax <= std::min(cd->tiles_x, most); ax++)
         for (int ay = 1; ay <= std::min(cd->tiles_y, most / ax); ay++) {
             const int64_t window = static_cast<int64_t>(div(wy, ay)) * div(wx, ax),
                           all = static_cast<int64_t>(div(cd->tiles_y, ay)) * div(cd->tiles_x, ax);
-            const int64_t cost = (window << 32) + all;
+            const int64_t cost = (window << 32) + (all > 32 ? all << 8 : ax * ay);
             if (cost < best) {
                 best = cost;
                 p.ax = ax;
                 p.ay = ay;
             }
         }
-    p.inv_ax = static_cast<uint32_t>(((1ull << 31) + p.ax - 1) / p.ax);
-    p.inv_ay = static_cast<uint32_t>(((1ull << 31) + p.ay - 1) / p.ay);
+    p.tiles_x = cd->tiles_x;
+    p.tiles_y = cd->tiles_y;
+    const uint32_t row_step = static_cast<uint32_t>(p.ay * kCdWarps * p.rows), col_step = static_cast<uint32_t>(p.ax * kTX);
+    p.inv_row = static_cast<uint32_t>(((1ull << kCdInvBits) + row_step - 1) / row_step);
+    p.inv_col = static_cast<uint32_t>(((1ull << kCdInvBits) + col_step - 1) / col_step);
     p.local_x = div(cd->tiles_x, p.ax);
     p.local_tiles = div(cd->tiles_y, p.ay) * p.local_x;
+    const size_t nt = static_cast<size_t>(cd->tiles_x) * cd->tiles_y;
+    CK(cd->tile_key.ensure(sizeof(unsigned long long) * nt));
+    CK(cd->cand.ensure(sizeof(CdCand) * kCdWarps * nt));
+    p.cand = cd->cand.as<CdCand>();
+    p.tile_key = cd->tile_key.as<unsigned long long>();
     return P9IDG_OK;
 }
 
 // Candidates of every tile with the parameters' lambda and alpha, control reset.
 p9idg_status cd_scan(p9idg_cd *cd) {
-    cd_scan_kernel<<<dim3(cd->tiles_x, cd->tiles_y), kCdNT, 0, cd->stream>>>(cd->hp);
+    const dim3 grid(cd->tiles_x, cd->tiles_y);
+    if (cd->hp.rows == 1)
+        cd_scan_kernel<1><<<grid, kCdNT, 0, cd->stream>>>(cd->hp);
+    else
+        cd_scan_kernel<2><<<grid, kCdNT, 0, cd->stream>>>(cd->hp);
     CK(cudaGetLastError());
     return P9IDG_OK;
 }
@@ -1217,10 +1311,11 @@ p9idg_status cd_run(p9idg_cd *cd, float *d_x, float *d_g, float lambda, float al
     // waits on the host; a launch after the stopping one does nothing (it sees the done flag).
     const int64_t launches = (static_cast<int64_t>(std::max(max_iter, 0)) + kCdLaunchIters - 1) / kCdLaunchIters;
     CdLaunch run(cd->hp.ax * cd->hp.ay, cd->stream);
-    if (launches > 0) CK(cudaLaunchKernelEx(&run.cfg, cd_run_kernel, cd->hp));
+    const auto kernel = cd->hp.rows == 1 ? cd_run_kernel<1> : cd_run_kernel<2>;
+    if (launches > 0) CK(cudaLaunchKernelEx(&run.cfg, kernel, cd->hp));
     for (int64_t r = 0; r < launches; r++) {
         CK(cudaEventRecord(cd->ev_ctl, cd->stream));
-        if (r + 1 < launches) CK(cudaLaunchKernelEx(&run.cfg, cd_run_kernel, cd->hp));
+        if (r + 1 < launches) CK(cudaLaunchKernelEx(&run.cfg, kernel, cd->hp));
         CK(cudaEventSynchronize(cd->ev_ctl));
         if (static_cast<volatile CdCtl *>(cd->h_ctl)->done) break;
     }
@@ -1272,12 +1367,7 @@ p9idg_status cd_init(p9idg_cd *cd, int n, const float *psf, int h, int w) {
     CK(cudaMallocHost(reinterpret_cast<void **>(&cd->h_pick), sizeof(unsigned long long)));
     CK(cudaEventCreateWithFlags(&cd->ev_ctl, cudaEventDisableTiming));
     cd->n = n;
-    cd->tiles_x = (n + kTX - 1) / kTX;
-    cd->tiles_y = (n + kTY - 1) / kTY;
-    const size_t nn = static_cast<size_t>(n) * n, nt = static_cast<size_t>(cd->tiles_x) * cd->tiles_y;
-    CK(cd->amap.ensure(sizeof(float) * nn));
-    CK(cd->tile_key.ensure(sizeof(unsigned long long) * nt));
-    CK(cd->cand.ensure(sizeof(CdCand) * kCdWarps * nt));
+    CK(cd->amap.ensure(sizeof(float) * static_cast<size_t>(n) * n));
     CK(cd->slots.ensure(sizeof(uint4) * 2 * kCdSlots));
     CK(cd->ctl.ensure(sizeof(CdCtl)));
     CK(cd->pick.ensure(sizeof(unsigned long long)));
@@ -1286,16 +1376,12 @@ p9idg_status cd_init(p9idg_cd *cd, int n, const float *psf, int h, int w) {
     cd->hp = CdParams{};
     cd->hp.a = cd->amap.as<float>();
     cd->hp.psf2 = cd->psf2.as<float>();
-    cd->hp.cand = cd->cand.as<CdCand>();
-    cd->hp.tile_key = cd->tile_key.as<unsigned long long>();
     cd->hp.slots = cd->slots.as<uint4>();
     cd->hp.ctl = cd->ctl.as<CdCtl>();
     cd->hp.report = cd->h_ctl;
     cd->hp.n = n;
     cd->hp.ph = cd->ph;
     cd->hp.pw = cd->pw;
-    cd->hp.tiles_x = cd->tiles_x;
-    cd->hp.tiles_y = cd->tiles_y;
     return cd_layout(cd);
 }
 
