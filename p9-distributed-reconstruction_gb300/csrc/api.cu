@@ -445,8 +445,10 @@ p9idg_status upload_items(p9idg_plan *p) {
 }
 
 // Device state for a call, without the uvw upload (in-place host calls start their transfers in
-// the other direction first and upload uvw beside them).
-p9idg_status prepare_state(p9idg_plan *p) {
+// the other direction first and upload uvw beside them).  Device calls (reset_status false) leave the
+// status word to the call that reads it: one launch less, and a check that trips is reported by the
+// next synchronisation whatever was queued after it.
+p9idg_status prepare_state(p9idg_plan *p, bool reset_status = true) {
     TRY(ensure_device(p));
     if (p->items_dirty) TRY(upload_items(p));
     if (p->taper_dirty) {
@@ -454,12 +456,13 @@ p9idg_status prepare_state(p9idg_plan *p) {
                            p->stream));
         p->taper_dirty = false;
     }
-    CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), p->stream));
+    if (reset_status) CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), p->stream));
     return P9IDG_OK;
 }
 
+// uvw null: a device call, on the plan's uvw
 p9idg_status prepare(p9idg_plan *p, const double *uvw) {
-    TRY(prepare_state(p));
+    TRY(prepare_state(p, uvw != nullptr));
     return upload_uvw(p, uvw);
 }
 
@@ -467,6 +470,7 @@ p9idg_status finish_call(p9idg_plan *p) {
     int32_t status = 0;
     CK(cudaMemcpyAsync(&status, p->d_status.p, sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
+    if (status != 0) CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), p->stream));
     if (p->timing) collect_timing(p);
     if (status == kStatusWTerm)
         return fail(P9IDG_UNSUPPORTED, "this call's uvw puts |dw r| above the bound of the plan's tensor-core "
@@ -643,7 +647,7 @@ p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const W
 
 // Subgrid IFFT + adder of nsub subgrids (all, or the subgrid list d_list) into the layers.
 p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const int32_t *d_list, int32_t nsub,
-                          bool dev_tc = false, bool device_call = false) {
+                          bool dev_tc = false, bool device_call = false, bool after_gridder = false) {
     StageScope t(p, P9IDG_STAGE_SUBGRID_IFFT_ADD);
     SubgridOpArgs a = subgrid_args(p);
     if (dev_tc) a.subs = static_cast<const DevSubgrid *>(p->tc.gsubs);
@@ -652,6 +656,7 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
     a.out_shifted = true;  // IDG.cs:17,37
     a.wstack = wstack;
     a.keep_bits = !device_call;
+    a.pdl = after_gridder && !p->timing;  // (a stage's events would be the launch before it)
     if (d_list) {
         a.sub_list = d_list;
         a.nsub = nsub;
@@ -676,7 +681,8 @@ p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d
         nitems = p->tc.ngitems;
     }
     const int64_t words = static_cast<int64_t>(nl) * static_cast<int64_t>(nn_of(p));
-    if (dev_tc && zero_in_kernel(words, nitems)) {
+    const bool fused = dev_tc && nitems > 0 && zero_in_kernel(words, nitems);
+    if (fused) {
         const ZeroFill zero{reinterpret_cast<uint2 *>(d_layers), nullptr, words, (words + kZeroPiece - 1) / kZeroPiece,
                             kZeroPiece, 0};
         TRY(grid_items(p, d_vis, vis_c128, items, nitems, dev_tc, zero));
@@ -687,7 +693,7 @@ p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d
         CK(launch_zero_c64_beside(d_layers, words, fill_outlasts_gridder(p, words, dev_tc || use_tc(p)), p->zside));
         TRY(z.join());
     }
-    return add_subgrids(p, d_layers, wstack, nullptr, 0, dev_tc, device_call);
+    return add_subgrids(p, d_layers, wstack, nullptr, 0, dev_tc, device_call, fused);
 }
 
 // grid (device complex64) -> vis (device, complex64 or complex128); uncovered samples are 0
@@ -733,6 +739,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         if (tc) {
             if (fused)
                 a.zero = {static_cast<uint2 *>(d_vis), p->d_gaps.as<int64_t>() + 2 * ngaps, 0, p->gap_pieces, 0, 0};
+            a.pdl = fused && !p->timing;
             TRY(tc_degrid(p->tc, a, p->mode, p->stream, g_last_error));
         } else {
             CK(launch_degridder_fp32(a, p->stream));

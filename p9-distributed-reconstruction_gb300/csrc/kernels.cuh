@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "p9idg_internal.h"
 
 namespace p9idg {
@@ -73,6 +75,29 @@ __device__ __forceinline__ void zero_piece(const ZeroFill &z, int64_t p, int thr
     }
 }
 
+// Programmatic dependent launch of a kernel after the one that feeds it: the first calls pdl_trigger when it
+// starts, the second pdl_wait before it touches anything the first (or an earlier kernel) writes, so that its
+// launch and set-up overlap the first one's last CTAs.  The wait holds until all of the first grid is done, and
+// does nothing in a launch without the attribute.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, bool pdl,
+                             Args &&...args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // ---- launchers (gridder_fp32.cu) ----
 struct GridderArgs {
     Geometry g;
@@ -92,6 +117,7 @@ struct GridderArgs {
     int32_t nsub;              // subgrids in `subs`
     int32_t *status;           // device status word
     ZeroFill zero;             // tensor-core kernels: what their loader warps zero (count 0: nothing)
+    bool pdl;                  // tensor-core degridder: the splitter is the launch before it
     // batched launches: work items left in this problem; the CTA finishing the last one
     // records the GPU time (ns) in *finish_ns.  Null when not tracked.
     int32_t *done;
@@ -136,6 +162,7 @@ struct SubgridOpArgs {
     const int32_t *sub_list;   // own launches: subgrid index per block (null: the block index)
     const float2 *twiddles;    // exp(+2 pi i j / S), j < S, made in FP64 (null, with keep_bits: made there)
     bool keep_bits;            // host-array calls: the form whose results those keep
+    bool pdl;                  // adder, own form: the tensor-core gridder is the launch before it
 };
 cudaError_t launch_subgrid_ifft_add(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);
 cudaError_t launch_split_subgrid_fft(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);

@@ -407,6 +407,8 @@ __global__ void __launch_bounds__(FftCfg<S>::kThreads, FftCfg<S>::kBlocks)
     const DevSubgrid sg = a.subs[sidx];
     int sx = sg.u, sy = sg.v, sw = sg.w;
     bool neg = false;
+    fft_twiddles<S>(tw, +1, a.twiddles);
+    pdl_wait();
     if (WSTACK) {
         neg = sw < 0;
         if (neg) {  // AdderWStack.cs:38-44
@@ -426,7 +428,6 @@ __global__ void __launch_bounds__(FftCfg<S>::kThreads, FftCfg<S>::kBlocks)
         }
         sw = 0;
     }
-    fft_twiddles<S>(tw, +1, a.twiddles);
     __syncthreads();
     const float2 *part = a.partials + static_cast<int64_t>(sg.item_begin) * S * S;
     float2 *layer = a.layers + static_cast<int64_t>(sw) * N * N;
@@ -469,6 +470,7 @@ __global__ void __launch_bounds__(FftCfg<S>::kThreads, FftCfg<S>::kBlocks)
     const bool neg = WSTACK && sg.w < 0;
     const bool in_range = WSTACK ? (sx >= 1 && sx < N - S && sy >= 1 && sy < N - S)
                                  : (sx >= 0 && sx < N - S && sy >= 0 && sy < N - S);
+    pdl_trigger();
     fft_twiddles<S>(tw, -1, a.twiddles);
     __syncthreads();
     float2 *out = a.subgrids + static_cast<int64_t>(sidx) * S * S;
@@ -506,10 +508,8 @@ template <int S, bool BATCH>
 cudaError_t fft_add_dispatch(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs) {
     if (a.nsub == 0) return cudaSuccess;
     if (a.wstack)
-        fft_ifft_add_kernel<S, true, BATCH><<<a.nsub, FftCfg<S>::kThreads, 0, st>>>(a, probs);
-    else
-        fft_ifft_add_kernel<S, false, BATCH><<<a.nsub, FftCfg<S>::kThreads, 0, st>>>(a, probs);
-    return cudaGetLastError();
+        return launch_dependent(fft_ifft_add_kernel<S, true, BATCH>, a.nsub, FftCfg<S>::kThreads, 0, st, a.pdl, a, probs);
+    return launch_dependent(fft_ifft_add_kernel<S, false, BATCH>, a.nsub, FftCfg<S>::kThreads, 0, st, a.pdl, a, probs);
 }
 
 template <int S, bool BATCH>

@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(kGThreads, 2)
         tmem_alloc(tmem_slot, kGTmemCols);
         tmem_relinquish();
     }
+    pdl_trigger();  // the adder
     const uint32_t sbase = smem_u32(smem), rbase = smem_u32(ring);
     tc_fence_before();
     __syncthreads();
@@ -808,6 +809,7 @@ __global__ void __launch_bounds__(kDThreads, 2)
         tmem_alloc(tmem_slot, kDTmemCols);
         tmem_relinquish();
     }
+    pdl_wait();  // for the splitter's subgrids (and coefficients just made)
     // Static B operand from the subgrid: row (block, 4 (y / 2) + 2 p + y % 2), k = 2x + q.  A thread
     // makes the four pixels of one (y, kg) once and writes their chunk of every block: taper, the
     // rotation by exp(-i dw0 r) to the subgrid's centre, r (.) and r^2 (.) for blocks 2 and 3; pixels
@@ -1455,11 +1457,11 @@ cudaError_t run_gridder(const TcArgs &t, const TcArgs *probs, int32_t nitems, co
 
 template <bool BF16, typename OutT, bool BATCH, bool TMA, bool O2>
 cudaError_t run_degridder(const TcArgs &t, const TcArgs *probs, int32_t nitems, const TmaMaps &maps,
-                          cudaStream_t stream) {
+                          cudaStream_t stream, bool pdl) {
     constexpr uint32_t smem = O2 ? kDSmem2 : kDSmem;
     cudaError_t e = set_smem(tc_degridder_kernel<BF16, OutT, BATCH, TMA, O2>, smem);
     if (e == cudaSuccess)
-        tc_degridder_kernel<BF16, OutT, BATCH, TMA, O2><<<nitems, kDThreads, smem, stream>>>(t, probs, maps);
+        e = launch_dependent(tc_degridder_kernel<BF16, OutT, BATCH, TMA, O2>, nitems, kDThreads, smem, stream, pdl, t, probs, maps);
     return e;
 }
 
@@ -1511,7 +1513,7 @@ p9idg_status launch_tc_gridder(const TcArgs &t, const TcArgs *probs, int32_t nit
 
 template <bool BATCH, bool O2>
 p9idg_status launch_tc_degridder(const TcArgs &t, const TcArgs *probs, int32_t nitems, bool c128, int mode,
-                                 const TmaMaps *maps, cudaStream_t stream, std::string &err) {
+                                 const TmaMaps *maps, cudaStream_t stream, std::string &err, bool pdl = false) {
     if (nitems == 0) return P9IDG_OK;
     static const TmaMaps kNoMaps{};
     const bool bf16 = mode == P9IDG_MODE_TC_BF16X3;
@@ -1521,25 +1523,25 @@ p9idg_status launch_tc_degridder(const TcArgs &t, const TcArgs *probs, int32_t n
     if constexpr (!BATCH) {
         if (maps) {
             if (bf16 && c128)
-                e = run_degridder<true, double2, false, true, O2>(t, probs, nitems, m, stream);
+                e = run_degridder<true, double2, false, true, O2>(t, probs, nitems, m, stream, pdl);
             else if (bf16)
-                e = run_degridder<true, float2, false, true, O2>(t, probs, nitems, m, stream);
+                e = run_degridder<true, float2, false, true, O2>(t, probs, nitems, m, stream, pdl);
             else if (c128)
-                e = run_degridder<false, double2, false, true, O2>(t, probs, nitems, m, stream);
+                e = run_degridder<false, double2, false, true, O2>(t, probs, nitems, m, stream, pdl);
             else
-                e = run_degridder<false, float2, false, true, O2>(t, probs, nitems, m, stream);
+                e = run_degridder<false, float2, false, true, O2>(t, probs, nitems, m, stream, pdl);
             done = true;
         }
     }
     if (!done) {
         if (bf16 && c128)
-            e = run_degridder<true, double2, BATCH, false, O2>(t, probs, nitems, m, stream);
+            e = run_degridder<true, double2, BATCH, false, O2>(t, probs, nitems, m, stream, pdl);
         else if (bf16)
-            e = run_degridder<true, float2, BATCH, false, O2>(t, probs, nitems, m, stream);
+            e = run_degridder<true, float2, BATCH, false, O2>(t, probs, nitems, m, stream, pdl);
         else if (c128)
-            e = run_degridder<false, double2, BATCH, false, O2>(t, probs, nitems, m, stream);
+            e = run_degridder<false, double2, BATCH, false, O2>(t, probs, nitems, m, stream, pdl);
         else
-            e = run_degridder<false, float2, BATCH, false, O2>(t, probs, nitems, m, stream);
+            e = run_degridder<false, float2, BATCH, false, O2>(t, probs, nitems, m, stream, pdl);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1641,9 +1643,9 @@ p9idg_status tc_degrid(TcPlanState &st, const GridderArgs &a, int mode, cudaStre
     TmaMaps maps;
     const bool tma = make_maps(maps, static_cast<const float4 *>(st.coef), st.ncoef, kDTile, nullptr, 0);
     return st.order == 2 ? launch_tc_degridder<false, true>(t, nullptr, st.nditems, a.out_c128, mode,
-                                                            tma ? &maps : nullptr, stream, err)
+                                                            tma ? &maps : nullptr, stream, err, a.pdl)
                          : launch_tc_degridder<false, false>(t, nullptr, st.nditems, a.out_c128, mode,
-                                                             tma ? &maps : nullptr, stream, err);
+                                                             tma ? &maps : nullptr, stream, err, a.pdl);
 }
 
 p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero, int mode,
