@@ -1340,35 +1340,57 @@ double tc_r_max(const std::vector<float> &lmn, int S) {
     return separable_tables(lmn, S, tabs);
 }
 
+// Host arrays that share one device allocation and one upload: a plan's first call pays for each of these
+// (an allocation and a copy of pageable memory take several microseconds apiece).
+namespace {
+struct Packed {
+    std::vector<unsigned char> host;
+    template <typename T>
+    size_t put(const std::vector<T> &v) {  // returns the offset
+        return put(v.data(), sizeof(T) * v.size());
+    }
+    size_t put(const void *src, size_t bytes) {
+        const size_t at = (host.size() + 255) / 256 * 256;
+        host.resize(at + std::max<size_t>(1, bytes));
+        if (src && bytes) std::memcpy(host.data() + at, src, bytes);
+        return at;
+    }
+    cudaError_t upload(void **block, cudaStream_t stream) const {
+        cudaError_t e = device_alloc(block, host.size());
+        return e == cudaSuccess ? cudaMemcpyAsync(*block, host.data(), host.size(), cudaMemcpyHostToDevice, stream) : e;
+    }
+};
+}  // namespace
+
 // The work items for the sizes asked for: degridder and gridder items (whole time samples, up to
-// degrid_chunk and grid_chunk visibilities each).
+// degrid_chunk and grid_chunk visibilities each).  Returns when the uploads queued before are done too.
 static p9idg_status tc_items(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, int nch, cudaStream_t stream,
                              std::string &err) {
     if (st.items_degrid == st.degrid_chunk && st.items_grid == st.grid_chunk) return P9IDG_OK;
-    cudaError_t e = cudaStreamSynchronize(stream);  // launches in flight read the lists replaced here
-    for (void **q : {&st.ditems, &st.gitems, &st.gsubs}) {
-        if (*q) cudaFree(*q);
-        *q = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (st.item_block) {
+        e = cudaStreamSynchronize(stream);  // launches in flight read the lists replaced here
+        cudaFree(st.item_block);
     }
+    st.item_block = st.ditems = st.gitems = st.gsubs = nullptr;
     st.items_degrid = st.items_grid = -1;
     std::vector<DevSubgrid> dtmp, gsubs;
     std::vector<WorkItem> ditems, gitems;
     build_work_items(subs, nch, st.degrid_chunk, dtmp, ditems);
     build_work_items(subs, nch, st.grid_chunk, gsubs, gitems);
-    const auto put = [&](void **dst, const auto &v) {
-        using T = typename std::decay<decltype(v)>::type::value_type;
-        if (e == cudaSuccess) e = device_alloc(dst, sizeof(T) * std::max<size_t>(1, v.size()));
-        if (e == cudaSuccess && !v.empty())
-            e = cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream);
-    };
-    put(&st.ditems, ditems);
-    put(&st.gitems, gitems);
-    put(&st.gsubs, gsubs);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    Packed p;
+    const size_t at_d = p.put(ditems), at_g = p.put(gitems), at_s = p.put(gsubs);
+    if (e == cudaSuccess) e = p.upload(&st.item_block, stream);
+    const cudaError_t es = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) {
         err = std::string("tensor-core work items: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
     }
+    unsigned char *base = static_cast<unsigned char *>(st.item_block);
+    st.ditems = base + at_d;
+    st.gitems = base + at_g;
+    st.gsubs = base + at_s;
     st.nditems = static_cast<int32_t>(ditems.size());
     st.ngitems = st.nslots = static_cast<int32_t>(gitems.size());
     st.items_degrid = st.degrid_chunk;
@@ -1405,24 +1427,25 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     st.dw_scale = pow2_below(dw_max * 1.0001);
     st.r_scale = pow2_below(rmax);
     st.ncoef = off.back();
-    cudaError_t e;
-    if ((e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef))) != cudaSuccess ||
-        (e = device_alloc(&st.coef_off, sizeof(int64_t) * off.size())) != cudaSuccess ||
-        (e = device_alloc(&st.center, sizeof(float) * std::max<size_t>(1, subs.size()))) != cudaSuccess ||
-        (e = device_alloc(&st.tables, sizeof(float) * tabs.size())) != cudaSuccess) {
+    Packed p;
+    const size_t at_off = p.put(off), at_tabs = p.put(tabs),
+                 at_center = p.put(nullptr, sizeof(float) * subs.size());  // made by the coefficient kernel
+    cudaError_t e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef));
+    if (e == cudaSuccess) e = p.upload(&st.block, stream);
+    if (e != cudaSuccess) {
         err = std::string("tensor-core buffers: ") + cudaGetErrorString(e);
         tc_release(st);
         return e == cudaErrorMemoryAllocation ? P9IDG_OUT_OF_MEMORY : P9IDG_CUDA_ERROR;
     }
-    cudaMemcpyAsync(st.coef_off, off.data(), sizeof(int64_t) * off.size(), cudaMemcpyHostToDevice, stream);
-    cudaMemcpyAsync(st.tables, tabs.data(), sizeof(float) * tabs.size(), cudaMemcpyHostToDevice, stream);
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) {
-        err = std::string("tensor-core tables: ") + cudaGetErrorString(e);
-        return P9IDG_CUDA_ERROR;
-    }
+    unsigned char *base = static_cast<unsigned char *>(st.block);
+    st.coef_off = base + at_off;
+    st.tables = base + at_tabs;
+    st.center = base + at_center;
     st.S = S;
     st.ready = true;
-    return tc_items(st, subs, nch, stream, err);
+    const p9idg_status s = tc_items(st, subs, nch, stream, err);
+    if (s != P9IDG_OK) cudaStreamSynchronize(stream);  // p's upload
+    return s;
 }
 
 // Per-visibility phase coefficients depend only on the plan and uvw: computed once and kept
@@ -1668,12 +1691,8 @@ p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t
 
 void tc_release(TcPlanState &st) {
     if (st.coef) cudaFree(st.coef);
-    if (st.coef_off) cudaFree(st.coef_off);
-    if (st.center) cudaFree(st.center);
-    if (st.tables) cudaFree(st.tables);
-    if (st.ditems) cudaFree(st.ditems);
-    if (st.gitems) cudaFree(st.gitems);
-    if (st.gsubs) cudaFree(st.gsubs);
+    if (st.block) cudaFree(st.block);
+    if (st.item_block) cudaFree(st.item_block);
     st = TcPlanState();
 }
 

@@ -18,6 +18,8 @@ struct TcPlanState {
     int S = 0;
     int64_t ncoef = 0;
     void *coef = nullptr;         // float4 {du, dv, dw, dw - centre} per gridded visibility, subgrid order
+    // one allocation each: center, coef_off and tables; ditems, gitems and gsubs
+    void *block = nullptr, *item_block = nullptr;
     void *center = nullptr;       // float per subgrid: its centre dw0 = mean(dw)
     void *coef_off = nullptr;     // int64 per subgrid: first coefficient of the subgrid
     void *tables = nullptr;       // float: g[32] (separable part of n), r[32][32] (remainder), l[32],
