@@ -195,17 +195,6 @@ __device__ __forceinline__ float block256_max(float v, float *red) {
 
 // ---------------- per-visibility coefficients (FP64 -> FP32) ----------------
 
-// Sum over the block (256 threads); red: 8 doubles of shared memory.
-__device__ __forceinline__ double block256_sum(double v, double *red) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    v = red[0];
-    for (int i = 1; i < 8; i++) v += red[i];
-    __syncthreads();
-    return v;
-}
-
 // One block per subgrid: its centre dw0 (the mean over its samples of dw = woff - k w; times and
 // channels are a full product, so the mean of k times the mean of w), then its visibilities'
 // coefficients.  dw_limit = the form's limit / max |r|: a visibility with a larger |dw| (possible only
@@ -214,7 +203,7 @@ __device__ __forceinline__ double block256_sum(double v, double *red) {
 __global__ void __launch_bounds__(256)
     tc_coef_kernel(const DevSubgrid *subs, const int64_t *coef_off, const double *uvw, const double *wn, Geometry g,
                    float4 *coef, float *center, const int32_t *recompute, double dw_limit, int32_t *status) {
-    __shared__ double red[8];
+    __shared__ double mean[2], off[3];  // of w and of k; the subgrid's u, v and w phase
     if (recompute && *recompute == 0) return;  // uvw bit-identical to the one coef was made from
     const DevSubgrid sg = subs[blockIdx.x];
     const int nvis = sg.nt * g.nch;
@@ -222,16 +211,24 @@ __global__ void __launch_bounds__(256)
         if (threadIdx.x == 0) center[blockIdx.x] = 0.f;
         return;
     }
-    const double uoff = static_cast<double>(sg.u + g.S / 2 - g.N / 2) * g.uv_scale;
-    const double voff = static_cast<double>(sg.v + g.S / 2 - g.N / 2) * g.uv_scale;
-    const double woff = 2 * kPi * (static_cast<double>(g.wstep_lambda) * (static_cast<double>(sg.w) + 0.5));
     const double *base = uvw + (static_cast<int64_t>(sg.bl) * g.nt_all + sg.t0) * 3;
-    double ws = 0, ks = 0;
-    for (int t = threadIdx.x; t < sg.nt; t += blockDim.x) ws += base[3 * static_cast<int64_t>(t) + 2];
-    for (int c = threadIdx.x; c < g.nch; c += blockDim.x) ks += wn[c];
-    ws = block256_sum(ws, red);
-    ks = block256_sum(ks, red);
-    const float dw0 = static_cast<float>(woff - (ks / g.nch) * (ws / sg.nt));
+    // FP64 instructions are what this kernel's time goes into (the pipe is 86 % busy), so one warp does each of
+    // these: 38 M visibilities in 12,889 subgrids 0.71 ms, 1.12 when every thread made them
+    if (threadIdx.x < 64) {
+        const bool of_k = threadIdx.x >= 32;
+        const int n = of_k ? g.nch : sg.nt;
+        double sum = 0;
+        for (int i = threadIdx.x & 31; i < n; i += 32) sum += of_k ? wn[i] : base[3 * static_cast<int64_t>(i) + 2];
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) mean[of_k] = sum / n;
+    } else if (threadIdx.x == 64) {
+        off[0] = static_cast<double>(sg.u + g.S / 2 - g.N / 2) * g.uv_scale;
+        off[1] = static_cast<double>(sg.v + g.S / 2 - g.N / 2) * g.uv_scale;
+        off[2] = 2 * kPi * (static_cast<double>(g.wstep_lambda) * (static_cast<double>(sg.w) + 0.5));
+    }
+    __syncthreads();
+    const double uoff = off[0], voff = off[1], woff = off[2];
+    const float dw0 = static_cast<float>(woff - mean[1] * mean[0]);
     if (threadIdx.x == 0) center[blockIdx.x] = dw0;
     float4 *out = coef + coef_off[blockIdx.x];
     bool over = false;
