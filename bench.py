@@ -678,7 +678,7 @@ def main():
     plan = part.plan
     info = plan.info()
     headline = "tc_bf16x3" if args.mode == "auto" else args.mode
-    # config 3 times both split-precision forms beside the FP32 kernels
+    # config 3 times both split-precision forms beside the FP32 mode
     compare = ["fp32", "tc_fp16x3"] if args.mode == "auto" else []
 
     stream = torch.cuda.Stream()
@@ -715,11 +715,11 @@ def main():
                              value=2 * total_gridded * args.steps / (ms * 1e-3) / 1e6)
     head = results[headline]
     stages = head["stages"]
-    # one launch per timed stage, plus the two zero-fills each step runs beside the gridder (w layers)
-    # and the degridder (uncovered visibilities), outside the stages
-    launches = sum(n for (_, n) in stages.values()) - stages["h2d"][1] - stages["d2h"][1] + 2 * args.steps
+    # one launch per timed stage (the gridder and the degridder zero the w layers and the uncovered
+    # visibilities themselves)
+    launches = sum(n for (_, n) in stages.values()) - stages["h2d"][1] - stages["d2h"][1]
 
-    # tensor-core vs FP32 kernels on the whole workload: w layers, degridded visibilities, dirty image
+    # split-precision vs FP32 mode on the whole workload: w layers, degridded visibilities, dirty image
     tc_vs_fp32 = None
     if compare:
         outs = {}
@@ -752,27 +752,25 @@ def main():
     peaks, peak_src = measured_peaks()
     kern = max(("gridder", "degridder"), key=lambda k: stages[k][0])
     kt_ms = stages[kern][0] / max(1, stages[kern][1])
-    if headline == "fp32":
-        sincos_peak, _ = pkg.measure_sincos_peak()
-        achieved = gridded * S * S / (kt_ms * 1e-3) / 1e9
-        roofline = {"bound": "sfu", "achieved": achieved, "peak": sincos_peak / 1e9, "unit": "Gsincos/s",
-                    "frac": achieved / (sincos_peak / 1e9), "traffic": traffic_per_launch(kern + "_fp32"),
-                    "kernel": kern + "_fp32", "peak_source": "measured on this GPU (hardware sincos probe loop)",
-                    "work_per_launch": f"{gridded} visibilities x {S * S} pixels, one sincos + 10 flop each"}
-    else:
+
+    def tensor_roofline(kern, kt_ms, mode):
         achieved = gridded * 10 * S * S / (kt_ms * 1e-3) / 1e12
         # tcgen05 work actually issued per visibility: gridder one M128 N192 K16 MMA per 16 visibilities;
         # degridder 3 MMAs (N128 + N64 + N64, K16) per 128 visibilities x 4 K chunks / 128
         phys = (2 * 128 * 192 * 16 / 16) if kern == "gridder" else (2 * 128 * 256 * 64 / 128)
-        roofline = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
-                    "frac": achieved / peaks["bf16_tflops"], "traffic": traffic_per_launch(kern + "_" + headline),
-                    "kernel": kern + "_" + headline,
-                    "peak_source": f"{peak_src} dense bf16 (MEASURED_PEAKS.json bf16_tflops)",
-                    "work_per_launch": f"{gridded} visibilities x {S * S} pixels x 10 algorithmic flop",
-                    "physical_mma_tflops": gridded * phys / (kt_ms * 1e-3) / 1e12,
-                    "physical_mma_frac": gridded * phys / (kt_ms * 1e-3) / 1e12 / peaks["bf16_tflops"],
-                    "note": "algorithmic flop counts one complex MAC + phase per pixel and visibility (the FP32 "
-                            "kernel's work); the tensor-core kernels issue the physical MMA flop instead"}
+        return {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
+                "frac": achieved / peaks["bf16_tflops"],
+                "traffic": traffic_per_launch(kern + "_" + mode) if mode != "fp32" else None,
+                "kernel": kern + "_" + mode,
+                "peak_source": f"{peak_src} dense bf16 (MEASURED_PEAKS.json bf16_tflops)",
+                "work_per_launch": f"{gridded} visibilities x {S * S} pixels x 10 algorithmic flop",
+                "physical_mma_tflops": gridded * phys / (kt_ms * 1e-3) / 1e12,
+                "physical_mma_frac": gridded * phys / (kt_ms * 1e-3) / 1e12 / peaks["bf16_tflops"],
+                "note": "algorithmic flop counts one complex MAC + phase per pixel and visibility (the sincos "
+                        "kernels' work); the tensor-core kernels issue the physical MMA flop instead"
+                        + (" (FP32 mode: FP16 hi+lo operands about each subgrid's own w)" if mode == "fp32" else "")}
+
+    roofline = tensor_roofline(kern, kt_ms, headline)
 
     # e2e through the reference-facing host API (IDG.GridW + IDG.DeGridW) with pinned host buffers
     e2e = None
@@ -892,23 +890,9 @@ def main():
                      "per_stage_ms": {k: round(v[0] / max(1, v[1]), 4) for k, v in r["stages"].items() if v[1]}}
                  for m, r in results.items()}
         if "fp32" in results and headline != "fp32":
-            # the FP32 kernels against their own ceiling: one hardware sincos per pixel and visibility,
-            # divided by the measured sincos rate of the same intrinsic on this GPU (an ncu capture shows
-            # the probe and the FP32 gridder at the same XU-pipe limit, ~49 % of the XU instruction peak)
-            sincos_peak, _ = pkg.measure_sincos_peak()
             st32 = results["fp32"]["stages"]
             k32 = max(("gridder", "degridder"), key=lambda k: st32[k][0])
-            per_kernel = {}
-            for k in ("gridder", "degridder"):
-                ms_k = st32[k][0] / max(1, st32[k][1])
-                per_kernel[k] = gridded * S * S / (ms_k * 1e-3) / 1e9
-            modes["fp32"]["roofline"] = {
-                "bound": "sfu", "achieved": per_kernel[k32], "peak": sincos_peak / 1e9, "unit": "Gsincos/s",
-                "frac": per_kernel[k32] / (sincos_peak / 1e9), "kernel": k32 + "_fp32",
-                "frac_per_kernel": {k: v / (sincos_peak / 1e9) for k, v in per_kernel.items()},
-                "traffic": traffic_per_launch(k32 + "_fp32"),
-                "peak_source": "measured on this GPU: p9idg_measure_sincos_peak (independent chains of __sincosf)",
-                "work_per_launch": f"{gridded} visibilities x {S * S} pixels, one sincos each"}
+            modes["fp32"]["roofline"] = tensor_roofline(k32, st32[k32][0] / max(1, st32[k32][1]), "fp32")
         out = {"metric": METRIC, "value": head["value"], "unit": "Mvis/s", "n_gpus": ws, "steps": args.steps,
                "warmup": max(3, args.warmup), "ms_per_step": head["ms"] / args.steps, "higher_is_better": True,
                "scaling": "strong", "vs_baseline": None, "dtype": "f32" if headline == "fp32" else headline,

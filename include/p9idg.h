@@ -198,9 +198,10 @@ p9idg_status p9idg_fft_shift(void *array, int32_t n, int32_t elem_bytes);
 
 /* ---------------- device-resident interface (HBM buffers, complex64 = float2) ---------------- */
 /* These run asynchronously on the plan's stream; p9idg_synchronize waits and
- * reports kernel-side check failures.  uvw and frequencies are the plan's.  The zeroing of an
- * output runs on a second stream of the plan, forked from the plan's stream and joined back into
- * it within the call, so all of a call's work is ordered on the plan's stream. */
+ * reports kernel-side check failures of the calls since the last report.  uvw and frequencies are the
+ * plan's.  An output is zeroed by the tensor-core kernels themselves or on a second stream of the plan,
+ * forked from the plan's stream and joined back into it within the call, so all of a call's work is
+ * ordered on the plan's stream. */
 
 /* Gridder + subgrid IFFT + w-stack adder: vis complex64[nbl][nt][nch] -> layers complex64[W][N][N]
  * (already FFT.Shift-ed, as IDG.GridW returns them).  The layers are overwritten. */
@@ -245,7 +246,9 @@ p9idg_status p9idg_grid_w_device_noalloc(const p9idg_params *c, const p9idg_subg
 typedef struct p9idg_batch p9idg_batch;
 
 /* Work-item sizes (visibilities per gridder / degridder item; 0 = default: FP32 1024 / 512,
- * tensor core 4096 / 16384) -- the time-chunk length the autotuner chooses. */
+ * tensor core 4096 / 16384, less where a small observation would not fill the GPU) -- the time-chunk
+ * length the autotuner chooses.  In FP32 mode the sizes are the sincos kernels' items; its tensor-core
+ * form takes 4 and 32 times as many visibilities. */
 p9idg_status p9idg_plan_set_chunking(p9idg_plan *plan, int32_t gridder_max_vis, int32_t degridder_max_vis);
 p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const void *const *d_vis,
                                 void *const *d_layers, const void *const *d_grids, void *const *d_vis_out,
