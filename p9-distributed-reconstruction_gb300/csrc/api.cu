@@ -1298,12 +1298,16 @@ p9idg_status batch_grid(p9idg_batch *b) {
                               b->tc_order, b->stream, g_last_error));
         }
     }
+    // the launch before the first adder is the last group's gridder
+    bool pdl = !b->groups.empty() && b->groups.back().tc && b->groups.back().gn > 0;
     for (const auto &g : b->groups) {
         SubgridOpArgs A{};
         A.g.S = g.S;
         A.refs = b->d_refs.as<int2>() + g.r0;
         A.nsub = g.rn;
         A.wstack = true;
+        A.pdl = pdl;
+        if (g.rn > 0) pdl = false;
         if (g.rn > 0) CK(launch_subgrid_ifft_add(A, b->stream, b->d_aargs.as<SubgridOpArgs>()));
     }
     return P9IDG_OK;
@@ -1331,11 +1335,13 @@ p9idg_status batch_degrid(p9idg_batch *b) {
         L.g.S = g.S;
         L.items = b->d_ditems.as<WorkItem>() + g.d0;
         L.nitems = g.dn;
+        // the launch before the first degridder is the last group's splitter
+        const bool pdl = k == 0 && b->groups.back().rn > 0;
         if (!g.tc) {
             if (g.dn > 0) CK(launch_degridder_fp32(L, b->stream, b->d_dargs.as<GridderArgs>()));
         } else {
             TRY(tc_degrid_batch(b->d_td.as<TcArgs>(), L.items, g.dn, static_cast<int>(k) == zk ? zero : ZeroFill{},
-                                b->mode, b->tc_order, b->stream, g_last_error));
+                                b->mode, b->tc_order, b->stream, g_last_error, pdl));
         }
     }
     return P9IDG_OK;

@@ -1678,12 +1678,12 @@ p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t n
 }
 
 p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero,
-                             int mode, int order, cudaStream_t stream, std::string &err) {
+                             int mode, int order, cudaStream_t stream, std::string &err, bool pdl) {
     TcArgs t{};
     t.items = items;
     t.zero = zero;
-    return order == 2 ? launch_tc_degridder<true, true>(t, probs, nitems, false, mode, nullptr, stream, err)
-                      : launch_tc_degridder<true, false>(t, probs, nitems, false, mode, nullptr, stream, err);
+    return order == 2 ? launch_tc_degridder<true, true>(t, probs, nitems, false, mode, nullptr, stream, err, pdl)
+                      : launch_tc_degridder<true, false>(t, probs, nitems, false, mode, nullptr, stream, err, pdl);
 }
 
 void tc_release(TcPlanState &st) {

@@ -95,7 +95,7 @@ p9idg_status tc_coefs(TcPlanState &st, const GridderArgs &a, cudaStream_t stream
 p9idg_status tc_grid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero, int mode,
                            int order, cudaStream_t stream, std::string &err);
 p9idg_status tc_degrid_batch(const TcArgs *probs, const WorkItem *items, int32_t nitems, const ZeroFill &zero,
-                             int mode, int order, cudaStream_t stream, std::string &err);
+                             int mode, int order, cudaStream_t stream, std::string &err, bool pdl);
 // The form (1 or 2) a plan with this w term runs for a requested order (0 = automatic), or 0 when
 // neither bound holds (the plan then keeps the FP32 kernels).
 int tc_order_for(double w_term, int want_order);
