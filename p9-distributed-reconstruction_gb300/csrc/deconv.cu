@@ -126,7 +126,7 @@ constexpr int kNT = 512, kWarps = kNT / 32;  // image reductions
 constexpr int kTX = 128, kCdNT = 640, kCdWarps = kCdNT / 32, kCdCols = kTX / 32;
 // Slots of the exchange, three for each lane of the polling warp; pairs of CTAs share one from
 // kCdPairFrom CTAs on.  Measured for the exchange alone: 1270 clocks with 30 CTAs, each polling every
-// slot, 3500 with 147 (the polls of one line queue up), 2490 with 74 pairs; pairs of 30 take 2040.
+// slot, 3500 with 147 (the polls of one line queue up), 2000 with 74 pairs; 30 CTAs in pairs take 1860.
 constexpr int kCdPoll = 3, kCdSlots = 32 * kCdPoll, kCdPairFrom = 56;
 // Iterations of one launch: few enough that other streams' kernels wait milliseconds for the SMs, not
 // for a whole deconvolution, and enough that a launch does not show.
