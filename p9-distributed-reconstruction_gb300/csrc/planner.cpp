@@ -297,15 +297,16 @@ void build_work_items(const std::vector<p9idg_subgrid> &subs, int32_t nch, int64
                       std::vector<DevSubgrid> &dsub, std::vector<WorkItem> &items) {
     dsub.resize(subs.size());
     items.clear();
-    const int32_t chunk = static_cast<int32_t>(std::max<int64_t>(1, max_vis / std::max<int32_t>(1, nch)));
+    // (64 bits: a size may be larger than any subgrid, which then is one item)
+    const int64_t chunk = std::max<int64_t>(1, max_vis / std::max<int32_t>(1, nch));
     int32_t slot = 0;
     for (size_t i = 0; i < subs.size(); i++) {
         const p9idg_subgrid &s = subs[i];
         DevSubgrid &d = dsub[i];
         d = {s.baseline_idx, s.time_sample_start, s.time_sample_count, s.u_pixel, s.v_pixel, s.w_lambda, slot, 0};
-        for (int32_t t = 0; t < s.time_sample_count; t += chunk) {
-            const int32_t len = std::min(chunk, s.time_sample_count - t);
-            items.push_back({static_cast<int32_t>(i), s.time_sample_start + t, len, slot++, 0, 0});
+        for (int64_t t = 0; t < s.time_sample_count; t += chunk) {
+            const int32_t len = static_cast<int32_t>(std::min<int64_t>(chunk, s.time_sample_count - t));
+            items.push_back({static_cast<int32_t>(i), s.time_sample_start + static_cast<int32_t>(t), len, slot++, 0, 0});
             d.item_count++;
         }
     }
