@@ -1240,6 +1240,7 @@ struct p9idg_batch {
         int32_t g0, gn, d0, dn, r0, rn;
     };
     std::vector<Group> groups;
+    std::vector<int32_t> prob_key;             // group of each problem: its plan's mode may change after the batch was made
     int tc_order = 1;  // tensor-core batches: 2 when any plan needs the second-order form
     std::vector<int64_t> prob_vis;             // visibilities per problem (for the schedules)
     int32_t schedule = P9IDG_SCHEDULE_THROUGHPUT;
@@ -1252,7 +1253,7 @@ struct p9idg_batch {
 
 namespace {
 
-// Whether a plan's batch launches run on the tensor cores, and the group it belongs to.
+// Whether a plan's launches in a batch made now run on the tensor cores, and the group it belongs to.
 bool batch_tc(const p9idg_plan *p) { return use_tc(p) || use_fp32_tc(p, true); }
 int32_t group_key(const p9idg_plan *p) { return 2 * p->c.subgrid_size + (batch_tc(p) ? 1 : 0); }
 
@@ -1366,7 +1367,7 @@ p9idg_status batch_order(p9idg_batch *b, int32_t schedule) {
             return pv[x.problem] != pv[y.problem] ? pv[x.problem] < pv[y.problem] : x.problem < y.problem;
         return item_vis(x) > item_vis(y);
     };
-    auto key_of = [&](const WorkItem &w) { return group_key(b->plans[w.problem]); };
+    auto key_of = [&](const WorkItem &w) { return b->prob_key[w.problem]; };
     for (auto *v : {&b->h_gitems, &b->h_ditems}) {
         if (schedule == P9IDG_SCHEDULE_SMALL_FIRST)
             std::stable_sort(v->begin(), v->end(), small_first);
@@ -1971,9 +1972,11 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         }
         done[i] = static_cast<int32_t>(dsrc.size());
         for (size_t s = 0; s < p->dsub.size(); s++) refs.push_back(make_int2(i, static_cast<int>(s)));
+        const int32_t key = group_key(p);
+        b->prob_key.push_back(key);
         bool known = false;
-        for (const auto &g : b->groups) known |= g.key == group_key(p);
-        if (!known) b->groups.push_back({group_key(p), S, tc, 0, 0, 0, 0, 0, 0});
+        for (const auto &g : b->groups) known |= g.key == key;
+        if (!known) b->groups.push_back({key, S, tc, 0, 0, 0, 0, 0, 0});
         if ((st = ensure_gaps(p)) != P9IDG_OK) return bail(st);
         const auto zero = [](std::vector<int64_t> &v, int64_t &total, void *base, int64_t first, int64_t words) {
             const int64_t at = static_cast<int64_t>(reinterpret_cast<uintptr_t>(base) / 8) + first;
@@ -1993,12 +1996,12 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
               [](const p9idg_batch::Group &x, const p9idg_batch::Group &y) { return x.key < y.key; });
     // subgrid references grouped the same way (plan order inside a group)
     std::stable_sort(refs.begin(), refs.end(),
-                     [&](const int2 &x, const int2 &y) { return group_key(plans[x.x]) < group_key(plans[y.x]); });
+                     [&](const int2 &x, const int2 &y) { return b->prob_key[x.x] < b->prob_key[y.x]; });
     for (auto &g : b->groups) {
         g.r0 = g.rn = 0;
         bool rs = false;
         for (size_t k = 0; k < refs.size(); k++)
-            if (group_key(plans[refs[k].x]) == g.key) {
+            if (b->prob_key[refs[k].x] == g.key) {
                 if (!rs) g.r0 = static_cast<int32_t>(k), rs = true;
                 g.rn++;
             }
