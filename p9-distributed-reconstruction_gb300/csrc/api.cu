@@ -1228,7 +1228,7 @@ struct p9idg_batch {
     int32_t mode = P9IDG_MODE_FP32;
     cudaStream_t stream = nullptr;
     DevBuf d_gargs, d_dargs, d_aargs, d_sargs, d_tg, d_td;  // per-problem argument tables
-    DevBuf d_gitems, d_ditems, d_subs, d_refs, d_done_init, d_done, d_finish, d_start;
+    DevBuf d_gitems, d_ditems, d_subs, d_partials, d_refs, d_done_init, d_done, d_finish, d_start;
     int32_t ngitems = 0, nditems = 0, nrefs = 0;
     std::vector<WorkItem> h_gitems, h_ditems;  // merged work items of all problems, in launch order
     // problems may mix subgrid sizes, and FP32 ones the two forms of that mode: the items and subgrid
@@ -1400,8 +1400,9 @@ p9idg_status batch_order(p9idg_batch *b, int32_t schedule) {
 void batch_release(p9idg_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
-    DevBuf *bufs[] = {&b->d_gargs, &b->d_dargs, &b->d_aargs, &b->d_sargs, &b->d_tg, &b->d_td, &b->d_gitems,
-                      &b->d_zgrid, &b->d_zvis, &b->d_ditems, &b->d_subs, &b->d_refs, &b->d_done_init, &b->d_done, &b->d_finish, &b->d_start};
+    DevBuf *bufs[] = {&b->d_gargs, &b->d_dargs,  &b->d_aargs,    &b->d_sargs, &b->d_tg,        &b->d_td,   &b->d_gitems, &b->d_zgrid,
+                      &b->d_zvis,  &b->d_ditems, &b->d_partials, &b->d_subs,  &b->d_refs,      &b->d_done_init, &b->d_done,
+                      &b->d_finish, &b->d_start};
     for (DevBuf *x : bufs) x->release();
     if (b->stream) cudaStreamDestroy(b->stream);
 }
@@ -1892,6 +1893,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     std::vector<int2> refs;
     std::vector<int64_t> zgrid, zvis;
     std::vector<int32_t> done(nplans, 0);
+    size_t partial_bytes = 0;
     // device-side completion tracking first: the argument tables point into it
     p9idg_status st;
     for (int i = 0; i < nplans; i++) {
@@ -1925,16 +1927,16 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
                              dslots, dwork);
         }
         const std::vector<WorkItem> &gsrc = tc ? gwork : p->gitems, &dsrc = tc ? dwork : p->ditems;
-        // (and room for the plan's own calls, which must not move the buffer under the batch)
-        const size_t slots_max = std::max({gsrc.size(), static_cast<size_t>(p->nslots),
-                                           static_cast<size_t>(tc ? p->tc.nslots : 0), size_t(1)});
-        cudaError_t e = p->d_partials.ensure(sizeof(float2) * S * S * slots_max);
-        if (e == cudaSuccess) e = p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size()));
+        // the partial subgrids too are the batch's own: the plan's grow with its mode and its work-item sizes, and
+        // would leave the batch with the address of freed memory (an offset here as well)
+        float2 *const partials = reinterpret_cast<float2 *>(partial_bytes);
+        partial_bytes += sizeof(float2) * S * S * gsrc.size();
+        cudaError_t e = p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size()));
         if (e != cudaSuccess) return bail(cuda_fail(e, "plan buffers"));
         ga[i] = gridder_args(p);
         ga[i].vis = d_vis[i];
         ga[i].vis_c128 = false;
-        ga[i].partials = p->d_partials.as<float2>();
+        ga[i].partials = partials;
         da[i] = gridder_args(p);
         da[i].subgrids = p->d_subgrids.as<float2>();
         da[i].vis_out = d_vis_out[i];
@@ -1947,7 +1949,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         aa[i].subs = reinterpret_cast<const DevSubgrid *>(sizeof(DevSubgrid) * subs.size());
         const std::vector<DevSubgrid> &slots = tc ? gslots : p->dsub;
         subs.insert(subs.end(), slots.begin(), slots.end());
-        aa[i].partials = p->d_partials.as<float2>();
+        aa[i].partials = partials;
         aa[i].layers = static_cast<float2 *>(d_layers[i]);
         aa[i].out_shifted = true;
         aa[i].wstack = true;
@@ -2018,8 +2020,17 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     if ((st = upload(b->d_zgrid, zgrid)) != P9IDG_OK || (st = upload(b->d_zvis, zvis)) != P9IDG_OK ||
         (st = upload(b->d_subs, subs)) != P9IDG_OK)
         return bail(st);
-    for (auto &x : aa)
-        x.subs = reinterpret_cast<const DevSubgrid *>(b->d_subs.as<char>() + reinterpret_cast<uintptr_t>(x.subs));
+    {
+        cudaError_t e = b->d_partials.ensure(std::max<size_t>(1, partial_bytes));
+        if (e != cudaSuccess) return bail(cuda_fail(e, "batch partial subgrids"));
+    }
+    const auto moved = [](const DevBuf &buf, const void *offset) { return buf.as<char>() + reinterpret_cast<uintptr_t>(offset); };
+    for (auto &x : aa) {
+        x.subs = reinterpret_cast<const DevSubgrid *>(moved(b->d_subs, x.subs));
+        x.partials = reinterpret_cast<float2 *>(moved(b->d_partials, x.partials));
+    }
+    for (auto &x : ga) x.partials = reinterpret_cast<float2 *>(moved(b->d_partials, x.partials));
+    for (auto &x : tg) x.partials = reinterpret_cast<float2 *>(moved(b->d_partials, x.partials));
     if ((st = upload(b->d_gargs, ga)) != P9IDG_OK || (st = upload(b->d_dargs, da)) != P9IDG_OK ||
         (st = upload(b->d_aargs, aa)) != P9IDG_OK || (st = upload(b->d_sargs, sa)) != P9IDG_OK ||
         (st = upload(b->d_tg, tg)) != P9IDG_OK || (st = upload(b->d_td, td)) != P9IDG_OK ||

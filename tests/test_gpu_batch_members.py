@@ -63,3 +63,30 @@ def test_member_changes_mode_then_schedule(need_gpu, mode, other, sizes):
     batch.capture_graph()
     _same(_run(batch, probs), ref)
     batch.destroy()
+
+
+def test_member_needs_more_partial_subgrids_of_its_own(need_gpu):
+    """The plan's own calls with smaller work items, in another mode and in the batch's, between runs and replays
+    of the batch: they need more partial subgrids than the batch does, in memory that the batch does not use."""
+    probs = _problems(pkg.MODE_TC_BF16X3, [(32, 8, 256), (16, 4, 300)])
+    batch = _batch(probs)
+    batch.capture_graph()
+    ref = _run(batch, probs)
+    for part, c, obs, b in probs:
+        plan = part.plan
+        slots = plan.info()["work_items"]
+        pkg.set_chunking(plan, 64, 64)
+        assert plan.info()["work_items"] > 4 * slots
+        lay, vis = torch.empty_like(b["layers"]), torch.empty_like(b["out"])
+        plan.grid_w_device(b["vis"].data_ptr(), lay.data_ptr())
+        plan.degrid_w_device(b["grid"].data_ptr(), vis.data_ptr())
+        plan.synchronize()
+        assert plan.set_mode(pkg.MODE_FP32) == pkg.MODE_FP32
+        pkg.IDG.GridW(c, part, obs.vis, obs.uvw, obs.frequencies)
+        # what the plans gave back is used by others, as a program's next allocation would
+        junk = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(32)]
+    _same(_run(batch, probs), ref)
+    batch.set_schedule(pkg.Batch.SMALL_FIRST)
+    _same(_run(batch, probs), ref)
+    del junk
+    batch.destroy()
