@@ -626,7 +626,9 @@ bool fill_outlasts_gridder(const p9idg_plan *p, int64_t words, bool tc) {
 p9idg_status grid_items(p9idg_plan *p, const void *d_vis, bool vis_c128, const WorkItem *d_items, int32_t nitems,
                         bool dev_tc = false, const ZeroFill &zero = {}) {
     const int S = p->c.subgrid_size;
-    const int32_t nslots = dev_tc ? p->tc.nslots : p->nslots;
+    // room for both forms' items: a host call after a device call does not move the buffer that a captured
+    // device call has the address of
+    const int32_t nslots = dev_tc ? std::max(p->tc.nslots, p->nslots) : p->nslots;
     CK(p->d_partials.ensure(sizeof(float2) * S * S * std::max<size_t>(1, nslots)));
     StageScope t(p, P9IDG_STAGE_GRIDDER);
     GridderArgs a = gridder_args(p);
@@ -1780,6 +1782,9 @@ p9idg_status p9idg_degrid_device(p9idg_plan *plan, const void *d_grid, void *d_v
 p9idg_status p9idg_wstack_image_device(p9idg_plan *plan, const void *d_layers, float *d_image, int32_t shift) {
     if (!plan || !d_layers || !d_image) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(ensure_device(plan));
+    // (the whole grid, of which the half plane below is a part: host calls on this plan need it all, and must not
+    // move it under a captured call)
+    CK(plan->d_grid64.ensure(sizeof(float2) * nn_of(plan)));
     StageScope t(plan, P9IDG_STAGE_LAYER_FFT);
     return layers_to_image(d_layers, false, plan->c.wlayer_count, plan->c.grid_size, plan->c.vis_count, shift != 0,
                            plan->fft, plan->fft_real, plan->d_grid64, d_image, plan->stream);
