@@ -71,6 +71,12 @@ enum {
 #define P9IDG_TC_MAX_W_TERM 0.01
 #define P9IDG_TC_MAX_W_TERM2 0.03
 
+/* The kernels a call runs (p9idg_plan_info.device_form). */
+enum {
+    P9IDG_FORM_SINCOS = 0,     /* one sincos per pixel and visibility */
+    P9IDG_FORM_TENSOR_CORE = 1
+};
+
 /* GriddingConstants (Core/ImageDomainGridder/GriddingConstants.cs:33-52).
  * scale_arcsec is the cell size in radians, stored as float like the
  * reference's ScaleArcSec.  WStepLambda is not a field: the reference never
@@ -114,7 +120,7 @@ typedef struct p9idg_plan_info {
     double tc_w_term;              /* max |dw| * max |r| of the plan's samples (vs P9IDG_TC_MAX_W_TERM);
                                       -1 until a tensor-core mode has been requested */
     int32_t tc_order;              /* tensor-core form the plan runs: 1 or 2; 0 when it runs FP32 */
-    int32_t reserved;
+    int32_t device_form;           /* kernels of the device (complex64) calls and batches: P9IDG_FORM_* */
 } p9idg_plan_info;
 
 /* ---------------- plans: Partitioner ---------------- */
@@ -142,6 +148,10 @@ p9idg_status p9idg_plan_set_mode(p9idg_plan *plan, int32_t mode);
  * second-order one; 2 = always the second-order form (smaller error, slower).  No counterpart in
  * the reference. */
 p9idg_status p9idg_plan_set_tc_order(p9idg_plan *plan, int32_t order);
+/* Device calls of the FP32 mode, and batches made afterwards: on the tensor cores where the plan
+ * allows it (tensor_cores 1, the default), or always on the sincos kernels (0), which keep no
+ * coefficients on the device. */
+p9idg_status p9idg_plan_set_fp32_tensor_cores(p9idg_plan *plan, int32_t tensor_cores);
 /* Subgrid taper float[S][S] applied by gridder and degridder (GriddingConstants.SubgridSpheroidal,
  * Gridder.cs:76,111); NULL restores the identity taper the reference uses. */
 p9idg_status p9idg_plan_set_taper(p9idg_plan *plan, const float *taper);

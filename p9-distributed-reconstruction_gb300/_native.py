@@ -50,13 +50,16 @@ class PlanInfo(ctypes.Structure):
                 ("gridded_visibilities", ctypes.c_int64), ("work_items", ctypes.c_int64),
                 ("nbl", ctypes.c_int32), ("nt", ctypes.c_int32), ("nch", ctypes.c_int32), ("mode", ctypes.c_int32),
                 ("requested_mode", ctypes.c_int32), ("tc_w_term", ctypes.c_double), ("tc_order", ctypes.c_int32),
-                ("reserved", ctypes.c_int32)]
+                ("device_form", ctypes.c_int32)]
 
 
 # Largest |dw r| of the tensor-core forms: first order (P9IDG_TC_MAX_W_TERM) and second order
 # (P9IDG_TC_MAX_W_TERM2)
 TC_MAX_W_TERM = 0.01
 TC_MAX_W_TERM2 = 0.03
+# kernels of a plan's device calls and batches: info()["device_form"]
+FORM_SINCOS = 0
+FORM_TENSOR_CORE = 1
 
 
 # name -> (restype, argtypes); every symbol include/p9idg.h declares
@@ -70,6 +73,7 @@ SIGNATURES = {
     "p9idg_plan_get_info": (i32, [P, ctypes.POINTER(PlanInfo)]),
     "p9idg_plan_set_mode": (i32, [P, i32]),
     "p9idg_plan_set_tc_order": (i32, [P, i32]),
+    "p9idg_plan_set_fp32_tensor_cores": (i32, [P, i32]),
     "p9idg_plan_set_taper": (i32, [P, P]),
     "p9idg_plan_set_stream": (i32, [P, P]),
     "p9idg_plan_get_stream": (i32, [P, ctypes.POINTER(P)]),

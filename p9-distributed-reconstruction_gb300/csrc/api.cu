@@ -151,6 +151,7 @@ struct p9idg_plan {
     // hi + lo: see fp32_on_tensor_cores.  The host-array calls, whose results keep to the last bit and
     // which may pass a uvw of their own, run the sincos kernels.
     bool fp32_tc = false;
+    bool fp32_tc_wanted = true;  // p9idg_plan_set_fp32_tensor_cores
     int64_t wave_grid = 0, wave_degrid = 0;  // default tensor-core work-item sizes (0: not worked out yet)
     std::vector<double> freq, wn, uvw;
     std::vector<p9idg_subgrid> subs;
@@ -550,7 +551,7 @@ SubgridOpArgs subgrid_args(p9idg_plan *p) {
 bool use_tc(const p9idg_plan *p) { return p->mode != P9IDG_MODE_FP32; }
 // Whether a device call (complex64 arrays, the plan's uvw) of the FP32 mode runs on the tensor cores.
 bool use_fp32_tc(const p9idg_plan *p, bool device_call) {
-    return p->mode == P9IDG_MODE_FP32 && p->fp32_tc && device_call;
+    return p->mode == P9IDG_MODE_FP32 && p->fp32_tc && p->fp32_tc_wanted && device_call;
 }
 
 // Adder.Add throws "invalid grid" for subgrids outside [0, N-S) (Adder.cs:30-50).
@@ -1493,6 +1494,7 @@ p9idg_status p9idg_plan_get_info(const p9idg_plan *plan, p9idg_plan_info *out) {
     out->requested_mode = plan->requested_mode;
     out->tc_w_term = plan->tc_w_term;
     out->tc_order = plan->mode == P9IDG_MODE_FP32 ? 0 : tc_order_for(plan->tc_w_term, plan->tc.want_order);
+    out->device_form = use_tc(plan) || use_fp32_tc(plan, true) ? P9IDG_FORM_TENSOR_CORE : P9IDG_FORM_SINCOS;
     return P9IDG_OK;
 }
 
@@ -1533,6 +1535,12 @@ p9idg_status p9idg_plan_set_tc_order(p9idg_plan *plan, int32_t order) {
         CK(cudaStreamSynchronize(plan->stream));  // launches in flight use the previous form's limit
     }
     tc_set_order(plan->tc, plan->mode, order);
+    return P9IDG_OK;
+}
+
+p9idg_status p9idg_plan_set_fp32_tensor_cores(p9idg_plan *plan, int32_t tensor_cores) {
+    if (!plan) return fail(P9IDG_INVALID_ARGUMENT, "null plan");
+    plan->fp32_tc_wanted = tensor_cores != 0;
     return P9IDG_OK;
 }
 

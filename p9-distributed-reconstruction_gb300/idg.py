@@ -182,6 +182,11 @@ class Plan:
         """Tensor-core form: 0 = automatic (first order where its bound holds), 2 = second order."""
         _check(nat.lib().p9idg_plan_set_tc_order(self.handle, int(order)))
 
+    def set_fp32_tensor_cores(self, on: bool):
+        """Device calls of the FP32 mode, and batches made afterwards: on the tensor cores where the plan
+        allows it (True, the default; ``info()["device_form"]`` says which), or on the sincos kernels."""
+        _check(nat.lib().p9idg_plan_set_fp32_tensor_cores(self.handle, int(bool(on))))
+
     def set_taper(self, taper):
         t = None if taper is None else np.ascontiguousarray(taper, np.float32)
         _check(nat.lib().p9idg_plan_set_taper(self.handle, _ptr(t)))
