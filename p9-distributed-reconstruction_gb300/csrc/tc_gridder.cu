@@ -42,13 +42,17 @@
 // operand is made, and T1 is weighted by dw - dw0, which is an order smaller than dw (channels
 // and a short track).  FP16 hi + lo holds 22 bits, so what is left is the two phases' FP32
 // rounding and the hardware sincos, as in the sincos kernel: against FP64 6e-7 where that has
-// 8.5e-7 (2047^2, S = 24), and at most its error in every shape tested.  kFp32MaxDev: with
+// 8.5e-7 (2047^2, S = 24).  kFp32MaxDev: with
 // |dw - dw0| |r| <= 8e-4 the second-order term left out (3e-7 at most, 4e-8 rms over a subgrid's
 // samples and pixels) and the 11 bits of the first-order rows stay below that.
 // 8.0 M visibilities, S = 24: sincos kernel 2.04 ms (bound by the SFUs at 576 sincos per
 // visibility), this form 0.41 ms (48 useful of 64 sincos).  The gridder (EX) rotates its sums by
 // exp(i dw0 r) at the end and moves them out of the tensor core's accumulator every stage: 16.0 M
-// visibilities, S = 32, sincos kernel 6.75 ms, this form 1.05 ms, error 3.1e-7 -> 2.4e-7.
+// visibilities, S = 32, sincos kernel 6.75 ms, this form 1.09 ms, error 3.0e-7 -> 2.5e-7 (mean of 20
+// skies).  Errors of both forms, of single calls, over 30 shapes of 261^2 to 2968^2 with four skies each:
+// degridding always below the sincos kernels, gridding below or, where the adder's atomics in a few
+// bright pixels make most of it, equal; the same within 2 % of the limit below and for noise, equal
+// visibilities, one in 64 and outliers of 10^4.
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -276,6 +280,8 @@ __host__ __device__ constexpr uint32_t g_smem(bool o2) {
 }
 constexpr uint32_t kGTmemCols = 256;  // the 192 (256) columns of the y rows
 
+constexpr float kStageExcess = 5.9604644775390625e-8f;  // 2^-24: see stage_gain
+
 // The gridder epilogue's last step for the 4 pixels a producer thread finishes: P = P0 + i r P1
 // (- (r^2 / 2) P2) from the planes E, times the taper, into the work item's partial subgrid
 // (fftshifted as Gridder.Forward writes it).  Rows and columns past the plan's S are padding:
@@ -295,6 +301,7 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
     }
     float2 *out = a.partials + static_cast<int64_t>(slot) * S * S;
     const float i0 = 1.f / sv, i1 = i0 / sw, i2 = 0.5f * i1 / sw;  // exact: powers of two
+    const float i0x = i0 * (1.f - kStageExcess);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int p = threadIdx.x + k * kGProducerWarps * 32;
@@ -304,12 +311,14 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
         auto pl = [&](int kind, int t, int u) {
             return E[(kind * 8 + 2 * t + u) * 1056 + e] + E[(kind * 8 + 4 + 2 * t + u) * 1056 + e];
         };
-        const float p0re = (pl(0, 0, 0) - pl(0, 1, 1)) * i0;
-        const float p0im = (pl(0, 0, 1) + pl(0, 1, 0)) * i0;
+        const float p0re = pl(0, 0, 0) - pl(0, 1, 1);
+        const float p0im = pl(0, 0, 1) + pl(0, 1, 0);
         const float p1re = (pl(1, 0, 0) - pl(1, 1, 1)) * i1;
         const float p1im = (pl(1, 0, 1) + pl(1, 1, 0)) * i1;
         const float rr = ep_r[k], tap = ep_t[k];
-        float re = fmaf(-rr, p1im, p0re), im = fmaf(rr, p1re, p0im);
+        // (EX: one rounding for the scaled sum and the first-order term, so that half a unit is not rounded away)
+        float re = EX ? fmaf(p0re, i0x, -(rr * p1im)) : fmaf(-rr, p1im, p0re * i0);
+        float im = EX ? fmaf(p0im, i0x, rr * p1re) : fmaf(rr, p1re, p0im * i0);
         if (O2) {  // - (r^2 / 2) P2
             const float h2 = rr * rr * i2;
             re = fmaf(-h2, pl(2, 0, 0) - pl(2, 1, 1), re);
@@ -326,13 +335,26 @@ __device__ __forceinline__ void gridder_finish(const TcArgs &a, const float *E, 
     }
 }
 
-// EX: what an accumulator of `valid` visibilities (at most a stage) is multiplied by.  Truncation toward zero
-// leaves it short by about 7e-8 of itself per K step of 16 (measured over 3072^2 to 287^2 grids, point
-// sources in noise: 2.4e-7 to 3.3e-7 after 4 steps, where the sincos kernel's sums are short by
-// 0.4e-7 to 1.4e-7), which 1 + 2^-22 undoes to within 1e-7.
+// EX: what an accumulator of `valid` visibilities (at most a stage) is multiplied by.  The tensor core rounds
+// toward zero: if each K step of 16 takes up to one unit in the last place (2^-23) off the sum so far, one
+// that grows evenly over four steps ends up between 0 and 2.5 units short (measured with an exact sincos,
+// point sources in noise: 1.0 to 1.8 units).  1.5 units are put back: 2 here, less half a unit of the whole
+// sum at the end (kStageExcess), as no float lies between; a sum that truncation did not shorten comes out
+// 1.8e-7 too large.
 __device__ __forceinline__ float stage_gain(int valid) {
-    const int steps = (valid + 15) >> 4;
-    return steps >= 3 ? 1.f + 2.384185791015625e-7f : steps == 2 ? 1.f + 1.1920928955078125e-7f : 1.f;
+    return valid > 32 ? 1.f + 2.384185791015625e-7f : 1.f + 1.1920928955078125e-7f;
+}
+
+// EX: a phase less the nearest multiple of 2 pi, in two steps (Cody and Waite): 2 pi as a float, then what
+// that float is too large by.  The hardware sincos's error grows with its argument, and here two of them
+// multiply in every pixel where the sincos kernel has one: without this step visibilities of which one in
+// 64 is not zero came out no better than there (3.8e-7 against FP64; 1024^2, S = 24), with it at 2.5e-7,
+// and noise at 4.2e-7 (7.5e-7 without it, sincos kernel 11e-7).  It takes 4 % of the kernel's time.
+__device__ __forceinline__ float2 within_turn(float2 p) {
+    const float2 inv = make_float2(0.15915494f, 0.15915494f), big = make_float2(12582912.f, 12582912.f);
+    const float2 hi = make_float2(-6.2831855f, -6.2831855f), lo = make_float2(1.7484556e-7f, 1.7484556e-7f);
+    const float2 n = __fadd2_rn(__ffma2_rn(p, inv, big), make_float2(-big.x, -big.y));  // rounded to a whole number
+    return __ffma2_rn(n, lo, __ffma2_rn(n, hi, p));
 }
 
 // O2: the second-order form (|dw r| up to P9IDG_TC_MAX_W_TERM2): y rows 192-255 carry
@@ -582,7 +604,11 @@ __global__ void __launch_bounds__(kGThreads, 2)
             for (int pr = 0; pr < 4; pr++) {
                 // the two rows of a pair side by side in packed FP32x2 arithmetic
                 const float2 zg = __fmul2_rn(cz2, gt[pr]);
-                const float2 pb = __ffma2_rn(cy2, mt[pr], zg), pa = __ffma2_rn(cx2, mt[pr], zg);
+                float2 pb = __ffma2_rn(cy2, mt[pr], zg), pa = __ffma2_rn(cx2, mt[pr], zg);
+                if (EX) {
+                    pb = within_turn(pb);
+                    pa = within_turn(pa);
+                }
                 float2 cb, sb, ca, sa;
                 __sincosf(pb.x, &sb.x, &cb.x);  // B_k(y)
                 __sincosf(pb.y, &sb.y, &cb.y);
