@@ -149,8 +149,10 @@ p9idg_status p9idg_plan_set_mode(p9idg_plan *plan, int32_t mode);
  * the reference. */
 p9idg_status p9idg_plan_set_tc_order(p9idg_plan *plan, int32_t order);
 /* Device calls of the FP32 mode, and batches made afterwards: on the tensor cores where the plan
- * allows it (tensor_cores 1, the default), or always on the sincos kernels (0), which keep no
- * coefficients on the device. */
+ * allows it (tensor_cores 1, the default), or always on the sincos kernels (0).  The tensor cores
+ * need 16 bytes of device memory a gridded visibility for as long as the plan lives; a plan that
+ * finds none goes over to the sincos kernels, which need none (device_form says so), until 1 is set
+ * again. */
 p9idg_status p9idg_plan_set_fp32_tensor_cores(p9idg_plan *plan, int32_t tensor_cores);
 /* Subgrid taper float[S][S] applied by gridder and degridder (GriddingConstants.SubgridSpheroidal,
  * Gridder.cs:76,111); NULL restores the identity taper the reference uses. */

@@ -126,7 +126,9 @@ cudaError_t p9idg::device_alloc(void **p, size_t bytes) {
         }
         if (g_alloc_budget.compare_exchange_weak(b, b - 1)) break;
     }
-    return cudaMalloc(p, bytes);
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here: a later launch's check must not find it
+    return e;
 }
 
 extern "C" p9idg_status p9idg_debug_tc_wait(int64_t wait_ns, int32_t skip_stage) {
@@ -537,6 +539,24 @@ p9idg_status ensure_tc(p9idg_plan *p) {
     return P9IDG_OK;
 }
 
+bool use_tc(const p9idg_plan *p) { return p->mode != P9IDG_MODE_FP32; }
+// Whether a device call (complex64 arrays, the plan's uvw) of the FP32 mode runs on the tensor cores.
+bool use_fp32_tc(const p9idg_plan *p, bool device_call) {
+    return p->mode == P9IDG_MODE_FP32 && p->fp32_tc && p->fp32_tc_wanted && device_call;
+}
+
+// Whether a call (or a batch's problem) runs on the tensor cores, with their state made ready.  Where there is
+// no memory for that state, 16 bytes a visibility, the FP32 mode's device calls run the sincos kernels, which
+// need none: from then on, so that a plan does not change its form from call to call.
+p9idg_status call_form(p9idg_plan *p, bool device_call, bool &tc) {
+    tc = use_tc(p) || use_fp32_tc(p, device_call);
+    if (!tc) return P9IDG_OK;
+    const p9idg_status st = ensure_tc(p);
+    if (st != P9IDG_OUT_OF_MEMORY || use_tc(p)) return st;
+    p->fp32_tc_wanted = tc = false;
+    return P9IDG_OK;
+}
+
 SubgridOpArgs subgrid_args(p9idg_plan *p) {
     SubgridOpArgs a{};
     a.g = p->geom();
@@ -546,12 +566,6 @@ SubgridOpArgs subgrid_args(p9idg_plan *p) {
     a.twiddles = p->d_phasor.as<float2>() + static_cast<size_t>(p->c.subgrid_size) * p->c.subgrid_size;
     a.status = p->d_status.as<int32_t>();
     return a;
-}
-
-bool use_tc(const p9idg_plan *p) { return p->mode != P9IDG_MODE_FP32; }
-// Whether a device call (complex64 arrays, the plan's uvw) of the FP32 mode runs on the tensor cores.
-bool use_fp32_tc(const p9idg_plan *p, bool device_call) {
-    return p->mode == P9IDG_MODE_FP32 && p->fp32_tc && p->fp32_tc_wanted && device_call;
 }
 
 // Adder.Add throws "invalid grid" for subgrids outside [0, N-S) (Adder.cs:30-50).
@@ -675,11 +689,11 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
 p9idg_status run_grid(p9idg_plan *p, const void *d_vis, bool vis_c128, float2 *d_layers, bool wstack,
                       bool device_call = false) {
     const int nl = wstack ? p->c.wlayer_count : 1;
-    const bool dev_tc = device_call && (use_tc(p) || use_fp32_tc(p, true));
+    bool dev_tc = false;
+    if (device_call) TRY(call_form(p, true, dev_tc));
     const WorkItem *items = p->d_gitems.as<WorkItem>();
     int32_t nitems = static_cast<int32_t>(p->gitems.size());
     if (dev_tc) {
-        TRY(ensure_tc(p));
         items = static_cast<const WorkItem *>(p->tc.gitems);
         nitems = p->tc.ngitems;
     }
@@ -714,8 +728,8 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
     CK(p->d_subgrids.ensure(sizeof(float2) * S * S * std::max<size_t>(1, p->dsub.size())));
     TRY(ensure_gaps(p));
     const int64_t ngaps = static_cast<int64_t>(p->gaps.size() / 2);
-    const bool tc = use_tc(p) || use_fp32_tc(p, !out_c128);
-    if (tc) TRY(ensure_tc(p));
+    bool tc;
+    TRY(call_form(p, !out_c128, tc));
     const bool fused = tc && !out_c128 && (ngaps == 0 || zero_in_kernel(p->gap_words, p->tc.nditems));
     ZeroSide z{p};
     if (!out_in_host && !fused) TRY(z.fork());
@@ -1928,8 +1942,9 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     for (int i = 0; i < nplans; i++) {
         p9idg_plan *p = plans[i];
         const int S = p->c.subgrid_size;
-        const bool tc = batch_tc(p), fp32 = p->mode == P9IDG_MODE_FP32;
-        if (tc && (st = ensure_tc(p)) != P9IDG_OK) return bail(st);
+        const bool fp32 = p->mode == P9IDG_MODE_FP32;
+        bool tc;
+        if ((st = call_form(p, true, tc)) != P9IDG_OK) return bail(st);
         // the whole batch shares the GPU, so its tensor-core items are full-sized however small a plan is
         std::vector<DevSubgrid> gslots, dslots;
         std::vector<WorkItem> gwork, dwork;

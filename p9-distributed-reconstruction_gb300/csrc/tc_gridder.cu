@@ -1716,7 +1716,9 @@ void tc_release(TcPlanState &st) {
     if (st.coef) cudaFree(st.coef);
     if (st.block) cudaFree(st.block);
     if (st.item_block) cudaFree(st.item_block);
+    const int want_order = st.want_order;  // what the program asked for stays
     st = TcPlanState();
+    st.want_order = want_order;
 }
 
 p9idg_status tc_selftest(int mode, int N, double *max_rel_err, std::string &err) {
