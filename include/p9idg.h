@@ -210,7 +210,8 @@ p9idg_status p9idg_fft_shift(void *array, int32_t n, int32_t elem_bytes);
 
 /* ---------------- device-resident interface (HBM buffers, complex64 = float2) ---------------- */
 /* These run asynchronously on the plan's stream; p9idg_synchronize waits and
- * reports kernel-side check failures of the calls since the last report.  uvw and frequencies are the
+ * reports kernel-side check failures of the device calls since the last report (a host call reports its
+ * own, a batch its problems' by p9idg_batch_synchronize).  uvw and frequencies are the
  * plan's.  An output is zeroed by the tensor-core kernels themselves or on a second stream of the plan,
  * forked from the plan's stream and joined back into it within the call, so all of a call's work is
  * ordered on the plan's stream. */

@@ -173,6 +173,7 @@ struct p9idg_plan {
     int device = -1;
     cudaStream_t own_stream = nullptr, stream = nullptr;
     bool uvw_uploaded = false;
+    bool host_call = false;  // the call in progress is a host call (its status word)
     DevBuf d_uvw, d_wn, d_sub, d_gitems, d_ditems, d_lmn, d_taper, d_phasor, d_status;
     DevBuf d_partials, d_subgrids, d_vis_in, d_vis_out, d_layers, d_out128, d_grid128, d_grid128b, d_grid64,
         d_flags, d_image;
@@ -384,13 +385,13 @@ p9idg_status ensure_device(p9idg_plan *p) {
     CK(p->d_lmn.ensure(sizeof(float) * p->lmn.size()));
     CK(p->d_taper.ensure(sizeof(float) * S * S));
     CK(p->d_phasor.ensure(sizeof(float) * p->add_phasor.size()));
-    CK(p->d_status.ensure(sizeof(int32_t)));
+    CK(p->d_status.ensure(2 * sizeof(int32_t)));
     cudaStream_t st = p->stream;
     CK(cudaMemcpyAsync(p->d_wn.p, p->wn.data(), sizeof(double) * p->nch, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(p->d_lmn.p, p->lmn.data(), sizeof(float) * p->lmn.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(p->d_phasor.p, p->add_phasor.data(), sizeof(float) * p->add_phasor.size(),
                        cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), st));
+    CK(cudaMemsetAsync(p->d_status.p, 0, 2 * sizeof(int32_t), st));
     CK(cudaStreamSynchronize(st));
     p->taper_dirty = true;
     p->dev_ready = true;
@@ -447,11 +448,13 @@ p9idg_status upload_items(p9idg_plan *p) {
     return P9IDG_OK;
 }
 
+int32_t *status_word(const p9idg_plan *p, bool host_call) { return p->d_status.as<int32_t>() + (host_call ? 1 : 0); }
+
 // Device state for a call, without the uvw upload (in-place host calls start their transfers in
-// the other direction first and upload uvw beside them).  Device calls (reset_status false) leave the
-// status word to the call that reads it: one launch less, and a check that trips is reported by the
-// next synchronisation whatever was queued after it.
-p9idg_status prepare_state(p9idg_plan *p, bool reset_status = true) {
+// the other direction first and upload uvw beside them).  Device and host calls have a status word each.
+// Device calls leave theirs to p9idg_synchronize: one launch less, and a check that trips is reported by the
+// next synchronisation whatever was queued after it.  A host call clears and reports its own.
+p9idg_status prepare_state(p9idg_plan *p, bool host_call = true) {
     TRY(ensure_device(p));
     if (p->items_dirty) TRY(upload_items(p));
     if (p->taper_dirty) {
@@ -459,28 +462,40 @@ p9idg_status prepare_state(p9idg_plan *p, bool reset_status = true) {
                            p->stream));
         p->taper_dirty = false;
     }
-    if (reset_status) CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), p->stream));
+    p->host_call = host_call;
+    if (host_call) CK(cudaMemsetAsync(status_word(p, true), 0, sizeof(int32_t), p->stream));
     return P9IDG_OK;
 }
 
-// uvw null: a device call, on the plan's uvw
+// A device call, on the plan's uvw
+p9idg_status prepare_device(p9idg_plan *p) {
+    TRY(prepare_state(p, false));
+    return upload_uvw(p, nullptr);
+}
+
+// A host call (uvw null: the plan's)
 p9idg_status prepare(p9idg_plan *p, const double *uvw) {
-    TRY(prepare_state(p, uvw != nullptr));
+    TRY(prepare_state(p));
     return upload_uvw(p, uvw);
 }
 
-p9idg_status finish_call(p9idg_plan *p) {
-    int32_t status = 0;
-    CK(cudaMemcpyAsync(&status, p->d_status.p, sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream));
-    CK(cudaStreamSynchronize(p->stream));
-    if (status != 0) CK(cudaMemsetAsync(p->d_status.p, 0, sizeof(int32_t), p->stream));
-    if (p->timing) collect_timing(p);
+p9idg_status status_error(int32_t status) {
     if (status == kStatusWTerm)
         return fail(P9IDG_UNSUPPORTED, "this call's uvw puts |dw r| above the bound of the plan's tensor-core "
                                        "form: use P9IDG_MODE_FP32 or a plan made from this uvw");
     if (status != 0)
         return fail(P9IDG_DEVICE_CHECK_FAILED, "a kernel bounds check tripped (status " + std::to_string(status) + ")");
     return P9IDG_OK;
+}
+
+// Waits for the plan's stream; reports what the host call tripped, or the device calls since the last report.
+p9idg_status finish_call(p9idg_plan *p, bool host_call = true) {
+    int32_t status = 0;
+    CK(cudaMemcpyAsync(&status, status_word(p, host_call), sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream));
+    CK(cudaStreamSynchronize(p->stream));
+    if (status != 0) CK(cudaMemsetAsync(status_word(p, host_call), 0, sizeof(int32_t), p->stream));
+    if (p->timing) collect_timing(p);
+    return status_error(status);
 }
 
 GridderArgs gridder_args(p9idg_plan *p) {
@@ -492,7 +507,7 @@ GridderArgs gridder_args(p9idg_plan *p) {
     a.lmn = p->d_lmn.as<float>();
     a.taper = p->d_taper.as<float>();
     a.nsub = static_cast<int32_t>(p->dsub.size());
-    a.status = p->d_status.as<int32_t>();
+    a.status = status_word(p, p->host_call);
     return a;
 }
 
@@ -564,7 +579,7 @@ SubgridOpArgs subgrid_args(p9idg_plan *p) {
     a.nsub = static_cast<int32_t>(p->dsub.size());
     a.add_phasor = p->d_phasor.as<float2>();
     a.twiddles = p->d_phasor.as<float2>() + static_cast<size_t>(p->c.subgrid_size) * p->c.subgrid_size;
-    a.status = p->d_status.as<int32_t>();
+    a.status = status_word(p, p->host_call);
     return a;
 }
 
@@ -1246,6 +1261,7 @@ struct p9idg_batch {
     cudaStream_t stream = nullptr;
     DevBuf d_gargs, d_dargs, d_aargs, d_sargs, d_tg, d_td;  // per-problem argument tables
     DevBuf d_gitems, d_ditems, d_subs, d_partials, d_refs, d_done_init, d_done, d_finish, d_start;
+    DevBuf d_status;  // a status word for each problem
     int32_t ngitems = 0, nditems = 0, nrefs = 0;
     std::vector<WorkItem> h_gitems, h_ditems;  // merged work items of all problems, in launch order
     // problems may mix subgrid sizes, and FP32 ones the two forms of that mode: the items and subgrid
@@ -1419,7 +1435,7 @@ void batch_release(p9idg_batch *b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     DevBuf *bufs[] = {&b->d_gargs, &b->d_dargs,  &b->d_aargs,    &b->d_sargs, &b->d_tg,        &b->d_td,   &b->d_gitems, &b->d_zgrid,
                       &b->d_zvis,  &b->d_ditems, &b->d_partials, &b->d_subs,  &b->d_refs,      &b->d_done_init, &b->d_done,
-                      &b->d_finish, &b->d_start};
+                      &b->d_finish, &b->d_start, &b->d_status};
     for (DevBuf *x : bufs) x->release();
     if (b->stream) cudaStreamDestroy(b->stream);
 }
@@ -1778,26 +1794,26 @@ p9idg_status p9idg_fft_shift(void *array, int32_t n, int32_t elem_bytes) {
 p9idg_status p9idg_grid_w_device(p9idg_plan *plan, const void *d_vis, void *d_layers) {
     if (!plan || !d_vis || !d_layers) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(check_wstack_layers(plan));
-    TRY(prepare(plan, nullptr));
+    TRY(prepare_device(plan));
     return run_grid(plan, d_vis, false, static_cast<float2 *>(d_layers), true, true);
 }
 
 p9idg_status p9idg_degrid_w_device(p9idg_plan *plan, const void *d_grid, void *d_vis) {
     if (!plan || !d_grid || !d_vis) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
-    TRY(prepare(plan, nullptr));
+    TRY(prepare_device(plan));
     return run_degrid(plan, static_cast<const float2 *>(d_grid), false, d_vis, false, true);
 }
 
 p9idg_status p9idg_grid_device(p9idg_plan *plan, const void *d_vis, void *d_grid) {
     if (!plan || !d_vis || !d_grid) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
     TRY(check_adder_range(plan));
-    TRY(prepare(plan, nullptr));
+    TRY(prepare_device(plan));
     return run_grid(plan, d_vis, false, static_cast<float2 *>(d_grid), false, true);
 }
 
 p9idg_status p9idg_degrid_device(p9idg_plan *plan, const void *d_grid, void *d_vis) {
     if (!plan || !d_grid || !d_vis) return fail(P9IDG_INVALID_ARGUMENT, "null argument");
-    TRY(prepare(plan, nullptr));
+    TRY(prepare_device(plan));
     return run_degrid(plan, static_cast<const float2 *>(d_grid), false, d_vis, false, false);
 }
 
@@ -1816,7 +1832,7 @@ p9idg_status p9idg_synchronize(p9idg_plan *plan) {
     if (!plan) return fail(P9IDG_INVALID_ARGUMENT, "null plan");
     if (!plan->dev_ready) return P9IDG_OK;
     CK(cudaSetDevice(plan->device));
-    return finish_call(plan);
+    return finish_call(plan, false);
 }
 
 // ---- timing ----
@@ -1926,7 +1942,7 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
     for (int i = 0; i < nplans; i++) {
         p9idg_plan *p = plans[i];
         if ((st = check_wstack_layers(p)) != P9IDG_OK) return bail(st);
-        if ((st = prepare(p, nullptr)) != P9IDG_OK) return bail(st);
+        if ((st = prepare_device(p)) != P9IDG_OK) return bail(st);
         if (i == 0) b->device = p->device;
         if (p->device != b->device) return bail(fail(P9IDG_UNSUPPORTED, "a batch runs on one device"));
     }
@@ -1937,6 +1953,8 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
         if (e == cudaSuccess) e = b->d_done_init.ensure(sizeof(int32_t) * nplans);
         if (e == cudaSuccess) e = b->d_finish.ensure(sizeof(unsigned long long) * nplans);
         if (e == cudaSuccess) e = b->d_start.ensure(sizeof(unsigned long long));
+        if (e == cudaSuccess) e = b->d_status.ensure(sizeof(int32_t) * nplans);
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->d_status.p, 0, sizeof(int32_t) * nplans, b->stream);
         if (e != cudaSuccess) return bail(cuda_fail(e, "batch buffers"));
     }
     for (int i = 0; i < nplans; i++) {
@@ -1992,6 +2010,8 @@ p9idg_status p9idg_batch_create(p9idg_plan *const *plans, int32_t nplans, const 
             tc_fill_args(p->tc, ga[i], tg[i]);
             tc_fill_args(p->tc, da[i], td[i]);
         }
+        ga[i].status = da[i].status = aa[i].status = sa[i].status = tg[i].status = td[i].status =
+            b->d_status.as<int32_t>() + i;
         for (WorkItem w : gsrc) {
             w.problem = i;
             gitems.push_back(w);
@@ -2136,8 +2156,20 @@ p9idg_status p9idg_batch_capture_graph(p9idg_batch *b) {
 p9idg_status p9idg_batch_synchronize(p9idg_batch *b) {
     if (!b) return fail(P9IDG_INVALID_ARGUMENT, "null batch");
     CK(cudaSetDevice(b->device));
+    // every problem's word is read and cleared, so that none is left for a later report; the plans' own calls
+    // report to their plans
+    const size_t n = b->plans.size();
+    std::vector<int32_t> status(n, 0);
+    CK(cudaMemcpyAsync(status.data(), b->d_status.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    for (p9idg_plan *p : b->plans) TRY(finish_call(p));
+    CK(cudaMemsetAsync(b->d_status.p, 0, sizeof(int32_t) * n, b->stream));
+    for (p9idg_plan *p : b->plans) CK(cudaStreamSynchronize(p->stream));
+    for (size_t i = 0; i < n; i++)
+        if (status[i] != 0) {
+            const p9idg_status st = status_error(status[i]);
+            g_last_error = "problem " + std::to_string(i) + ": " + g_last_error;
+            return st;
+        }
     return P9IDG_OK;
 }
 
