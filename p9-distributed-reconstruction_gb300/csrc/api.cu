@@ -494,6 +494,10 @@ p9idg_status finish_call(p9idg_plan *p, bool host_call = true) {
     CK(cudaMemcpyAsync(&status, status_word(p, host_call), sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     if (status != 0) CK(cudaMemsetAsync(status_word(p, host_call), 0, sizeof(int32_t), p->stream));
+    if (status & kStatusWTerm) {  // the check is made as coefficients are: the same uvw again is checked again
+        p->tc.coef_valid = false;
+        p->tc.coef_recompute_flag = nullptr;
+    }
     if (p->timing) collect_timing(p);
     return status_error(status);
 }

@@ -88,3 +88,20 @@ def test_batch_reports_every_problem_once(need_gpu):
     plans[0].synchronize()
     _fails(plans[1].synchronize)
     batch.destroy()
+
+
+def test_refused_uvw_is_refused_again(need_gpu):
+    """A uvw beyond the tensor-core form's w bound is refused however often it is passed."""
+    from test_tc_w_term import wide_field
+
+    obs, uvw, c, d = wide_field(0.5 * pkg.TC_MAX_W_TERM)
+    part = pkg.Partitioner.CreatePartition(c, uvw, obs.frequencies)
+    assert part.plan.set_mode(pkg.MODE_TC_BF16X3) == pkg.MODE_TC_BF16X3
+    big = uvw.copy()
+    big[..., 2] *= 3.0
+    pkg.IDG.GridW(c, part, obs.vis, uvw, obs.frequencies)
+    for _ in range(3):
+        with pytest.raises(pkg.P9IDGError) as e:
+            pkg.IDG.GridW(c, part, obs.vis, big, obs.frequencies)
+        assert e.value.code == 8
+    pkg.IDG.GridW(c, part, obs.vis, uvw, obs.frequencies)
