@@ -1552,10 +1552,8 @@ p9idg_status p9idg_plan_set_mode(p9idg_plan *plan, int32_t mode) {
         }
     }
     const bool regroup = (plan->mode == P9IDG_MODE_FP32) != (mode == P9IDG_MODE_FP32);
-    if (plan->mode != mode) {  // the modes check a uvw differently: the next call recomputes its coefficients
-        plan->tc.coef_valid = false;
-        plan->tc.coef_recompute_flag = nullptr;
-    }
+    // (the coefficients stay: they do not depend on the mode, and those the FP32 mode makes are of the plan's own
+    // uvw, which a tensor-core mode has just been checked for)
     plan->mode = mode;
     if (regroup) build_gridder_items(plan);
     return P9IDG_OK;
