@@ -26,6 +26,8 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1037,14 +1039,24 @@ p9idg_status dev_sumsq(const float *d_img, int64_t count, Buf &partial, double *
 // factors are 2, 3, 5 and 7 (a size with a large prime factor costs several times as much).
 // 3072^2 with a 384^2 PSF: 5.26 -> 2.97 ms; 2.5 to 3.9 times faster at sizes with larger factors
 // (in place, with one buffer less: 3.03 ms).
+struct ConvSize {  // what the transforms of one size need
+    int my = 0, mx = 0;
+    Buf kernel, real, spec, work;  // half plane, padded image, its half plane, cuFFT's area
+    cufftHandle fwd = 0, inv = 0;
+    ~ConvSize() {
+        if (fwd) cufftDestroy(fwd);
+        if (inv) cufftDestroy(inv);
+    }
+};
+
 struct p9idg_convolver {
     int device = -1;
     cudaStream_t stream = nullptr, own = nullptr;
     int H = 0, W = 0, ky = 0, kx = 0;  // the padded size and the PSF's
-    int my = 0, mx = 0;                // the transforms' size (>= H x W)
-    int n_max = 0;                     // largest image that size serves
-    Buf kernel, real, spec, work, psf; // half plane, padded image, its half plane, cuFFT's area, PSF (correlations)
-    cufftHandle fwd = 0, inv = 0;
+    int n_max = 0;                     // largest image that `made` serves
+    std::unique_ptr<ConvSize> made;    // size >= H x W
+    std::unique_ptr<ConvSize> padded;  // correlations: H x W, once an image larger than n_max has been seen
+    Buf psf;                           // (correlations)
 };
 
 namespace {
@@ -1058,37 +1070,33 @@ int smooth_size(int n) {  // smallest even m >= n with no prime factor above 7
     }
 }
 
-p9idg_status conv_plans(p9idg_convolver *c, int my, int mx) {
-    for (cufftHandle *h : {&c->fwd, &c->inv}) {
-        if (*h) cufftDestroy(*h);
-        *h = 0;
-    }
-    c->my = my;
-    c->mx = mx;
+p9idg_status conv_plans(ConvSize *z, int my, int mx) {
+    z->my = my;
+    z->mx = mx;
     const size_t half = static_cast<size_t>(my) * (mx / 2 + 1);
-    CK(c->kernel.ensure(sizeof(double2) * half));
-    CK(c->spec.ensure(sizeof(double2) * half));
-    CK(c->real.ensure(sizeof(double) * static_cast<size_t>(my) * mx));
+    CK(z->kernel.ensure(sizeof(double2) * half));
+    CK(z->spec.ensure(sizeof(double2) * half));
+    CK(z->real.ensure(sizeof(double) * static_cast<size_t>(my) * mx));
     size_t need = 0, w = 0;  // the two transforms never run at once: one work area
     for (int k = 0; k < 2; k++) {
-        cufftHandle *h = k ? &c->inv : &c->fwd;
+        cufftHandle *h = k ? &z->inv : &z->fwd;
         CUFFT(cufftCreate(h));
         CUFFT(cufftSetAutoAllocation(*h, 0));
         CUFFT(cufftMakePlan2d(*h, my, mx, k ? CUFFT_Z2D : CUFFT_D2Z, &w));
         need = std::max(need, w);
     }
-    CK(c->work.ensure(need));
-    CUFFT(cufftSetWorkArea(c->fwd, c->work.p));
-    CUFFT(cufftSetWorkArea(c->inv, c->work.p));
+    CK(z->work.ensure(need));
+    CUFFT(cufftSetWorkArea(z->fwd, z->work.p));
+    CUFFT(cufftSetWorkArea(z->inv, z->work.p));
     return P9IDG_OK;
 }
 
 // What the unnormalised inverse of size my x mx is multiplied by: its own size, and the reference's
 // count over its Length, a 32-bit int (PaddedConvolver.cs:57).
-double conv_factor(const p9idg_convolver *c) {
+double conv_factor(const p9idg_convolver *c, const ConvSize *z) {
     const int64_t count = static_cast<int64_t>(c->H) * c->W;
     return static_cast<double>(count) / static_cast<double>(static_cast<int32_t>(count)) /
-           (static_cast<double>(c->my) * c->mx);
+           (static_cast<double>(z->my) * z->mx);
 }
 
 p9idg_status conv_init(p9idg_convolver *c, int H, int W, int ky, int kx) {
@@ -1104,23 +1112,27 @@ p9idg_status conv_init(p9idg_convolver *c, int H, int W, int ky, int kx) {
 
 void conv_release(p9idg_convolver *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (Buf *b : {&c->kernel, &c->real, &c->spec, &c->work, &c->psf}) b->release();
-    if (c->fwd) cufftDestroy(c->fwd);
-    if (c->inv) cufftDestroy(c->inv);
+    c->made.reset();
+    c->padded.reset();
+    c->psf.release();
     if (c->own) cudaStreamDestroy(c->own);
 }
 
-// The Fourier kernel of a correlation with c->psf for transforms of m x m.
-p9idg_status conv_correlation(p9idg_convolver *c, int m, int n) {
-    TRY(conv_plans(c, m, m));
+// The transforms of m x m for a correlation with c->psf, made for images of n x n, into `out` once they are
+// complete.
+p9idg_status conv_correlation(p9idg_convolver *c, int m, int n, std::unique_ptr<ConvSize> &out) {
+    std::unique_ptr<ConvSize> z(new (std::nothrow) ConvSize());
+    if (!z) return fail(P9IDG_OUT_OF_MEMORY, "convolver allocation");
+    TRY(conv_plans(z.get(), m, m));
     corr_real_kernel<<<grid_for(static_cast<int64_t>(m) * m), 256, 0, c->stream>>>(
-        c->psf.as<float>(), c->ky, c->kx, c->H, m, n / 2, n / 2, c->real.as<double>());
+        c->psf.as<float>(), c->ky, c->kx, c->H, m, n / 2, n / 2, z->real.as<double>());
     CK(cudaGetLastError());
-    CUFFT(cufftSetStream(c->fwd, c->stream));
-    CUFFT(cufftExecD2Z(c->fwd, c->real.as<double>(), reinterpret_cast<cufftDoubleComplex *>(c->kernel.p)));
+    CUFFT(cufftSetStream(z->fwd, c->stream));
+    CUFFT(cufftExecD2Z(z->fwd, z->real.as<double>(), reinterpret_cast<cufftDoubleComplex *>(z->kernel.p)));
     const int64_t half = static_cast<int64_t>(m) * (m / 2 + 1);
-    conv_scale_kernel<<<grid_for(half), 256, 0, c->stream>>>(c->kernel.as<double2>(), half, conv_factor(c));
+    conv_scale_kernel<<<grid_for(half), 256, 0, c->stream>>>(z->kernel.as<double2>(), half, conv_factor(c, z.get()));
     CK(cudaGetLastError());
+    out = std::move(z);
     return P9IDG_OK;
 }
 
@@ -1128,26 +1140,24 @@ p9idg_status conv_correlation(p9idg_convolver *c, int m, int n) {
 p9idg_status conv_run(p9idg_convolver *c, const float *d_img, int n, float *d_out) {
     if (n + c->ky / 2 > c->H || n + c->kx / 2 > c->W)
         return fail(P9IDG_INVALID_ARGUMENT, "image larger than the convolver's padded buffer");
-    if (n > c->n_max) {  // a larger image than the correlation was made for wraps at the padded size
-        CK(cudaStreamSynchronize(c->stream));
-        const int made_for = c->n_max;
-        TRY(conv_correlation(c, c->H, made_for));
-        c->n_max = c->H;
-    }
-    const int64_t half = static_cast<int64_t>(c->my) * (c->mx / 2 + 1);
+    // an image larger than the correlation was made for wraps at the padded size, which keeps transforms of its own
+    const bool larger = n > c->n_max;
+    if (larger && !c->padded) TRY(conv_correlation(c, c->H, c->n_max, c->padded));
+    const ConvSize *z = larger ? c->padded.get() : c->made.get();
+    const int64_t half = static_cast<int64_t>(z->my) * (z->mx / 2 + 1);
     const auto cols = [](int w) { return static_cast<unsigned>((w + 511) / 512); };
-    conv_pad_kernel<<<dim3(c->my, cols(c->mx)), 256, 0, c->stream>>>(d_img, n, c->mx, c->ky / 2, c->kx / 2,
-                                                                     c->real.as<double>());
+    conv_pad_kernel<<<dim3(z->my, cols(z->mx)), 256, 0, c->stream>>>(d_img, n, z->mx, c->ky / 2, c->kx / 2,
+                                                                     z->real.as<double>());
     CK(cudaGetLastError());
-    auto *s = reinterpret_cast<cufftDoubleComplex *>(c->spec.p);
-    CUFFT(cufftSetStream(c->fwd, c->stream));
-    CUFFT(cufftSetStream(c->inv, c->stream));
-    CUFFT(cufftExecD2Z(c->fwd, c->real.as<double>(), s));
+    auto *s = reinterpret_cast<cufftDoubleComplex *>(z->spec.p);
+    CUFFT(cufftSetStream(z->fwd, c->stream));
+    CUFFT(cufftSetStream(z->inv, c->stream));
+    CUFFT(cufftExecD2Z(z->fwd, z->real.as<double>(), s));
     conv_mul_kernel<<<static_cast<unsigned>((half + 511) / 512), 256, 0, c->stream>>>(
-        c->spec.as<double2>(), c->kernel.as<double2>(), half);
+        z->spec.as<double2>(), z->kernel.as<double2>(), half);
     CK(cudaGetLastError());
-    CUFFT(cufftExecZ2D(c->inv, s, c->real.as<double>()));
-    conv_crop_kernel<<<dim3(n, cols(n)), 256, 0, c->stream>>>(c->real.as<double>(), c->mx, c->ky / 2, c->kx / 2, n, d_out);
+    CUFFT(cufftExecZ2D(z->inv, s, z->real.as<double>()));
+    conv_crop_kernel<<<dim3(n, cols(n)), 256, 0, c->stream>>>(z->real.as<double>(), z->mx, c->ky / 2, c->kx / 2, n, d_out);
     CK(cudaGetLastError());
     return P9IDG_OK;
 }
@@ -1583,7 +1593,10 @@ p9idg_status p9idg_convolver_create(const double *kernel, int32_t h, int32_t w, 
     auto *c = new (std::nothrow) p9idg_convolver();
     if (!c) return fail(P9IDG_OUT_OF_MEMORY, "convolver allocation");
     p9idg_status st = conv_init(c, h, w, kernel_h, kernel_w);
-    if (st == P9IDG_OK) st = conv_plans(c, h, w);
+    if (st == P9IDG_OK) {
+        c->made.reset(new (std::nothrow) ConvSize());
+        st = c->made ? conv_plans(c->made.get(), h, w) : fail(P9IDG_OUT_OF_MEMORY, "convolver allocation");
+    }
     if (st == P9IDG_OK) {
         Buf full;
         const int64_t half = static_cast<int64_t>(h) * (w / 2 + 1);
@@ -1592,8 +1605,9 @@ p9idg_status p9idg_convolver_create(const double *kernel, int32_t h, int32_t w, 
             e = cudaMemcpyAsync(full.p, kernel, sizeof(double2) * static_cast<size_t>(h) * w, cudaMemcpyHostToDevice,
                                 c->stream);
         if (e == cudaSuccess) {
-            conv_kernel_half<<<grid_for(half), 256, 0, c->stream>>>(full.as<double2>(), h, w, conv_factor(c),
-                                                                    c->kernel.as<double2>());
+            conv_kernel_half<<<grid_for(half), 256, 0, c->stream>>>(full.as<double2>(), h, w,
+                                                                    conv_factor(c, c->made.get()),
+                                                                    c->made->kernel.as<double2>());
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1629,7 +1643,7 @@ p9idg_status p9idg_convolver_create_correlation(const float *psf, int32_t psf_h,
     // (tiny images keep the padded size: there the shifted PSF can reach the last row, which
     // FFT.Shift leaves in place)
     const int m = n >= 8 ? smooth_size(n + psf_h) : n + psf_h;
-    if (st == P9IDG_OK) st = conv_correlation(c, m, n);
+    if (st == P9IDG_OK) st = conv_correlation(c, m, n, c->made);
     if (st == P9IDG_OK) {
         c->n_max = m == c->H ? c->H : n;
         cudaError_t e = cudaStreamSynchronize(c->stream);
