@@ -223,17 +223,28 @@ __device__ __forceinline__ void cd_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
-// CTA scope: what st.async delivers is in shared memory when its bytes are counted.  Acquiring at cluster
-// scope empties L1 each time, and the tiles' pixels then come from L2 in every iteration.
-__device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase) {
+// The scope of the acquire holds the CTAs whose data is waited for: the cluster where st.async delivers it,
+// else the CTA alone.  The former empties L1, and the tiles' pixels then come from L2 in that iteration: 1000
+// iterations at 3072^2 take 4.68 ms, against 4.50 with CTA scope, which the memory model does not let stand for
+// it (16-byte packets that carry their iteration, in place of st.async, 4.67 and 3 % more without pairs).
+__device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase, bool from_peer) {
     long long t0 = 0;
     while (true) {
         uint32_t done;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(phase)
-            : "memory");
+        if (from_peer)
+            asm volatile(
+                "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                "selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(done)
+                : "r"(bar), "r"(phase)
+                : "memory");
+        else
+            asm volatile(
+                "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n"
+                "selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(done)
+                : "r"(bar), "r"(phase)
+                : "memory");
         if (done) return true;
         const long long t = clock64();
         if (t0 == 0) t0 = t;
@@ -439,9 +450,9 @@ __global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const unsigned long long
 // slots alternate between two sets: a slot is overwritten only after every cluster has posted the
 // iteration after it, hence read it.
 //
-// Measured for 1000 iterations at 3072^2 with a 768^2 window: 4.5 us an iteration, against 6.5 us for a
+// Measured for 1000 iterations at 3072^2 with a 768^2 window: 4.7 us an iteration, against 6.5 us for a
 // launch per iteration (graph replays with programmatic dependent launches, every CTA reducing all tile
-// keys).  Of the 4.5 us about 1.3 are the exchange and its two hops within a pair, 1.5 a warp's loads and
+// keys).  Of the 4.7 us about 1.3 are the exchange and its two hops within a pair, 1.5 a warp's loads and
 // evaluation, and the rest the wait for the slowest of 147 CTAs.
 //
 // A lane keeps in registers the candidate of its warp's rows of local tile `lane`; images of more than 32
@@ -531,7 +542,7 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
             }
         }
         if (rank == 0 && warp == 0) {
-            ok = __all_sync(0xffffffffu, cd_wait(in_b, phase));
+            ok = __all_sync(0xffffffffu, cd_wait(in_b, phase, pair));
             if (ok) {
                 uint4 *slots = P.slots + (c.iter & 1) * kCdSlots;
                 const unsigned epoch = static_cast<unsigned>(c.iter) + 1u;
@@ -573,7 +584,7 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
             }
         }
         settle();  // while the exchange is under way
-        ok = __all_sync(0xffffffffu, ok && cd_wait(sel_b, phase));
+        ok = __all_sync(0xffffffffu, ok && cd_wait(sel_b, phase, rank == 1));
         if (!ok) {
             c = CdCtl{c.iter, 1, 0, 2};
             if (lane == 0) P.report[1].error = 2;
