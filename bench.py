@@ -678,8 +678,12 @@ def main():
     plan = part.plan
     info = plan.info()
     headline = "tc_bf16x3" if args.mode == "auto" else args.mode
-    # config 3 times both split-precision forms beside the FP32 mode
-    compare = ["fp32", "tc_fp16x3"] if args.mode == "auto" else []
+    # config 3 times both split-precision forms beside the FP32 mode, and that in both of its forms
+    compare = ["fp32_sincos", "fp32", "tc_fp16x3"] if args.mode == "auto" else []
+
+    def select(mode):
+        plan.set_fp32_tensor_cores(mode != "fp32_sincos")
+        plan.set_mode(MODES["fp32" if mode == "fp32_sincos" else mode])
 
     stream = torch.cuda.Stream()
     plan.set_stream(stream.cuda_stream)
@@ -709,7 +713,8 @@ def main():
         assert int(tg.item()) == total_gridded, "the blocks' partitions must add up to the global one" 
     results = {}
     for mode in compare + [headline]:  # headline last: its clocks are sampled
-        ms, stages, clk = time_mode(plan, pkg, mode, step, stream, args.steps, args.warmup, ws,
+        select(mode)
+        ms, stages, clk = time_mode(plan, pkg, "fp32" if mode == "fp32_sincos" else mode, step, stream, args.steps, args.warmup, ws,
                                     clock_gpu=local if mode == headline else None)
         results[mode] = dict(ms=ms, stages=stages, clk=clk,
                              value=2 * total_gridded * args.steps / (ms * 1e-3) / 1e6)
@@ -719,12 +724,13 @@ def main():
     # visibilities themselves)
     launches = sum(n for (_, n) in stages.values()) - stages["h2d"][1] - stages["d2h"][1]
 
-    # split-precision vs FP32 mode on the whole workload: w layers, degridded visibilities, dirty image
-    tc_vs_fp32 = None
+    # split-precision vs FP32 mode, in its default form and on the sincos kernels, on the whole workload: w layers,
+    # degridded visibilities, dirty image
+    tc_vs_fp32 = tc_vs_sincos = None
     if compare:
         outs = {}
-        for mode in ("fp32", headline):
-            plan.set_mode(MODES[mode])
+        for mode in ("fp32", "fp32_sincos", headline):
+            select(mode)
             step()
             plan.wstack_image_device(d_layers.data_ptr(), d_img.data_ptr(), True)
             plan.synchronize()
@@ -733,11 +739,14 @@ def main():
         def rel_dev(a, b):
             return float(torch.linalg.vector_norm(a - b) / torch.linalg.vector_norm(b))
 
-        a, b = outs[headline], outs["fp32"]
-        tc_vs_fp32 = {"grid_w": rel_dev(a[0], b[0]), "degrid_w": rel_dev(a[1], b[1]),
-                      "dirty_image": rel_dev(a[2], b[2]), "visibilities": int(gridded)}
-        del outs, a, b
-        plan.set_mode(MODES[headline])
+        def versus(base):
+            a, b = outs[headline], outs[base]
+            return {"grid_w": rel_dev(a[0], b[0]), "degrid_w": rel_dev(a[1], b[1]),
+                    "dirty_image": rel_dev(a[2], b[2]), "visibilities": int(gridded)}
+
+        tc_vs_fp32, tc_vs_sincos = versus("fp32"), versus("fp32_sincos")
+        del outs
+        select(headline)
 
     # the full-grid w-layer FFT (FFT.WStackIFFTFloat + FFT.Shift), timed separately
     plan.reset_timing()
@@ -752,6 +761,19 @@ def main():
     peaks, peak_src = measured_peaks()
     kern = max(("gridder", "degridder"), key=lambda k: stages[k][0])
     kt_ms = stages[kern][0] / max(1, stages[kern][1])
+
+    def sincos_roofline(stages):
+        # one hardware sincos per pixel and visibility, divided by the measured sincos rate of the same intrinsic on
+        # this GPU (an ncu capture shows the probe and the sincos gridder at the same XU-pipe limit)
+        sincos_peak, _ = pkg.measure_sincos_peak()
+        rate = {k: gridded * S * S / (stages[k][0] / max(1, stages[k][1]) * 1e-3) / 1e9 for k in ("gridder", "degridder")}
+        k = max(rate, key=lambda k: stages[k][0])
+        return {"bound": "sfu", "achieved": rate[k], "peak": sincos_peak / 1e9, "unit": "Gsincos/s",
+                "frac": rate[k] / (sincos_peak / 1e9), "kernel": k + "_fp32",
+                "frac_per_kernel": {j: v / (sincos_peak / 1e9) for j, v in rate.items()},
+                "traffic": traffic_per_launch(k + "_fp32"),
+                "peak_source": "measured on this GPU: p9idg_measure_sincos_peak (independent chains of __sincosf)",
+                "work_per_launch": f"{gridded} visibilities x {S * S} pixels, one sincos each"}
 
     def tensor_roofline(kern, kt_ms, mode):
         achieved = gridded * 10 * S * S / (kt_ms * 1e-3) / 1e12
@@ -770,7 +792,8 @@ def main():
                         "kernels' work); the tensor-core kernels issue the physical MMA flop instead"
                         + (" (FP32 mode: FP16 hi+lo operands about each subgrid's own w)" if mode == "fp32" else "")}
 
-    roofline = tensor_roofline(kern, kt_ms, headline)
+    fp32_sincos = headline == "fp32" and info["device_form"] == pkg.FORM_SINCOS
+    roofline = sincos_roofline(stages) if fp32_sincos else tensor_roofline(kern, kt_ms, headline)
 
     # e2e through the reference-facing host API (IDG.GridW + IDG.DeGridW) with pinned host buffers
     e2e = None
@@ -878,7 +901,22 @@ def main():
             spart = pkg.Partition([[]], sp)
             lay_gpu = pkg.IDG.GridW(c, spart, obs.vis, obs.uvw, obs.frequencies)
             vis_gpu = pkg.IDG.DeGridW(c, spart, model_grid.copy(), obs.uvw, obs.frequencies)
-            acc[mode] = {"grid_w": rl(lay_gpu, layers_ref), "degrid_w": rl(vis_gpu, vis_ref)}
+            # (host calls: the FP32 mode's run the sincos kernels)
+            acc["fp32_sincos" if mode == "fp32" else mode] = {"grid_w": rl(lay_gpu, layers_ref),
+                                                              "degrid_w": rl(vis_gpu, vis_ref)}
+            if mode == "fp32":  # its device calls, in the form the plan runs
+                d_vis_s = torch.from_numpy(obs.vis.astype(np.complex64)).cuda()
+                d_grid_s = torch.from_numpy(model_grid.astype(np.complex64)).cuda()
+                d_lay_s = torch.empty((W, N, N), dtype=torch.complex64, device="cuda")
+                torch.cuda.synchronize()
+                form = "tensor cores" if sp.info()["device_form"] == pkg.FORM_TENSOR_CORE else "sincos"
+                sp.grid_w_device(d_vis_s.data_ptr(), d_lay_s.data_ptr())
+                sp.synchronize()
+                e = {"grid_w": rl(d_lay_s.cpu().numpy(), layers_ref)}
+                sp.degrid_w_device(d_grid_s.data_ptr(), d_vis_s.data_ptr())
+                sp.synchronize()
+                acc["fp32"] = dict(e, degrid_w=rl(d_vis_s.cpu().numpy(), vis_ref), form=form)
+                del d_vis_s, d_grid_s, d_lay_s
             sp.destroy()
         cpu = {"value": 2 * nv / t_cpu / 1e6, "unit": "Mvis/s", "cores": oracle.num_threads(), "kind": "port",
                "sample": f"{len(sample)} of {len(subs)} subgrids ({nv} of {gridded} gridded visibilities), "
@@ -892,7 +930,10 @@ def main():
         if "fp32" in results and headline != "fp32":
             st32 = results["fp32"]["stages"]
             k32 = max(("gridder", "degridder"), key=lambda k: st32[k][0])
-            modes["fp32"]["roofline"] = tensor_roofline(k32, st32[k32][0] / max(1, st32[k32][1]), "fp32")
+            if info["device_form"] == pkg.FORM_TENSOR_CORE:
+                modes["fp32"]["roofline"] = tensor_roofline(k32, st32[k32][0] / max(1, st32[k32][1]), "fp32")
+            modes["fp32"]["form"] = "tensor cores" if info["device_form"] == pkg.FORM_TENSOR_CORE else "sincos"
+            modes["fp32_sincos"]["roofline"] = sincos_roofline(results["fp32_sincos"]["stages"])
         out = {"metric": METRIC, "value": head["value"], "unit": "Mvis/s", "n_gpus": ws, "steps": args.steps,
                "warmup": max(3, args.warmup), "ms_per_step": head["ms"] / args.steps, "higher_is_better": True,
                "scaling": "strong", "vs_baseline": None, "dtype": "f32" if headline == "fp32" else headline,
@@ -913,6 +954,7 @@ def main():
                "tc_over_fp32": (head["value"] / results["fp32"]["value"]) if "fp32" in results and
                headline != "fp32" else None,
                "rel_l2_tc_vs_fp32_full_workload": tc_vs_fp32,
+               "rel_l2_tc_vs_fp32_sincos_full_workload": tc_vs_sincos,
                "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": int(launches),
                "clocks": head["clk"]}
         print(json.dumps(out), flush=True)
