@@ -779,9 +779,8 @@ template <bool BF16, typename OutT, bool BATCH, bool TMA, bool O2>
 __global__ void __launch_bounds__(kDThreads, 2)
     tc_degridder_kernel(const TcArgs L, const TcArgs *__restrict__ probs, const __grid_constant__ TmaMaps maps) {
     constexpr int NB = O2 ? 1 : 2;  // accumulator buffers
-    // FP16 operands with complex64 outputs expand about the subgrid's centre dw0; complex128 outputs (the
-    // host-array calls, whose results keep to the last bit) and BF16 (whose device and host calls agree
-    // to rounding) about dw = 0
+    // FP16 operands with complex64 outputs, which also serve the FP32 mode, expand about the subgrid's centre
+    // dw0; complex128 outputs (host-array calls, in the FP16 mode only) and BF16 about dw = 0
     constexpr bool kCentred = !BF16 && sizeof(OutT) == 8;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_1k(smem_raw);
@@ -1378,8 +1377,16 @@ struct Packed {
         if (src && bytes) std::memcpy(host.data() + at, src, bytes);
         return at;
     }
-    cudaError_t upload(void **block, cudaStream_t stream) const {
-        cudaError_t e = device_alloc(block, host.size());
+    // *block, of *room bytes, stays where it is if that is enough
+    cudaError_t upload(void **block, size_t *room, cudaStream_t stream) const {
+        cudaError_t e = cudaSuccess;
+        if (!*block || *room < host.size()) {
+            if (*block) cudaFree(*block);
+            *block = nullptr;
+            *room = 0;
+            e = device_alloc(block, host.size());
+            if (e == cudaSuccess) *room = host.size();
+        }
         return e == cudaSuccess ? cudaMemcpyAsync(*block, host.data(), host.size(), cudaMemcpyHostToDevice, stream) : e;
     }
 };
@@ -1390,12 +1397,10 @@ struct Packed {
 static p9idg_status tc_items(TcPlanState &st, const std::vector<p9idg_subgrid> &subs, int nch, cudaStream_t stream,
                              std::string &err) {
     if (st.items_degrid == st.degrid_chunk && st.items_grid == st.grid_chunk) return P9IDG_OK;
-    cudaError_t e = cudaSuccess;
-    if (st.item_block) {
-        e = cudaStreamSynchronize(stream);  // launches in flight read the lists replaced here
-        cudaFree(st.item_block);
-    }
-    st.item_block = st.ditems = st.gitems = st.gsubs = nullptr;
+    // launches in flight read the lists replaced here; their memory stays, so that sizes which come back (a change
+    // of mode and back) find their lists where a captured call looks for them
+    cudaError_t e = st.item_block ? cudaStreamSynchronize(stream) : cudaSuccess;
+    st.ditems = st.gitems = st.gsubs = nullptr;
     st.items_degrid = st.items_grid = -1;
     std::vector<DevSubgrid> dtmp, gsubs;
     std::vector<WorkItem> ditems, gitems;
@@ -1403,7 +1408,7 @@ static p9idg_status tc_items(TcPlanState &st, const std::vector<p9idg_subgrid> &
     build_work_items(subs, nch, st.grid_chunk, gsubs, gitems);
     Packed p;
     const size_t at_d = p.put(ditems), at_g = p.put(gitems), at_s = p.put(gsubs);
-    if (e == cudaSuccess) e = p.upload(&st.item_block, stream);
+    if (e == cudaSuccess) e = p.upload(&st.item_block, &st.item_room, stream);
     const cudaError_t es = cudaStreamSynchronize(stream);
     if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) {
@@ -1454,7 +1459,7 @@ p9idg_status tc_prepare(TcPlanState &st, const std::vector<p9idg_subgrid> &subs,
     const size_t at_off = p.put(off), at_tabs = p.put(tabs),
                  at_center = p.put(nullptr, sizeof(float) * subs.size());  // made by the coefficient kernel
     cudaError_t e = device_alloc(&st.coef, sizeof(float4) * std::max<int64_t>(1, st.ncoef));
-    if (e == cudaSuccess) e = p.upload(&st.block, stream);
+    if (e == cudaSuccess) e = p.upload(&st.block, &st.block_room, stream);
     if (e != cudaSuccess) {
         err = std::string("tensor-core buffers: ") + cudaGetErrorString(e);
         tc_release(st);

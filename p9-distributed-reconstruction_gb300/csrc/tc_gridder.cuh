@@ -20,6 +20,7 @@ struct TcPlanState {
     void *coef = nullptr;         // float4 {du, dv, dw, dw - centre} per gridded visibility, subgrid order
     // one allocation each: center, coef_off and tables; ditems, gitems and gsubs
     void *block = nullptr, *item_block = nullptr;
+    size_t block_room = 0, item_room = 0;
     void *center = nullptr;       // float per subgrid: its centre dw0 = mean(dw)
     void *coef_off = nullptr;     // int64 per subgrid: first coefficient of the subgrid
     void *tables = nullptr;       // float: g[32] (separable part of n), r[32][32] (remainder), l[32],
