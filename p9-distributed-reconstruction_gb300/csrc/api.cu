@@ -150,8 +150,8 @@ struct p9idg_plan {
     double tc_w_term = -1;  // max |dw| * max |r| of the plan's samples, once a tensor-core mode was asked for
     double dw_max = 0;      // max |k| * max |w| over the plan's samples
     // Whether the FP32 mode's device (complex64) calls run on the tensor cores, with FP16 operands split
-    // hi + lo: see fp32_on_tensor_cores.  The host-array calls, whose results keep to the last bit and
-    // which may pass a uvw of their own, run the sincos kernels.
+    // hi + lo: see fp32_on_tensor_cores.  The host-array calls run the sincos kernels: the choice rests on the
+    // plan's uvw, and they may pass one of their own.
     bool fp32_tc = false;
     bool fp32_tc_wanted = true;  // p9idg_plan_set_fp32_tensor_cores
     int64_t wave_grid = 0, wave_degrid = 0;  // default tensor-core work-item sizes (0: not worked out yet)
@@ -691,7 +691,7 @@ p9idg_status add_subgrids(p9idg_plan *p, float2 *d_layers, bool wstack, const in
     a.layers = d_layers;
     a.out_shifted = true;  // IDG.cs:17,37
     a.wstack = wstack;
-    a.keep_bits = !device_call;
+    a.two_pass = !device_call;
     a.pdl = after_gridder && !p->timing;  // (a stage's events would be the launch before it)
     if (d_list) {
         a.sub_list = d_list;
@@ -759,7 +759,7 @@ p9idg_status run_degrid(p9idg_plan *p, const float2 *d_grid, bool grid_shifted, 
         a.grid_shifted = grid_shifted;
         a.subgrids = p->d_subgrids.as<float2>();
         a.wstack = wstack;
-        a.keep_bits = out_c128;
+        a.two_pass = out_c128;
         CK(launch_split_subgrid_fft(a, p->stream));
     }
     if (!out_in_host && !fused) CK(launch_zero_ranges_beside(d_vis, out_c128, p->d_gaps.as<int64_t>(), ngaps, p->zside));

@@ -160,8 +160,8 @@ struct SubgridOpArgs {
     int32_t *status;
     const int2 *refs;          // batched launches: (problem, subgrid) per block; nsub = count
     const int32_t *sub_list;   // own launches: subgrid index per block (null: the block index)
-    const float2 *twiddles;    // exp(+2 pi i j / S), j < S, made in FP64 (null, with keep_bits: made there)
-    bool keep_bits;            // host-array calls: the form whose results those keep
+    const float2 *twiddles;    // exp(+2 pi i j / S), j < S, made in FP64 (null, with two_pass: made there)
+    bool two_pass;             // host-array calls: DFTs in two passes instead of FFTs in registers
     bool pdl;                  // adder, own form: the tensor-core gridder is the launch before it
 };
 cudaError_t launch_subgrid_ifft_add(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs = nullptr);

@@ -268,7 +268,7 @@ extern "C" p9idg_status p9idg_grid_w_device_noalloc(const p9idg_params *c, const
         o.out_shifted = true;
         o.wstack = true;
         o.status = d_status;
-        o.keep_bits = true;  // (its scratch holds no twiddles)
+        o.two_pass = true;  // (its scratch holds no twiddles)
         e = launch_subgrid_ifft_add(o, st);
     }
     if (e != cudaSuccess) return noalloc_fail(P9IDG_CUDA_ERROR, std::string("launch: ") + cudaGetErrorString(e));

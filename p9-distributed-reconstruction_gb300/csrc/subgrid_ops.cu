@@ -14,10 +14,10 @@
 //
 // One CTA per subgrid, in two forms.  Device calls and batches run S = 8 Q points a line as an 8-point
 // transform in registers, twiddles, and a Q-point one, four such steps for both axes: each value
-// crosses shared memory three times (fft_* below).  Host-array calls, whose results keep to the last
-// bit, run two passes of S-point DFTs against a twiddle table in shared memory, each split radix-4 and
-// then in two (dft_* below; an eighth of the O(S^3) multiply-adds, seven shared-memory reads a value
-// and pass, which bound them).
+// crosses shared memory three times (fft_* below).  Host-array calls, which wait for the host's memory and
+// not for these kernels, and the allocation-free gridder run two passes of S-point DFTs against a twiddle
+// table in shared memory, each split radix-4 and then in two (dft_* below; an eighth of the O(S^3)
+// multiply-adds, seven shared-memory reads a value and pass, which bound them).
 
 #include "kernels.cuh"
 
@@ -583,12 +583,12 @@ cudaError_t split_by_size(const SubgridOpArgs &a, cudaStream_t st) {
 
 cudaError_t launch_subgrid_ifft_add(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs) {
     if (probs) return fft_by_size<true, false>(a, st, probs);
-    return a.keep_bits ? ifft_add_by_size(a, st) : fft_by_size<false, false>(a, st, nullptr);
+    return a.two_pass ? ifft_add_by_size(a, st) : fft_by_size<false, false>(a, st, nullptr);
 }
 
 cudaError_t launch_split_subgrid_fft(const SubgridOpArgs &a, cudaStream_t st, const SubgridOpArgs *probs) {
     if (probs) return fft_by_size<true, true>(a, st, probs);
-    return a.keep_bits ? split_by_size(a, st) : fft_by_size<false, true>(a, st, nullptr);
+    return a.two_pass ? split_by_size(a, st) : fft_by_size<false, true>(a, st, nullptr);
 }
 
 }  // namespace p9idg
