@@ -51,7 +51,8 @@ enum {
     P9IDG_MODE_FP32 = 0,      /* FP32 accuracy, FP64 per-visibility phase argument: sincos + FMA kernels, and for
                                * device (complex64) calls on subgrids of 16, 24 and 32 whose w spread allows it
                                * FP16 hi+lo tensor-core operands about each subgrid's own w, summed in FP32 every
-                               * 64 visibilities, no less accurate */
+                               * 64 visibilities: measured no further from 64 bits than the sincos kernels
+                               * (p9idg_plan_info.device_form, p9idg_plan_set_fp32_tensor_cores) */
     P9IDG_MODE_TC_BF16X3 = 1, /* tensor cores, BF16 hi+lo split (3 products), FP32 accumulation */
     P9IDG_MODE_TC_FP16X3 = 2  /* tensor cores, FP16 hi+lo split (3 products), FP32 accumulation */
 };
