@@ -208,43 +208,66 @@ __device__ __forceinline__ uint32_t cd_peer(uint32_t addr, unsigned rank) {
     return r;
 }
 
-// 16 bytes into another CTA's shared memory; they count towards that CTA's barrier when they are there.
-__device__ __forceinline__ void cd_st_peer(uint32_t dst, uint32_t bar, const uint4 &v) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(v.x),
-                 "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+// The same into another CTA's shared memory, and from this one's.  The packets carry their epoch at the scope of
+// the pair, so nothing has to be acquired: a wait for st.async has to acquire at cluster scope, which empties
+// L1, and the tiles' pixels then come from L2 in every iteration (1000 iterations at 3072^2, whole windows: 4.68 ms
+// against 4.62, windows clipped by the edges 3.73 against 3.53 us an iteration).
+__device__ __forceinline__ void st_peer(uint32_t dst, const uint4 &v) {
+    const unsigned long long lo = v.x | (static_cast<unsigned long long>(v.y) << 32),
+                             hi = v.z | (static_cast<unsigned long long>(v.w) << 32);
+    asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.cluster.shared::cluster.b128 [%0], q;\n}\n" ::"r"(dst),
+                 "l"(lo), "l"(hi)
                  : "memory");
+}
+
+__device__ __forceinline__ uint4 ld_peer(uint32_t p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n.reg .b128 q;\nld.relaxed.cluster.shared::cta.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}\n"
+                 : "=l"(lo), "=l"(hi)
+                 : "r"(p)
+                 : "memory");
+    return make_uint4(static_cast<unsigned>(lo), static_cast<unsigned>(lo >> 32), static_cast<unsigned>(hi),
+                      static_cast<unsigned>(hi >> 32));
+}
+
+// A packet's candidate: |change| is not sent, it is the difference of the two values.
+__device__ __forceinline__ CdCand cd_unpack(const uint4 &q) {
+    return make_uint4(__float_as_uint(fabsf(__fsub_rn(__uint_as_float(q.w), __uint_as_float(q.z)))), q.y, q.z, q.w);
+}
+
+// Waits for the packet of this epoch at p (every lane its own, or the same one); false if it does not come.
+__device__ __forceinline__ bool cd_await_peer(uint32_t p, unsigned epoch, CdCand &v) {
+    const long long t0 = clock64();
+    while (true) {
+        const uint4 q = ld_peer(p);
+        if (q.x == epoch) {
+            v = cd_unpack(q);
+            return true;
+        }
+        if (clock64() - t0 > kCdPatience) return false;
+    }
 }
 
 __device__ __forceinline__ void cd_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void cd_expect(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+// An arrival on another CTA's barrier, which only says that a packet is on its way: waiting for it spares the polls
+// of its epoch (without it 4.69 ms and 3.63 us), which are what tells that the packet is there.
+__device__ __forceinline__ void cd_signal(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// The scope of the acquire holds the CTAs whose data is waited for: the cluster where st.async delivers it,
-// else the CTA alone.  The former empties L1, and the tiles' pixels then come from L2 in that iteration: 1000
-// iterations at 3072^2 take 4.68 ms, against 4.50 with CTA scope, which the memory model does not let stand for
-// it (16-byte packets that carry their iteration, in place of st.async, 4.67 and 3 % more without pairs).
-__device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase, bool from_peer) {
+// For what this CTA's own warps wrote to its shared memory.
+__device__ __forceinline__ bool cd_wait(uint32_t bar, uint32_t phase) {
     long long t0 = 0;
     while (true) {
         uint32_t done;
-        if (from_peer)
-            asm volatile(
-                "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                "selp.u32 %0, 1, 0, p;\n}\n"
-                : "=r"(done)
-                : "r"(bar), "r"(phase)
-                : "memory");
-        else
-            asm volatile(
-                "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n"
-                "selp.u32 %0, 1, 0, p;\n}\n"
-                : "=r"(done)
-                : "r"(bar), "r"(phase)
-                : "memory");
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(phase)
+            : "memory");
         if (done) return true;
         const long long t = clock64();
         if (t0 == 0) t0 = t;
@@ -444,23 +467,25 @@ __global__ void __launch_bounds__(kCdNT) cd_pick_kernel(const unsigned long long
 // ay x ax CTAs: a window of at most that many tiles gives no CTA two of them.
 //
 // The exchange: every warp puts its best candidate into its cluster's first CTA (a cluster is one CTA or
-// a pair), whose first warp posts the best of them as one 16-byte packet that carries the iteration's
+// a PAIR), whose first warp posts the best of them as one 16-byte packet that carries the iteration's
 // number, reads every cluster's packet until all carry it, and hands the best to the cluster's warps.  No
 // fence, atomic or grid-wide counter is needed, and gradients and model stay out of it.  Buffers and
 // slots alternate between two sets: a slot is overwritten only after every cluster has posted the
 // iteration after it, hence read it.
 //
-// Measured for 1000 iterations at 3072^2 with a 768^2 window: 4.7 us an iteration, against 6.5 us for a
+// Measured for 1000 iterations at 3072^2 with a 768^2 window: 4.6 us an iteration, against 6.5 us for a
 // launch per iteration (graph replays with programmatic dependent launches, every CTA reducing all tile
-// keys).  Of the 4.7 us about 1.3 are the exchange and its two hops within a pair, 1.5 a warp's loads and
+// keys).  Of the 4.6 us about 1.3 are the exchange and its two hops within a pair, 1.5 a warp's loads and
 // evaluation, and the rest the wait for the slowest of 147 CTAs.
 //
 // A lane keeps in registers the candidate of its warp's rows of local tile `lane`; images of more than 32
 // tiles a CTA (4864 tiles, 5000^2 with two rows a warp) keep them in P.cand, which only this warp touches.
-template <int R>
+template <int R, bool PAIR>
 __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant__ CdParams P) {
-    __shared__ CdCand sm_in[2][2 * kCdWarps];  // candidates of the cluster's warps (first CTA)
-    __shared__ CdCand sm_sel[2];               // the selected candidate
+    __shared__ CdCand sm_in[2][kCdWarps];  // candidates of the first CTA's warps
+    __shared__ CdCand sm_sel[2];           // the selected candidate (first CTA)
+    __shared__ __align__(16) uint4 sm_peer[2][kCdWarps];  // packets: candidates of the second CTA's warps (first CTA)
+    __shared__ __align__(16) uint4 sm_told[2];            // the selected candidate (second CTA)
     __shared__ unsigned long long bar_in[2], bar_sel[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const CdCtl c0 = *P.ctl;
@@ -468,26 +493,22 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
         if (blockIdx.x == 0 && threadIdx.x == 0) P.report[0] = c0;
         return;
     }
-    unsigned rank, csize;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
-    const bool pair = csize == 2;
+    constexpr unsigned csize = PAIR ? 2 : 1;
+    unsigned rank = 0;
+    if (PAIR) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const CdCand none = make_uint4(0u, 0u, 0u, 0u);
     const int nslots = static_cast<int>(gridDim.x / csize), slot = static_cast<int>(blockIdx.x / csize);
     const uint32_t in_bar = cd_shared(bar_in), sel_bar = cd_shared(bar_sel);
     if (threadIdx.x == 0) {
         for (int b = 0; b < 2; b++) {
-            // candidates: an arrival of each warp here, and in a pair the bytes of the other CTA's warps
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(in_bar + 8 * b), "r"(kCdWarps + (pair ? 1 : 0)));
-            // selection: an arrival of the first warp, or the bytes that it sends to the second CTA
+            // candidates: an arrival of each warp of the cluster; selection: one of its first warp
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(in_bar + 8 * b), "r"(csize * kCdWarps));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sel_bar + 8 * b));
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int b = 0; b < 2; b++) {
-            if (pair && rank == 0) cd_expect(in_bar + 8 * b, kCdWarps * sizeof(CdCand));
-            if (rank == 1) cd_expect(sel_bar + 8 * b, sizeof(CdCand));
-        }
     }
-    if (pair)
+    if (threadIdx.x < 2 * kCdWarps) sm_peer[threadIdx.x / kCdWarps][threadIdx.x % kCdWarps] = none;  // epochs start at 1
+    if (threadIdx.x < 2) sm_told[threadIdx.x] = none;
+    if (PAIR)
         cd_cluster_sync();
     else
         __syncthreads();
@@ -495,7 +516,6 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
     const int cta = blockIdx.x, cy = static_cast<int>(static_cast<uint32_t>(cta) / static_cast<uint32_t>(P.ax)), cx = cta - cy * P.ax;
     const bool owner = cy < P.ay;  // the last CTA of an odd number in pairs owns nothing
     const bool in_regs = P.local_tiles <= 32;
-    const CdCand none = make_uint4(0u, 0u, 0u, 0u);
     // this warp's candidate of local tile l = (ty / ay) * local_x + tx / ax; null past the image
     const auto at = [&](int l) -> CdCand * {
         const int q = l / P.local_x, ty = cy + q * P.ay, tx = cx + (l - q * P.local_x) * P.ax;
@@ -532,25 +552,25 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
         if (step == kCdLaunchIters) break;
         const int b = step & 1;
         const uint32_t phase = (step >> 1) & 1, in_b = in_bar + 8 * b, sel_b = sel_bar + 8 * b;
+        const unsigned epoch = static_cast<unsigned>(c.iter) + 1u;
         bool ok = true;
         if (lane == best_lane(best)) {
             if (rank == 0) {
                 sm_in[b][warp] = best;
                 cd_arrive(in_b);
             } else {
-                cd_st_peer(cd_peer(cd_shared(&sm_in[b][kCdWarps + warp]), 0), cd_peer(in_b, 0), best);
+                st_peer(cd_peer(cd_shared(&sm_peer[b][warp]), 0), make_uint4(epoch, best.y, best.z, best.w));
+                cd_signal(cd_peer(in_b, 0));
             }
         }
         if (rank == 0 && warp == 0) {
-            ok = __all_sync(0xffffffffu, cd_wait(in_b, phase, pair));
+            ok = cd_wait(in_b, phase);
+            CdCand v = none;
+            if (PAIR && ok && lane < kCdWarps) ok = cd_await_peer(cd_shared(&sm_peer[b][lane]), epoch, v);
+            ok = __all_sync(0xffffffffu, ok);
             if (ok) {
                 uint4 *slots = P.slots + (c.iter & 1) * kCdSlots;
-                const unsigned epoch = static_cast<unsigned>(c.iter) + 1u;
-                CdCand v = lane < kCdWarps ? sm_in[b][lane] : none;
-                if (pair) {
-                    if (lane < kCdWarps) v = better(v, sm_in[b][kCdWarps + lane]);
-                    if (lane == 0) cd_expect(in_b, kCdWarps * sizeof(CdCand));
-                }
+                if (lane < kCdWarps) v = PAIR ? better(sm_in[b][lane], v) : sm_in[b][lane];
                 if (lane == best_lane(v)) st_packet(slots + slot, make_uint4(epoch, v.y, v.z, v.w));
                 v = none;
                 unsigned want = 0;
@@ -566,9 +586,7 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
                     for (int j = 0; j < kCdPoll; j++) {
                         if (q[j].x != epoch) continue;  // epochs start at 1
                         want &= ~(1u << j);
-                        // |change| is not sent: it is the difference of the two values
-                        q[j].x = __float_as_uint(fabsf(__fsub_rn(__uint_as_float(q[j].w), __uint_as_float(q[j].z))));
-                        v = better(q[j], v);
+                        v = better(cd_unpack(q[j]), v);
                     }
                     if (!__any_sync(0xffffffffu, want != 0u)) break;
                     if (__any_sync(0xffffffffu, clock64() - t0 > kCdPatience)) {
@@ -577,21 +595,26 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
                     }
                 }
                 if (ok && lane == best_lane(v)) {
-                    if (pair) cd_st_peer(cd_peer(cd_shared(&sm_sel[b]), 1), cd_peer(sel_b, 1), v);
+                    if (PAIR) {
+                        st_peer(cd_peer(cd_shared(&sm_told[b]), 1), make_uint4(epoch, v.y, v.z, v.w));
+                        cd_signal(cd_peer(sel_b, 1));
+                    }
                     sm_sel[b] = v;
                     cd_arrive(sel_b);
                 }
             }
         }
         settle();  // while the exchange is under way
-        ok = __all_sync(0xffffffffu, ok && cd_wait(sel_b, phase, rank == 1));
+        CdCand s = none;
+        ok = ok && cd_wait(sel_b, phase);
+        if (PAIR && rank == 1) ok = ok && cd_await_peer(cd_shared(&sm_told[b]), epoch, s);
+        ok = __all_sync(0xffffffffu, ok);
+        if (rank == 0) s = sm_sel[b];
         if (!ok) {
             c = CdCtl{c.iter, 1, 0, 2};
             if (lane == 0) P.report[1].error = 2;
             break;
         }
-        if (rank == 1 && threadIdx.x == 0) cd_expect(sel_b, sizeof(CdCand));
-        const CdCand s = sm_sel[b];
         if (__uint_as_float(s.x) < P.eps) {  // converged = maxPixel.PixelMaxDiff < epsilon
             c = CdCtl{c.iter, 1, 1, 0};
             break;
@@ -652,7 +675,7 @@ __global__ void __launch_bounds__(kCdNT, 1) cd_run_kernel(const __grid_constant_
         *P.ctl = c;
         P.report[0] = c;
     }
-    if (pair) cd_cluster_sync();  // no CTA leaves while the other may still write to it
+    if (PAIR) cd_cluster_sync();  // no CTA leaves while the other may still write to it
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1235,8 +1258,9 @@ p9idg_status cd_set_maps(p9idg_cd *cd, const float *h_psf, int h, int w) {
 struct CdLaunch {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    CdLaunch(int nctas, cudaStream_t stream) {
-        const unsigned c = nctas >= kCdPairFrom ? 2 : 1;
+    bool pairs;
+    CdLaunch(int nctas, cudaStream_t stream) : pairs(nctas >= kCdPairFrom) {
+        const unsigned c = pairs ? 2 : 1;
         cfg.gridDim = dim3((static_cast<unsigned>(nctas) + c - 1) / c * c);
         cfg.blockDim = dim3(kCdNT);
         cfg.stream = stream;
@@ -1260,7 +1284,7 @@ p9idg_status cd_layout(p9idg_cd *cd) {
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, cd->device));
     CdLaunch two(kCdPairFrom, cd->stream);
     two.cfg.numAttrs = 1;
-    CK(cudaOccupancyMaxActiveClusters(&pairs, cd_run_kernel<2>, &two.cfg));
+    CK(cudaOccupancyMaxActiveClusters(&pairs, cd_run_kernel<2, true>, &two.cfg));
     const int most = 2 * std::min(pairs, kCdSlots);
     if (!coop || most < 2) return fail(P9IDG_UNSUPPORTED, "the device cannot run the coordinate-descent kernel");
     const auto div = [](int a, int b) { return (a + b - 1) / b; };
@@ -1332,7 +1356,9 @@ p9idg_status cd_run(p9idg_cd *cd, float *d_x, float *d_g, float lambda, float al
     // waits on the host; a launch after the stopping one does nothing (it sees the done flag).
     const int64_t launches = (static_cast<int64_t>(std::max(max_iter, 0)) + kCdLaunchIters - 1) / kCdLaunchIters;
     CdLaunch run(cd->hp.ax * cd->hp.ay, cd->stream);
-    const auto kernel = cd->hp.rows == 1 ? cd_run_kernel<1> : cd_run_kernel<2>;
+    const auto of_rows = [&](auto one, auto two) { return cd->hp.rows == 1 ? one : two; };
+    const auto kernel = run.pairs ? of_rows(cd_run_kernel<1, true>, cd_run_kernel<2, true>)
+                                  : of_rows(cd_run_kernel<1, false>, cd_run_kernel<2, false>);
     if (launches > 0) CK(cudaLaunchKernelEx(&run.cfg, kernel, cd->hp));
     for (int64_t r = 0; r < launches; r++) {
         CK(cudaEventRecord(cd->ev_ctl, cd->stream));
